@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(256) adjoint_walk_kernel(Workspace ws, Travers
   const int lane = threadIdx.x & 31;
   const int n = ws.n;
   const int m = sc->n_nodes;
-  const int n_groups = p.group_mode ? sc->n_tgroups : (n + 31) >> 5;
+  const int n_groups = sc->n_tgroups;
   const double g = p.g;
   bool singular = false;
   while (true) {
@@ -145,8 +145,8 @@ __global__ void __launch_bounds__(256) adjoint_walk_kernel(Workspace ws, Travers
     if (lane == 0) grp = (int)atomicAdd(&sc->work_counter, 1u);
     grp = __shfl_sync(kFull, grp, 0);
     if (grp >= n_groups) break;
-    const int g0 = p.group_mode ? ws.tstart[grp] : grp * 32;
-    const int g1 = p.group_mode ? ((grp + 1 < n_groups) ? ws.tstart[grp + 1] : n) : min(g0 + 32, n);
+    const int g0 = ws.tstart[grp];
+    const int g1 = (grp + 1 < n_groups) ? ws.tstart[grp + 1] : n;
     // a group larger than a warp is walked 32 targets at a time
     for (int c0 = g0; c0 < g1; c0 += 32) {
       const int c1 = min(c0 + 32, g1);
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(256) frozen_walk_kernel(Workspace ws, Traversa
   const int n = ws.n;
   const int m = sc->n_nodes;
   const size_t cap = (size_t)ws.cap_nodes;
-  const int n_groups = p.group_mode ? sc->n_tgroups : (n + 31) >> 5;
+  const int n_groups = sc->n_tgroups;
   const unsigned items = (unsigned)n_groups * (unsigned)fb.copies;
   const double g = p.g;
   bool singular = false;
@@ -400,8 +400,8 @@ __global__ void __launch_bounds__(256) frozen_walk_kernel(Workspace ws, Traversa
     const int grp = (int)(item - (unsigned)q * (unsigned)n_groups);
     const double4 *pm4q = fb.pm4q + (size_t)q * n;
     const double4 *node_aq = fb.node_aq + (size_t)q * cap;
-    const int g0 = p.group_mode ? ws.tstart[grp] : grp * 32;
-    const int g1 = p.group_mode ? ((grp + 1 < n_groups) ? ws.tstart[grp + 1] : n) : min(g0 + 32, n);
+    const int g0 = ws.tstart[grp];
+    const int g1 = (grp + 1 < n_groups) ? ws.tstart[grp + 1] : n;
     // a group larger than a warp is walked 32 targets at a time
     for (int c0 = g0; c0 < g1; c0 += 32) {
       const int c1 = min(c0 + 32, g1);

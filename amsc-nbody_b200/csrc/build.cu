@@ -1300,7 +1300,10 @@ __global__ void __launch_bounds__(kBlock) layout_kernel(Workspace ws, double the
     if (pc <= 0 && cnt == 0 && mass != 0.0) record_error(sc, kStageTraversal, 5);
     const double comx = ws.comx[node], comy = ws.comy[node], comz = ws.comz[node];
     const double cx = ws.cx[node], cy = ws.cy[node], cz = ws.cz[node];
-    ws.node_a[pre] = make_double4(comx, comy, comz, mass);
+    // an occupied leaf's record carries its first particle (what the walks
+    // take from a leaf; its centre of mass is only combined upwards)
+    const double4 rec_a = pc > 0 ? ws.pm4[f] : make_double4(comx, comy, comz, mass);
+    ws.node_a[pre] = rec_a;
     ws.node_b[pre] = make_double4(cx, cy, cz, h);
     const double side = __dmul_rn(2.0, h);
     const double ox = __dsub_rn(comx, cx), oy = __dsub_rn(comy, cy), oz = __dsub_rn(comz, cz);
@@ -1325,7 +1328,7 @@ __global__ void __launch_bounds__(kBlock) layout_kernel(Workspace ws, double the
     ws.node_meta[pre] = make_int4(pre + size, pc > 0 ? f : -1, pc > 0 ? pc : 0, j);
     if (ws.node_m) {
       MixedNode rec;
-      rec.a = make_double4(comx, comy, comz, mass);
+      rec.a = rec_a;
       rec.cr2 = __double2float_ru(cm * cm * (1.0 + 0x1p-18));
       rec.first = pc > 0 ? f : -1;
       rec.count = pc > 0 ? pc : 0;
@@ -1417,6 +1420,35 @@ __global__ void __launch_bounds__(kScanThreads) group_scan_kernel(Workspace ws) 
   for (int k = 0; k < kScanItems; ++k) {
     const int i = base + k * kScanThreads + threadIdx.x;
     flag[k] = (i < n) ? (int)ws.tflag[i] : 0;
+  }
+  if (ws.group_chunk > 0) {
+    // groups cut into runs of group_chunk (a power of two) particles: a
+    // particle starts one when its distance from its group's start is a
+    // multiple of it.  The start lies at most kGroupMaxLimit - 1 before it:
+    // the tile's marks and the words before it as bits.
+    constexpr int kLead = kGroupMaxLimit / 32;
+    __shared__ unsigned marks[kLead + kScanTile / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+      const unsigned w = __ballot_sync(0xffffffffu, flag[k]);
+      if (lane == 0) marks[kLead + k * (kScanThreads / 32) + warp] = w;
+    }
+    if (warp < kLead) {
+      const int i = base - kGroupMaxLimit + 32 * warp + lane;
+      const unsigned w = __ballot_sync(0xffffffffu, i >= 0 && ws.tflag[i] != 0);
+      if (lane == 0) marks[warp] = w;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+      const int at = kGroupMaxLimit + k * kScanThreads + threadIdx.x;
+      int word = at >> 5;
+      unsigned w = marks[word] & ((2u << (at & 31)) - 1u);
+      while (w == 0u && word > 0) w = marks[--word];
+      const int start = 32 * word + 31 - __clz(w);
+      flag[k] = (base + k * kScanThreads + threadIdx.x < n && w != 0u && ((at - start) & (ws.group_chunk - 1)) == 0) ? 1 : 0;
+    }
   }
   const unsigned long long total = block_scan_rows<kScanItems, kScanThreads>(flag, excl, row_warp, &s_total);
   if (threadIdx.x < 32) {
@@ -1908,6 +1940,7 @@ __device__ __forceinline__ bool lo_leaf_cell(const Workspace &ws, int g, int M, 
     wz = __fma_rn(q.w, q.z, wz);
   }
   lo_emit_node(ws, bleaf, tm, wx, wy, wz, c);
+  c.a = ws.pm4[pf];  // the traversal records of a leaf carry its first particle
   const int np = pe - pf;
   if (lo_whole_group(ws, c.level, np, true)) {
     if (c.level == ws.sys_levels) ws.tflag[pf] = 1;

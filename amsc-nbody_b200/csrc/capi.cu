@@ -243,10 +243,26 @@ cudaError_t alloc_workspace(Workspace &ws, Allocation &al, int n, bool with_stat
 
 bool finite_nonneg(double v) { return std::isfinite(v) && v >= 0.0; }
 
-// The plain walk's per-lane acceptance test tolerates wide warps and prefers
-// full ones (fixed 32-particle slices); the mixed walk shares one acceptance
-// test per warp and needs compact octree target groups.
-int default_group_mode(int precision) { return precision == NBB_PRECISION_MIXED ? 1 : 0; }
+// Targets per warp of the plain FP64 walk.  A walk costs a warp hardly less
+// for one target than for 32, so one is taken only while that leaves the GPU
+// unfilled: traversal of Plummer spheres, 1 / 32 targets per warp, 60 / 156 us
+// at 1000 particles, 208 / 400 at 4096, 1040 / 570 at 16384.
+int fp64_targets(int n) { return n < 8192 ? 1 : 32; }
+
+// The target groups a walk needs: their largest size and the pieces the plain
+// walk takes them in.  Groups of up to 128 cut into 32 fill the lanes better
+// than groups of up to 32 (27 targets per warp against 23 at 2^18 particles:
+// 2.9 against 3.1 ms), which in turn give smaller systems more warps (16384
+// particles: 700 against 780 us).
+void set_groups(Workspace &ws, const TraversalParams &tp) {
+  if (tp.precision == NBB_PRECISION_MIXED) {
+    ws.group_max = tp.group_size > 64 ? 128 : (tp.group_size > 32 ? 64 : 32);
+    ws.group_chunk = 0;
+  } else {
+    ws.group_max = ws.n < 131072 ? 32 : 128;
+    ws.group_chunk = tp.targets;
+  }
+}
 
 template <typename T>
 cudaError_t d2h_opt(T *dst, const T *src, size_t count, cudaStream_t s) {
@@ -329,7 +345,7 @@ int check_device(const Workspace &ws, cudaStream_t s) {
 // walk + kick.
 cudaError_t enqueue_rebuild_force(Workspace &ws, const TraversalParams &tp, double dt, int kd,
                                   cudaStream_t s, int part = 0) {
-  ws.group_max = (tp.group_mode && tp.group_size > 32) ? (tp.group_size > 64 ? 128 : 64) : 32;
+  set_groups(ws, tp);
   // the level-order build writes only the records of this walk
   ws.records = tp.precision == NBB_PRECISION_MIXED ? kRecordsMixed : kRecordsFp64;
   cudaError_t e = cudaSuccess;
@@ -431,8 +447,8 @@ struct nbb_sim {
   cudaGraph_t step_graph_def = nullptr;
   uint64_t graph_kernels = 0;
   int tuned_group_size = 0;
+  int walk_targets = 0;           // targets per warp of the plain walk; 0: by size
   int tuned_cache_depth = -1;     // mixed walk's node-cache depth; -1 untuned
-  int tuned_fp64_grouping = -1;  // plain walk: 0 Morton slices, 1 octree groups; -1 untuned
   double min_softening = 0.0;  // ensembles: smallest per-system softening
   std::unique_ptr<RolloutRecord> rollout;
   std::unique_ptr<FrameBuffers> frames;
@@ -610,15 +626,11 @@ static TraversalParams traversal_params(const nbb_sim *sim, int kick) {
   tp.precision = sim->cfg.precision;
   tp.group_size = sim->cfg.group_size > 0 ? sim->cfg.group_size
                                           : (sim->tuned_group_size > 0 ? sim->tuned_group_size : 32);
-  tp.group_mode = default_group_mode(tp.precision);
+  tp.targets = sim->walk_targets > 0 ? sim->walk_targets : fp64_targets(sim->ws.n);
   if (tp.precision == NBB_PRECISION_MIXED && sim->ws.top && sim->ws.n_systems == 1)
     tp.cache_depth = sim->cfg.cache_depth >= 0 ? sim->cfg.cache_depth
                                                : (sim->tuned_cache_depth > 0 ? sim->tuned_cache_depth : 0);
-  if (tp.precision == NBB_PRECISION_FP64 && sim->tuned_fp64_grouping >= 0) tp.group_mode = sim->tuned_fp64_grouping;
-  if (sim->ws.n_systems > 1) {
-    tp.group_mode = 1;  // a warp's targets must share a system
-    tp.soft = sim->min_softening;
-  }
+  if (sim->ws.n_systems > 1) tp.soft = sim->min_softening;
   return tp;
 }
 
@@ -674,7 +686,7 @@ static int autotune_mixed_walk(nbb_sim *sim) {
       for (int c = 0; c < n_sizes && e == cudaSuccess; ++c) {
         TraversalParams tp = traversal_params(sim, 0);
         tp.group_size = pinned ? pinned : sizes[c];
-        ws.group_max = tp.group_size;
+        set_groups(ws, tp);
         for (int d = 0; d < n_depths && e == cudaSuccess; ++d) {
           tp.cache_depth = cacheable ? (pinned_depth >= 0 ? pinned_depth : d) : 0;
           e = launch_retarget(ws, s);
@@ -709,64 +721,10 @@ static int autotune_mixed_walk(nbb_sim *sim) {
   }
   // the initial acceleration comes from the chosen setting
   TraversalParams tp = traversal_params(sim, 0);
-  ws.group_max = tp.group_size;
+  set_groups(ws, tp);
   NBB_CUDA(launch_retarget(ws, sim->stream), "retarget");
   NBB_CUDA(launch_traversal(ws, tp, sim->stream), "traversal");
   return check_device(ws, sim->stream);
-}
-
-// Grouping autotuner of the plain FP64 walk: every lane follows its own
-// target's node sequence, so results do not depend on which targets share a
-// warp, only the time does -- fixed slices of 32 Morton-consecutive targets
-// (short runs, best for large systems) or octree target groups of at most 32
-// (compact, best where few warps must fill the GPU).  Timed on the tree of
-// the first force evaluation (best of two each), cached per process and
-// power-of-two size bucket.
-static std::vector<std::pair<int, int>> g_tuned_fp64;  // (log2 bucket, grouping)
-
-static int autotune_fp64_grouping(nbb_sim *sim) {
-  Workspace &ws = sim->ws;
-  int bucket = 0;
-  while ((1 << bucket) < ws.n && bucket < 31) ++bucket;
-  {
-    std::lock_guard<std::mutex> g(g_tune_lock);
-    for (const auto &kv : g_tuned_fp64)
-      if (kv.first == bucket) {
-        sim->tuned_fp64_grouping = kv.second;
-        return ok();
-      }
-  }
-  cudaStream_t s = sim->stream;
-  cudaEvent_t e0, e1;
-  NBB_CUDA(cudaEventCreate(&e0), "cudaEventCreate");
-  NBB_CUDA(cudaEventCreate(&e1), "cudaEventCreate");
-  float best = 1e30f;
-  int best_mode = 0;
-  cudaError_t e = cudaSuccess;
-  for (int mode = 0; mode < 2 && e == cudaSuccess; ++mode) {
-    TraversalParams tp = traversal_params(sim, 0);
-    tp.group_mode = mode;
-    for (int rep = 0; rep < 2 && e == cudaSuccess; ++rep) {
-      e = launch_retarget(ws, s);
-      if (e == cudaSuccess) e = cudaEventRecord(e0, s);
-      if (e == cudaSuccess) e = launch_traversal(ws, tp, s);
-      if (e == cudaSuccess) e = cudaEventRecord(e1, s);
-      if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-      float ms = 0.f;
-      if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-      if (e == cudaSuccess && ms < best) {
-        best = ms;
-        best_mode = mode;
-      }
-    }
-  }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  if (e != cudaSuccess) return cuda_fail(e, "walk grouping autotuning");
-  sim->tuned_fp64_grouping = best_mode;
-  std::lock_guard<std::mutex> g(g_tune_lock);
-  g_tuned_fp64.emplace_back(bucket, best_mode);
-  return check_device(ws, s);
 }
 
 int nbb_sim_initialize(nbb_sim *sim) {
@@ -787,13 +745,6 @@ int nbb_sim_initialize(nbb_sim *sim) {
   }
   if (sim->cfg.precision == NBB_PRECISION_MIXED) {
     st = autotune_mixed_walk(sim);
-    if (st) {
-      sim->state = nbb_sim::State::failed;
-      return st;
-    }
-  }
-  if (sim->cfg.precision == NBB_PRECISION_FP64 && ws.n_systems == 1) {
-    st = autotune_fp64_grouping(sim);
     if (st) {
       sim->state = nbb_sim::State::failed;
       return st;
@@ -1153,7 +1104,7 @@ int nbb_accel(size_t n, const double *mass, const double *x, const double *y, co
   tp.soft = softening;
   tp.g = g;
   tp.precision = precision;
-  tp.group_mode = default_group_mode(precision);
+  tp.targets = fp64_targets((int)n);
   NBB_CUDA(enqueue_rebuild_force(ws, tp, 0.0, 0, sc.s), "Barnes-Hut evaluation");
   int st = check_device(ws, sc.s);
   if (st) return st;
@@ -1709,14 +1660,16 @@ cudaError_t copy_state(nbb_sim *sim, double *slot, int count, bool save) {
 cudaError_t enqueue_vjp(nbb_sim *sim, const TraversalParams &tpa, const AdjointBuffers &ab) {
   Workspace &ws = sim->ws;
   cudaStream_t s = sim->stream;
-  const int group_max = ws.group_max;
+  const int group_max = ws.group_max, group_chunk = ws.group_chunk;
   ws.group_max = 32;  // target groups of one warp (kernels take the workspace by value)
+  ws.group_chunk = 0;
   cudaError_t e = launch_step_reset(ws, s);
   if (e == cudaSuccess) e = launch_kd_bbox(ws, 0.0, 0, s);
   if (e == cudaSuccess) e = launch_morton_sort_groups(ws, s);
   if (e == cudaSuccess) e = launch_tree(ws, tpa.theta, s);
   if (e == cudaSuccess) e = launch_adjoint_force(ws, tpa, ab, s);
   ws.group_max = group_max;
+  ws.group_chunk = group_chunk;
   return e;
 }
 
@@ -1826,7 +1779,6 @@ int nbb_sim_backward(nbb_sim *sim, const double *gx, const double *gy, const dou
   TraversalParams tpa = traversal_params(sim, 0);
   tpa.precision = sim->cfg.precision == NBB_PRECISION_MIXED ? 1 : 0;
   tpa.kick = 0;
-  tpa.group_mode = 1;  // compact warps; the plain form's sums do not depend on it
   tpa.group_size = 32;
   tpa.cache_depth = 0;
   cudaError_t e = cudaSuccess;
@@ -1888,8 +1840,10 @@ int nbb_frozen_rollout(const nbb_config *cfg, size_t n, const double *mass, cons
   int st = create_sim(&c2, n, 1, nullptr, nullptr, mass, x, y, z, vx, vy, vz, nullptr, on_device, &sim);
   if (st) return st;
   std::unique_ptr<nbb_sim, int (*)(nbb_sim *)> guard(sim, nbb_sim_destroy);
-  // the frozen walk reads the octree in the reference numbering
+  // the frozen walk reads the octree in the reference numbering, and takes
+  // the target groups a warp at a time
   sim->ws.level_order = 0;
+  sim->walk_targets = 32;
   st = nbb_sim_initialize(sim);
   if (st) return st;
   Workspace &ws = sim->ws;
@@ -2116,15 +2070,16 @@ int nbb_sim_diagnostics(nbb_sim *sim, int potential, nbb_diagnostics *d) {
     // to other positions, e.g. after a backward pass)
     TraversalParams tp = traversal_params(sim, 0);
     tp.precision = 0;
-    tp.group_mode = 1;
-    const int group_max = ws.group_max;
+    const int group_max = ws.group_max, group_chunk = ws.group_chunk;
     ws.group_max = 32;  // target groups of one warp
+    ws.group_chunk = 0;
     cudaError_t e = launch_step_reset(ws, s);
     if (e == cudaSuccess) e = launch_kd_bbox(ws, 0.0, 0, s);
     if (e == cudaSuccess) e = launch_morton_sort_groups(ws, s);
     if (e == cudaSuccess) e = launch_tree(ws, tp.theta, s);
     if (e == cudaSuccess) e = launch_potential_tree(ws, tp, db.phi, s);
     ws.group_max = group_max;
+    ws.group_chunk = group_chunk;
     NBB_CUDA(e, "potential evaluation");
     phi = db.phi;
   } else if (potential == NBB_POTENTIAL_DIRECT) {

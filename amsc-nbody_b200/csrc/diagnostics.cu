@@ -90,14 +90,14 @@ __global__ void __launch_bounds__(256) potential_tree_kernel(Workspace ws, Trave
   const int lane = threadIdx.x & 31;
   const int n = ws.n;
   const int m = sc->n_nodes;
-  const int n_groups = p.group_mode ? sc->n_tgroups : (n + 31) >> 5;
+  const int n_groups = sc->n_tgroups;
   while (true) {
     int grp = 0;
     if (lane == 0) grp = (int)atomicAdd(&sc->work_counter, 1u);
     grp = __shfl_sync(kFull, grp, 0);
     if (grp >= n_groups) break;
-    const int g0 = p.group_mode ? ws.tstart[grp] : grp * 32;
-    const int g1 = p.group_mode ? ((grp + 1 < n_groups) ? ws.tstart[grp + 1] : n) : min(g0 + 32, n);
+    const int g0 = ws.tstart[grp];
+    const int g1 = (grp + 1 < n_groups) ? ws.tstart[grp + 1] : n;
     // a group larger than a warp is walked 32 targets at a time
     for (int c0 = g0; c0 < g1; c0 += 32) {
       const int c1 = min(c0 + 32, g1);
@@ -205,7 +205,7 @@ cudaError_t launch_moments(const double *m, const double *x, const double *y, co
 cudaError_t launch_potential_tree(Workspace &ws, const TraversalParams &p, double *phi, cudaStream_t s) {
   // the walk takes work from the traversal counter; the build's reset
   // zeroed it
-  potential_tree_kernel<<<ws.fp64_grid > 0 ? ws.fp64_grid : 148, 256, 0, s>>>(ws, p, phi);
+  potential_tree_kernel<<<(ws.num_sms > 0 ? ws.num_sms : 148) * 4, 256, 0, s>>>(ws, p, phi);
   count_launches(1);
   return cudaGetLastError();
 }

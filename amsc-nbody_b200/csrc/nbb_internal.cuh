@@ -90,7 +90,7 @@ constexpr int kScanTile = kScanThreads * kScanItems;
 // centre of mass and mass, the squared acceptance radius for a target box
 // rounded up to FP32, and the node's particle range and child count.
 struct __align__(16) MixedNode {
-  double4 a;   // com x, y, z, mass
+  double4 a;   // com x, y, z, mass (an occupied leaf: its first particle)
   float cr2;   // (max(crit, sqrt(3) h + |com - centre|) (1 + 2^-40))^2 (1 + 2^-18), rounded up
   int first;   // first particle of an occupied leaf, -1 otherwise
   int count;   // particles of an occupied leaf, 0 otherwise
@@ -142,12 +142,13 @@ struct Workspace {
   int n = 0;            // particle count
   int cap_nodes = 0;    // octree node capacity (sum over levels of min(8^L, n))
   int num_sms = 0;
-  int fp64_grid = 0;    // persistent traversal grids (blocks)
+  int fp64_grid[2] = {0, 0};  // persistent traversal grids (blocks): 32 and 1 targets per warp
   int mixed_grid[2][3] = {{0, 0, 0}, {0, 0, 0}};  // [track source][1, 2 or 4 targets per lane]
   int vjp_grid = 0;     // the mixed walk's adjoint form
   int walk_warps = 0;     // warps of the largest mixed-walk grid
   int walk_ext_cap = 0;   // entries per warp of the mixed walk's stack extension
   int group_max = 32;   // largest octree target group: 32, 64 or 128 (32 x target slots per lane)
+  int group_chunk = 0;  // particles per work item a group is cut into (a power of two; 0: not cut)
   int group_depth = kGroupDepth;  // shallowest cell (levels below its system's root) a group may span
 
   // key layout: an ensemble's system id sits above the 30 Morton bits and
@@ -217,7 +218,7 @@ struct Workspace {
   int *tstart = nullptr;           // n, start of each target group
 
   // traversal layout: depth-first preorder, children visited octant 7 -> 0
-  double4 *node_a = nullptr;  // com x, y, z, mass
+  double4 *node_a = nullptr;  // com x, y, z, mass (an occupied leaf: its first particle)
   double4 *node_b = nullptr;  // centre x, y, z, half size
   double4 *node_c = nullptr;  // crit, crit^2 lower/upper band, mixed walk's squared box radius
   int4 *node_meta = nullptr;  // skip, first particle, particle count, nchild
@@ -316,9 +317,7 @@ struct TraversalParams {
   int kick = 0;
   int precision = 0;     // 0 FP64 plain, 1 mixed
   int group_size = 32;
-  // warp target sets: 0 = fixed slices of 32 consecutive Morton-ordered
-  // particles, 1 = octree target groups (contiguous, inside one parent cell)
-  int group_mode = 0;
+  int targets = 32;  // FP64: targets per warp, 32 or 1 (the build's group_chunk)
   // mixed walk: tree levels below the root staged in shared memory per block
   // (0: none; 1 or 2: the top 9 or 73 cells; level-order builds of a single
   // system only)

@@ -12,6 +12,7 @@
 //  kick / kick_drift      integrator.cu:51-106.
 #include "nbb_internal.cuh"
 #include "walk_fp64.cuh"
+#include "walk_list.cuh"
 
 #include <algorithm>
 #include <climits>
@@ -28,119 +29,134 @@ __device__ __forceinline__ long long warp_sum_ll(long long v) {
   return v;
 }
 
-// Plain FP64 traversal, one warp per 32 Morton-consecutive targets.
+// Plain FP64 traversal: one warp per set of at most kTargets Morton-consecutive
+// targets, on the ordered interaction list of walk_list.cuh.  Every target
+// sees its own node sequence of the reference's stackless walk
+// (barnes_hut.cu:90-162): a list entry counts for a target when its preorder
+// index has reached the target's resume index, and an undecided cell that the
+// target accepts moves that index past the cell's subtree.
 //
-// The tree is laid out in depth-first preorder with children visited octant
-// 7 -> 0, so the reference's per-thread stackless walk (barnes_hut.cu:90-162)
-// becomes: a target opened at node i continues at i + 1, a target done with
-// node i (accepted, zero mass, or a leaf) continues at skip(i).  Each lane
-// keeps its own resume index and the warp always visits the smallest one, so
-// every lane sees exactly its own node sequence -- the reference's
-// interaction set in the reference's order -- while node records are fetched
-// once per warp (broadcast loads) instead of once per thread.
-__global__ void __launch_bounds__(256) traverse_fp64_kernel(Workspace ws, TraversalParams p) {
+// With 32 targets a lane holds one target and the warp takes the entries in
+// order, four in flight.  With one target the 32 lanes form the terms of 32
+// consecutive entries at once; the terms are then added in entry order, each
+// component's sum by one lane, so the result has the same bits.  One target
+// per warp wastes the walk on a single target but fills the GPU from small
+// systems (see fp64_targets).
+//
+// Bound at 2^20 particles: instruction issue and FP64 latency (FP64 pipe 49 %,
+// issue 61 % busy at 16 warps per SM; an entry takes 25 FP64 operations of
+// 2.2 cycles).  16 warps with 128 registers, four entries in flight, beat 20
+// warps of 96 registers and 24 of 80 (10.7, 11.8 and 12.4 ms).
+constexpr int kFp64Warps = 2;
+
+template <int kTargets>
+struct Fp64Shared {
+  ListShared list[kFp64Warps];
+  double4 term[kTargets < 32 ? kFp64Warps : 1][kTargets < 32 ? 32 : 1];  // offset and factor of each lane's entry
+};
+
+template <int kTargets>
+__global__ void __launch_bounds__(kFp64Warps * 32, kTargets == 32 ? 8 : 10)
+    traverse_fp64_kernel(Workspace ws, TraversalParams p) {
+  constexpr int kLanes = 32 / kTargets;  // lanes per target
+  __shared__ Fp64Shared<kTargets> shared;
   DevScalars *sc = ws.sc;
   if (sc->error) return;
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tl = lane & (kTargets - 1), el = lane / kTargets;
+  ListShared &sh = shared.list[warp];
   const int n = ws.n;
   const int m = sc->n_nodes;
-  const int n_groups = p.group_mode ? sc->n_tgroups : (n + 31) >> 5;
-  const double g = p.g;
+  const int n_sets = sc->n_tgroups;
   long long inter = 0, tests = 0;
   bool singular = false;
   while (true) {
-    int grp = 0;
-    if (lane == 0) grp = (int)atomicAdd(&sc->work_counter, 1u);
-    grp = __shfl_sync(kFull, grp, 0);
-    if (grp >= n_groups) break;
-    const int g0 = p.group_mode ? ws.tstart[grp] : grp * 32;
-    const int g1 = p.group_mode ? ((grp + 1 < n_groups) ? ws.tstart[grp + 1] : n) : min(g0 + 32, n);
-    // a group larger than a warp is walked 32 targets at a time
-    for (int c0 = g0; c0 < g1; c0 += 32) {
-      const int c1 = min(c0 + 32, g1);
-      const int s = c0 + lane;
-      const bool valid = s < c1 && s < n;
-      double4 t = make_double4(0.0, 0.0, 0.0, 0.0);
-      if (valid) t = ws.pm4[s];
-      // a warp's targets belong to one system: walk that system's subtree
-      const int sys = ws.n_systems > 1 ? ws.psys[g0] : 0;
-      const int root = ws.root_pre[sys];
-      const int end = (root >= 0 && root < m) ? min(ws.node_meta[root].x, m) : 0;
-      const double soft = ws.sys_eps ? ws.sys_eps[sys] : p.soft;
-      const double soft2 = __dmul_rn(soft, soft);
+    int set = 0;
+    if (lane == 0) set = (int)atomicAdd(&sc->work_counter, 1u);
+    set = __shfl_sync(kFull, set, 0);
+    if (set >= n_sets) break;
+    const int g0 = ws.tstart[set];
+    const int g1 = min(set + 1 < n_sets ? ws.tstart[set + 1] : n, g0 + kTargets);
+    const int s = g0 + tl;
+    const bool valid = s < g1;
+    const double4 t = ws.pm4[valid ? s : g0];
+    // a warp's targets belong to one system: walk that system's subtree
+    const int sys = ws.n_systems > 1 ? ws.psys[g0] : 0;
+    const int root = ws.root_pre[sys];
+    set_target_box(sh, t, ws.sys_box[4 * sys + 3]);
+    const double soft = ws.sys_eps ? ws.sys_eps[sys] : p.soft;
+    const double soft2 = __dmul_rn(soft, soft);
+    // no squared distance of the system leaves inv_sqrt_core's range
+    const bool in_range = soft2 > 0x1p-900 && soft2 < 0x1p900 && ws.sys_box[4 * sys + 3] < 0x1p400;
+    int resume = valid ? 0 : INT_MAX;
+    unsigned count_inter = 0, count_tests = 0;
+    if constexpr (kTargets == 32) {
       double ax = 0.0, ay = 0.0, az = 0.0;
-      int resume = valid ? root : INT_MAX;
-      int node = __reduce_min_sync(kFull, resume);
-      while (node < end) {
-        // every record of the node in one round trip (warp-uniform address:
-        // one broadcast transaction each)
-        const int4 meta = ws.node_meta[node];
-        const double4 a = ws.node_a[node];
-        const double4 c = ws.node_c[node];
-        if (resume == node) {
-          if (meta.z > 0) {
-            // occupied leaf: exact sum over its particles, self excluded
-            // (barnes_hut.cu:204-257).  Two particles at a time: their square
-            // roots and divisions are independent and overlap; the sums
-            // still take them in the reference's order.
-            int k = 0;
-            for (; k + 1 < meta.z; k += 2) {
-              const int s0 = meta.y + k, s1 = s0 + 1;
-              const double4 q0 = ws.pm4[s0], q1 = ws.pm4[s1];
-              const double dx0 = __dsub_rn(q0.x, t.x), dy0 = __dsub_rn(q0.y, t.y), dz0 = __dsub_rn(q0.z, t.z);
-              const double dx1 = __dsub_rn(q1.x, t.x), dy1 = __dsub_rn(q1.y, t.y), dz1 = __dsub_rn(q1.z, t.z);
-              double f0, f1;
-              const bool ok0 = point_mass_factor(sqdist(dx0, dy0, dz0), q0.w, g, soft2, f0);
-              const bool ok1 = point_mass_factor(sqdist(dx1, dy1, dz1), q1.w, g, soft2, f1);
-              if (s0 != s && q0.w != 0.0) {
-                singular |= !ok0;
-                if (ok0) {
-                  ax = __fma_rn(f0, dx0, ax);
-                  ay = __fma_rn(f0, dy0, ay);
-                  az = __fma_rn(f0, dz0, az);
-                }
-                ++inter;
+      auto eval = [&](int count) {
+        for (int j = 0; j < count; j += 4) {
+          double dx[4], dy[4], dz[4], r2[4], f[4];
+          int pre[4], aux[4];
+          bool act[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const double4 v = sh.src[j + q];
+            const int2 tag = sh.tag[j + q];
+            pre[q] = tag.x;
+            aux[q] = tag.y;
+            dx[q] = __dsub_rn(v.x, t.x);
+            dy[q] = __dsub_rn(v.y, t.y);
+            dz[q] = __dsub_rn(v.z, t.z);
+            f[q] = v.w;
+            r2[q] = sqdist(dx[q], dy[q], dz[q]);
+            act[q] = pre[q] >= resume && aux[q] != s;
+          }
+          if (min(min(aux[0], aux[1]), min(aux[2], aux[3])) < -1) {
+            // undecided cells: a target that accepts one resumes past it
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              act[q] = act[q] && pre[q] >= resume;
+              if (aux[q] < -1) {
+                act[q] = act[q] && accept_entry(sh, j + q, ws, pre[q], t, r2[q]);
+                if (act[q]) resume = -aux[q];
               }
-              if (s1 != s && q1.w != 0.0) {
-                singular |= !ok1;
-                if (ok1) {
-                  ax = __fma_rn(f1, dx1, ax);
-                  ay = __fma_rn(f1, dy1, ay);
-                  az = __fma_rn(f1, dz1, az);
-                }
-                ++inter;
-              }
-            }
-            if (k < meta.z) {
-              const int sp = meta.y + k;
-              const double4 q = ws.pm4[sp];
-              if (sp != s && q.w != 0.0) {
-                const double dx = __dsub_rn(q.x, t.x), dy = __dsub_rn(q.y, t.y), dz = __dsub_rn(q.z, t.z);
-                singular |= !point_mass_fp64(dx, dy, dz, sqdist(dx, dy, dz), q.w, g, soft2, ax, ay, az);
-                ++inter;
-              }
-            }
-            resume = meta.x;
-          } else if (a.w == 0.0) {
-            resume = meta.x;  // zero-mass node (barnes_hut.cu:259-271)
-          } else {
-            double dx, dy, dz, d2;
-            const bool accept = accept_fp64(a, ws.node_b + node, c, t, dx, dy, dz, d2);
-            ++tests;
-            if (accept) {
-              singular |= !point_mass_fp64(dx, dy, dz, d2, a.w, g, soft2, ax, ay, az);
-              ++inter;
-              resume = meta.x;
-            } else {
-              resume = node + 1;
             }
           }
+          // all terms are formed before any is added; the sums take them in
+          // the reference's order
+          bool plain = in_range;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            r2[q] = __dadd_rn(r2[q], soft2);
+            plain = plain && __double2loint(r2[q]) != -1;
+          }
+          double inv[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) inv[q] = inv_sqrt_core(r2[q]);
+          if (!plain) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              inv[q] = inv_sqrt_general(r2[q]);
+              if (act[q] && r2[q] <= 0.0) {
+                singular = true;
+                act[q] = false;
+                ++count_inter;
+              }
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) f[q] = __dmul_rn(f[q], __dmul_rn(__dmul_rn(inv[q], inv[q]), inv[q]));
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (act[q]) {
+              ax = __fma_rn(f[q], dx[q], ax);
+              ay = __fma_rn(f[q], dy[q], ay);
+              az = __fma_rn(f[q], dz[q], az);
+              ++count_inter;
+            }
         }
-        // a lane's resume index always moves forward (skip > node); this keeps
-        // the walk finite whatever the node records hold
-        if (resume <= node) resume = node + 1;
-        node = __reduce_min_sync(kFull, resume);
-      }
+        return __reduce_min_sync(kFull, resume);
+      };
+      ordered_walk(ws, m, root, p.g, sh, count_tests, eval);
       if (valid) {
         const uint32_t ti = ws.idx[s];
         ws.ax[ti] = ax;
@@ -153,7 +169,67 @@ __global__ void __launch_bounds__(256) traverse_fp64_kernel(Workspace ws, Traver
           ws.vz[ti] = __fma_rn(p.half_dt, az, ws.vz[ti]);
         }
       }
+    } else {
+      // lane (el, tl): entry el of each block of kLanes, target tl; lanes
+      // el = 0, 1, 2 sum the x, y, z component
+      double acc = 0.0;
+      double4 *term = shared.term[warp];
+      const int comp = min(el, 2);
+      auto eval = [&](int count) {
+        for (int e0 = 0; e0 < count; e0 += kLanes) {
+          const bool has = e0 + el < count;
+          const int j = has ? e0 + el : e0;
+          const double4 q = sh.src[j];
+          const int2 tg = sh.tag[j];
+          const double dx = __dsub_rn(q.x, t.x), dy = __dsub_rn(q.y, t.y), dz = __dsub_rn(q.z, t.z);
+          const double d2 = sqdist(dx, dy, dz);
+          const bool undecided = has && tg.y < -1;
+          bool act = has && tg.x >= resume && tg.y != s;
+          if (__any_sync(kFull, undecided)) {
+            // the entries' decisions in order: each may move the resume
+            // index of the target's later entries
+            const bool take = act && (!undecided || accept_entry(sh, j, ws, tg.x, t, d2));
+            act = false;
+            for (int e = 0; e < kLanes; ++e) {
+              if (e == el) act = take && tg.x >= resume;
+              const int moved = (act && undecided) ? -tg.y : resume;
+              resume = __shfl_sync(kFull, moved, e * kTargets + tl);
+            }
+          }
+          const double r2 = __dadd_rn(d2, soft2);
+          double inv = inv_sqrt_core(r2);
+          if (!inv_sqrt_in_range(r2)) inv = inv_sqrt_general(r2);
+          const double f = __dmul_rn(q.w, __dmul_rn(__dmul_rn(inv, inv), inv));
+          const bool zero = r2 <= 0.0;
+          singular |= act && zero;
+          count_inter += act ? 1 : 0;
+          // an idle lane's term is 0, which leaves a sum's bits alone
+          const bool on = act && !zero;
+          term[lane] = make_double4(on ? dx : 0.0, on ? dy : 0.0, on ? dz : 0.0, on ? f : 0.0);
+          __syncwarp();
+#pragma unroll
+          for (int e = 0; e < kLanes; ++e) {
+            const double *v = reinterpret_cast<const double *>(term + e * kTargets + tl);
+            acc = __fma_rn(v[3], v[comp], acc);
+          }
+          __syncwarp();
+        }
+        return __reduce_min_sync(kFull, resume);
+      };
+      ordered_walk(ws, m, root, p.g, sh, count_tests, eval);
+      if (valid && el < 3) {
+        const uint32_t ti = ws.idx[s];
+        double *a = el == 0 ? ws.ax : (el == 1 ? ws.ay : ws.az);
+        a[ti] = acc;
+        if (p.kick) {
+          double *v = el == 0 ? ws.vx : (el == 1 ? ws.vy : ws.vz);
+          v[ti] = __fma_rn(p.half_dt, acc, v[ti]);
+        }
+      }
     }
+    inter += count_inter;
+    tests += count_tests;
+    __syncwarp();
   }
   if (__any_sync(kFull, singular) && lane == 0) record_error(sc, kStageTraversal, 6);
   inter = warp_sum_ll(inter);
@@ -569,7 +645,7 @@ __global__ void __launch_bounds__(kMixedWarps * 32,
   int *src = sh.src[wid];
   const int n = ws.n;
   const int m = sc->n_nodes;
-  const int n_groups = p.group_mode ? sc->n_tgroups : (n + 32 * kTPL - 1) / (32 * kTPL);
+  const int n_groups = sc->n_tgroups;
   const unsigned lt = lanemask_lt();
   int ccount = 0;
   if (p.cache_depth > 0 && ws.top && ws.n_systems == 1) {
@@ -603,8 +679,8 @@ __global__ void __launch_bounds__(kMixedWarps * 32,
     if (lane == 0) grp = (int)atomicAdd(&sc->work_counter, 1u);
     grp = __shfl_sync(kFull, grp, 0);
     if (grp >= n_groups) break;
-    const int g0 = p.group_mode ? ws.tstart[grp] : grp * 32 * kTPL;
-    const int g1 = p.group_mode ? ((grp + 1 < n_groups) ? ws.tstart[grp + 1] : n) : min(g0 + 32 * kTPL, n);
+    const int g0 = ws.tstart[grp];
+    const int g1 = (grp + 1 < n_groups) ? ws.tstart[grp + 1] : n;
     const int nq = min(kTPL, max(1, (g1 - g0 + 31) >> 5));  // occupied target slots
     LaneTargets<kTPL> T;
     LaneVjp V;
@@ -863,8 +939,9 @@ __global__ void __launch_bounds__(kMixedWarps * 32,
       if (ls + ltotal <= list_cap_of<kTrackSource>()) {
         const int base = ls + lexcl;
         double4 q0 = make_double4(0.0, 0.0, 0.0, 0.0), q1 = q0;
-        if (lc0 > 0) q0 = ws.pm4[m0.y];
-        if (lc1 > 0) q1 = ws.pm4[m1.y];
+        // a leaf's record carries its first particle
+        if (lc0 > 0) q0 = a0;
+        if (lc1 > 0) q1 = a1;
         if (lc0 > 0) {
           list.put(base, (float)(q0.x - gbox[6]), (float)(q0.y - gbox[7]), (float)(q0.z - gbox[8]), (float)q0.w);
           if (kTrackSource) src[base] = m0.y;
@@ -1293,7 +1370,8 @@ static cudaError_t grid_of(K kernel, int threads, int sms, int &grid) {
 
 cudaError_t configure_traversal(Workspace &ws) {
   const int sms = ws.num_sms > 0 ? ws.num_sms : 148;
-  cudaError_t e = grid_of(traverse_fp64_kernel, 256, sms, ws.fp64_grid);
+  cudaError_t e = grid_of(traverse_fp64_kernel<32>, kFp64Warps * 32, sms, ws.fp64_grid[0]);
+  if (e == cudaSuccess) e = grid_of(traverse_fp64_kernel<1>, kFp64Warps * 32, sms, ws.fp64_grid[1]);
   if (e == cudaSuccess) e = grid_of(traverse_mixed_kernel<false, 1>, kMixedWarps * 32, sms, ws.mixed_grid[0][0]);
   if (e == cudaSuccess) e = grid_of(traverse_mixed_kernel<true, 1>, kMixedWarps * 32, sms, ws.mixed_grid[1][0]);
   if (e == cudaSuccess) e = grid_of(traverse_mixed_kernel<false, 2>, kMixedWarps * 32, sms, ws.mixed_grid[0][1]);
@@ -1317,12 +1395,15 @@ cudaError_t configure_traversal(Workspace &ws) {
 
 cudaError_t launch_traversal(Workspace &ws, const TraversalParams &p, cudaStream_t s) {
   // target slots per lane: 1, 2 or 4 for groups of at most 32, 64 or 128
-  const int slot = !p.group_mode ? 0 : (p.group_size > 64 ? 2 : (p.group_size > 32 ? 1 : 0));
+  const int slot = p.group_size > 64 ? 2 : (p.group_size > 32 ? 1 : 0);
   const int track = p.soft > 0.0 ? 0 : 1;
   const int grid = ws.mixed_grid[track][slot] > 0 ? ws.mixed_grid[track][slot] : 148;
-  if (p.precision == 0)
-    traverse_fp64_kernel<<<ws.fp64_grid > 0 ? ws.fp64_grid : 148, 256, 0, s>>>(ws, p);
-  else if (slot == 0)
+  if (p.precision == 0) {
+    if (p.targets > 1)
+      traverse_fp64_kernel<32><<<ws.fp64_grid[0] > 0 ? ws.fp64_grid[0] : 148, kFp64Warps * 32, 0, s>>>(ws, p);
+    else
+      traverse_fp64_kernel<1><<<ws.fp64_grid[1] > 0 ? ws.fp64_grid[1] : 148, kFp64Warps * 32, 0, s>>>(ws, p);
+  } else if (slot == 0)
     (track ? traverse_mixed_kernel<true, 1> : traverse_mixed_kernel<false, 1>)<<<grid, kMixedWarps * 32, 0, s>>>(
         ws, p, AdjointBuffers{});
   else if (slot == 1)

@@ -7,16 +7,56 @@
 
 namespace nbb {
 
+// 1 / sqrt(x), square root and reciprocal each correctly rounded (the bits of
+// __drcp_rn(__dsqrt_rn(x))), for x in [2^-927, 2^993): one hardware estimate
+// shared by both and the residual corrections of Markstein ("Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990), 10 FP64
+// operations.
+//   y0      the estimate, 20 bits, so y0^2 is exact; r = 1 - x y0^2 is rounded
+//           once and |r| < 2^-18
+//   y       y0 (1 + r/2 + 3/8 r^2): relative error 2^-53 from its rounding,
+//           5/16 |r|^3 < 2^-55.6 from the series
+//   g, d    x y and the exact residual x - g^2
+//   s       g + d y/2, in error by less than 2^-103.5 sqrt(x) before its
+//           rounding
+//   e, 1/s  y + y (1 - s y), in error by less than 2^-103.5 / s before its
+//           rounding
+// A result rounds wrongly only when the exact value lies that close to the
+// middle of two neighbours.  For the square root that takes an x with
+// m^2 - x = k 2^-106 (|k| < 48, m the middle, sqrt(x) in [1, 2)), for the
+// reciprocal an s with s m - 1 = k 2^-106 (|k| < 8); both sets are small and
+// were enumerated and checked one by one: only s = 2 - 2^-52 comes out wrong
+// (Markstein's exception), and inv_sqrt_in_range leaves it to the general
+// form.
+__device__ __forceinline__ double inv_sqrt_core(double x) {
+  double y0;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(x));
+  const double r = __fma_rn(-x, __dmul_rn(y0, y0), 1.0);
+  const double y = __fma_rn(__fma_rn(r, 0.375, 0.5), __dmul_rn(y0, r), y0);
+  const double g = __dmul_rn(x, y);
+  const double d = __fma_rn(-g, g, x);
+  const double half_y = __hiloint2double(__double2hiint(y) - 0x00100000, __double2loint(y));
+  const double s = __fma_rn(d, half_y, g);
+  return __fma_rn(__fma_rn(-s, y, 1.0), y, y);
+}
+// Whether inv_sqrt_core gives the right bits for x: its range, without the
+// one significand that rounds wrongly (all ones, whose root is all ones too).
+__device__ __forceinline__ bool inv_sqrt_in_range(double x) {
+  return (unsigned)(__double2hiint(x) - 0x06000000) < 0x78000000u && __double2loint(x) != -1;
+}
+static __device__ __noinline__ double inv_sqrt_general(double x) { return __drcp_rn(__dsqrt_rn(x)); }
+
 // barnes_hut.cu:56-80, the factor G m (d^2 + eps^2)^-3/2 with the
 // reference's operation order.  The reference's 1.0 / sqrt(r2) is a
-// correctly rounded division of 1, which is the correctly rounded reciprocal
-// (__drcp_rn, a shorter sequence than the general division): the same bits
-// for every input.  Returns false on a singular interaction.
-__device__ __forceinline__ bool point_mass_factor(double d2, double m, double g, double soft2, double &f) {
+// correctly rounded division of 1, which is the correctly rounded reciprocal:
+// the same bits for every input.  Returns false on a singular interaction.
+// gm is the product G m.
+__device__ __forceinline__ bool scaled_mass_factor(double d2, double gm, double soft2, double &f) {
   const double r2 = __dadd_rn(d2, soft2);
-  const double inv = __drcp_rn(__dsqrt_rn(r2));
+  double inv = inv_sqrt_core(r2);
+  if (!inv_sqrt_in_range(r2)) inv = inv_sqrt_general(r2);
   const double inv3 = __dmul_rn(__dmul_rn(inv, inv), inv);
-  f = __dmul_rn(__dmul_rn(g, m), inv3);
+  f = __dmul_rn(gm, inv3);
   return !(r2 <= 0.0);
 }
 
@@ -26,7 +66,7 @@ __device__ __forceinline__ bool point_mass_fp64(double dx, double dy, double dz,
                                                 double m, double g, double soft2, double &ax,
                                                 double &ay, double &az) {
   double f;
-  if (!point_mass_factor(d2, m, g, soft2, f)) return false;
+  if (!scaled_mass_factor(d2, __dmul_rn(g, m), soft2, f)) return false;
   ax = __fma_rn(f, dx, ax);
   ay = __fma_rn(f, dy, ay);
   az = __fma_rn(f, dz, az);
