@@ -19,6 +19,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <utility>
 #include <vector>
 
 namespace nbb {
@@ -167,10 +168,42 @@ struct Allocation {
   }
 };
 
-// Allocate every buffer of a workspace for n particles (state included when
-// with_state).  All device memory is taken here; nothing is allocated later.
-cudaError_t alloc_workspace(Workspace &ws, Allocation &al, int n, bool with_state, int n_systems = 1,
-                            bool level_order = false) {
+// Arrays taken together from one device allocation: an allocation and its
+// release cost about 0.2 ms whatever the size, and a workspace has 70 arrays
+// (15 ms of creating a 65536-particle simulation, and nearly all of a one-shot
+// force evaluation).
+struct Arena {
+  std::vector<std::pair<void **, size_t>> parts;
+  size_t bytes = 0;
+  template <typename T>
+  void add(T *&out, size_t count) {
+    parts.emplace_back(reinterpret_cast<void **>(&out), bytes);
+    bytes += ((count > 0 ? count : 1) * sizeof(T) + 255) & ~(size_t)255;
+  }
+  cudaError_t take(Allocation &al) {
+    char *base = nullptr;
+    const cudaError_t e = al.get(base, bytes);
+    if (e != cudaSuccess) return e;
+    for (const auto &p : parts) *p.first = base + p.second;
+    return cudaSuccess;
+  }
+};
+
+// Which arrays a workspace has: all of them (a simulation steps the
+// level-order octree and exports the reference-numbered one), or those of one
+// force evaluation.
+struct WorkspaceParts {
+  bool state = true;         // the particles
+  bool motion = true;        // their velocities and types
+  bool reference = true;     // the reference-numbered build
+  bool level_order = false;  // the level-order build
+  bool cache = false;        // the mixed walk's node-cache table
+  int records = kRecordsFp64 | kRecordsMixed;
+};
+
+// Allocate every buffer of a workspace for n particles.  All device memory is
+// taken here; nothing is allocated later.
+cudaError_t alloc_workspace(Workspace &ws, Allocation &al, int n, const WorkspaceParts &parts, int n_systems = 1) {
   ws = Workspace{};
   ws.n = n;
   ws.n_systems = n_systems;
@@ -184,17 +217,19 @@ cudaError_t alloc_workspace(Workspace &ws, Allocation &al, int n, bool with_stat
   int dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&ws.num_sms, cudaDevAttrMultiProcessorCount, dev);
-  const size_t N = (size_t)n, C = (size_t)ws.cap_nodes;
-  cudaError_t e = cudaSuccess;
-#define GET(ptr, cnt) \
-  if ((e = al.get(ptr, cnt)) != cudaSuccess) return e
-  if (with_state) {
+  cudaError_t e = configure_traversal(ws);
+  if (e != cudaSuccess) return e;
+  const size_t N = (size_t)n, C = (size_t)ws.cap_nodes, S = (size_t)n_systems;
+  Arena ar;
+#define GET(ptr, cnt) ar.add(ptr, cnt)
+  if (parts.state) {
     GET(ws.m, N); GET(ws.x, N); GET(ws.y, N); GET(ws.z, N);
-    GET(ws.vx, N); GET(ws.vy, N); GET(ws.vz, N);
     GET(ws.ax, N); GET(ws.ay, N); GET(ws.az, N);
+  }
+  if (parts.state && parts.motion) {
+    GET(ws.vx, N); GET(ws.vy, N); GET(ws.vz, N);
     GET(ws.type, N);
   }
-  const size_t S = (size_t)n_systems;
   if (n_systems > 1) {
     GET(ws.sys_of, N);
     GET(ws.sys_eps, S);
@@ -210,35 +245,39 @@ cudaError_t alloc_workspace(Workspace &ws, Allocation &al, int n, bool with_stat
   GET(ws.scan_status, (size_t)(3 * ws.scan_tiles_n + ws.scan_tiles_r));
   GET(ws.keys, N); GET(ws.idx, N); GET(ws.pm4, N); GET(ws.psys, N);
   GET(ws.ukey, N); GET(ws.uniq, N); GET(ws.gfirst, N); GET(ws.gcount, N); GET(ws.glast, N);
-  GET(ws.left, N); GET(ws.right, N); GET(ws.rfirst, N); GET(ws.rlast, N); GET(ws.plen, N);
-  GET(ws.rparent, 2 * N);
-  GET(ws.plevel, 2 * N); GET(ws.pcount, 2 * N); GET(ws.poffset, 2 * N);
-  GET(ws.children, 8 * C);
-  GET(ws.oparent, C); GET(ws.olevel, C); GET(ws.oprefix, C); GET(ws.ofirst, C); GET(ws.ocount, C);
-  GET(ws.child_count, C); GET(ws.pre_of, C); GET(ws.by_level, C); GET(ws.subtree, C); GET(ws.preoff, C);
-  GET(ws.psub, C); GET(ws.pfirst, C); GET(ws.pends, N);
   GET(ws.tflag, N); GET(ws.tstart, N);
-  GET(ws.cx, C); GET(ws.cy, C); GET(ws.cz, C); GET(ws.half, C);
-  GET(ws.mass, C); GET(ws.comx, C); GET(ws.comy, C); GET(ws.comz, C);
-  GET(ws.node_a, C); GET(ws.node_b, C); GET(ws.node_c, C); GET(ws.node_meta, C);
+  if (parts.reference) {
+    GET(ws.left, N); GET(ws.right, N); GET(ws.rfirst, N); GET(ws.rlast, N); GET(ws.plen, N);
+    GET(ws.rparent, 2 * N);
+    GET(ws.plevel, 2 * N); GET(ws.pcount, 2 * N); GET(ws.poffset, 2 * N);
+    GET(ws.children, 8 * C);
+    GET(ws.oparent, C); GET(ws.olevel, C); GET(ws.oprefix, C); GET(ws.ofirst, C); GET(ws.ocount, C);
+    GET(ws.child_count, C); GET(ws.pre_of, C); GET(ws.by_level, C); GET(ws.subtree, C); GET(ws.preoff, C);
+    GET(ws.psub, C); GET(ws.pfirst, C); GET(ws.pends, N);
+    GET(ws.cx, C); GET(ws.cy, C); GET(ws.cz, C); GET(ws.half, C);
+    GET(ws.mass, C); GET(ws.comx, C); GET(ws.comy, C); GET(ws.comz, C);
+  }
+  if (parts.records & kRecordsFp64) {
+    GET(ws.node_a, C); GET(ws.node_b, C); GET(ws.node_c, C); GET(ws.node_meta, C);
+  }
+  if (parts.records & kRecordsMixed) {
+    GET(ws.node_m, C);
+    GET(ws.walk_ext, (size_t)ws.walk_warps * ws.walk_ext_cap);
+  }
   GET(ws.node_kids, 8 * C);
-  GET(ws.node_m, C);
-  if (level_order) {
+  if (parts.level_order) {
     ws.level_order = 1;
     GET(ws.gspan, N);
     GET(ws.lo_first, C); GET(ws.lo_arrive, C); GET(ws.lo_last, C); GET(ws.lo_node, C); GET(ws.lo_gleaf, N);
     GET(ws.pos4, N);
     GET(ws.lo_tiles, (size_t)ws.scan_tiles_n * kLevelOrderChannels);
-    GET(ws.top, (size_t)kTopMax);
   }
+  if (parts.cache) GET(ws.top, (size_t)kTopMax);
 #undef GET
-  e = cudaMemset(ws.sc, 0, sizeof(DevScalars));
-  if (e != cudaSuccess) return e;
-  e = cudaMemset(ws.root_pre, 0, S * sizeof(int));
-  if (e != cudaSuccess) return e;
-  e = configure_traversal(ws);
-  if (e != cudaSuccess) return e;
-  return al.get(ws.walk_ext, (size_t)ws.walk_warps * ws.walk_ext_cap);
+  e = ar.take(al);
+  if (e == cudaSuccess) e = cudaMemset(ws.sc, 0, sizeof(DevScalars));
+  if (e == cudaSuccess) e = cudaMemset(ws.root_pre, 0, S * sizeof(int));
+  return e;
 }
 
 bool finite_nonneg(double v) { return std::isfinite(v) && v >= 0.0; }
@@ -382,10 +421,10 @@ cudaError_t stage_in(const T *src, size_t count, bool on_device, Allocation &al,
 // Device storage of a recorded rollout: (x, v, a) every `every` steps, the
 // final state, one segment of recomputed positions and the reverse-mode
 // buffers.  Taken when the rollout starts, released with the handle or by
-// the next rollout.
+// the next rollout of another length.
 struct RolloutRecord {
   Allocation al;
-  uint64_t steps = 0, every = 0, slots = 0;
+  uint64_t steps = 0, every = 0, slots = 0, seg_slots = 0;
   double *ckpt = nullptr;         // slots x 9 x n: x y z vx vy vz ax ay az
   double *final_state = nullptr;  // 9 x n
   double *seg = nullptr;          // (every - 1) x 3 x n recomputed positions
@@ -564,7 +603,9 @@ static int create_sim(const nbb_config *cfg, size_t n, int n_systems, const int6
   sim->cfg = *cfg;
   sim->min_softening = min_eps;
   cudaError_t e = cudaStreamCreateWithFlags(&sim->own_stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = alloc_workspace(sim->ws, sim->alloc, (int)n, true, n_systems > 1 ? n_systems : 1, true);
+  WorkspaceParts parts;
+  parts.level_order = parts.cache = true;
+  if (e == cudaSuccess) e = alloc_workspace(sim->ws, sim->alloc, (int)n, parts, n_systems > 1 ? n_systems : 1);
   if (e != cudaSuccess) {
     if (sim->own_stream) cudaStreamDestroy(sim->own_stream);
     delete sim;
@@ -1091,7 +1132,14 @@ int nbb_accel(size_t n, const double *mass, const double *x, const double *y, co
     return fail(NBB_ERR_INVALID_ARGUMENT, "Unknown traversal precision");
   Scratch sc;
   NBB_CUDA(cudaStreamCreateWithFlags(&sc.s, cudaStreamNonBlocking), "create stream");
-  NBB_CUDA(alloc_workspace(sc.ws, sc.al, (int)n, true), "allocate workspace");
+  // the octree in the reference's numbering only when it is exported; the
+  // level-order build gives the same records with fewer passes
+  WorkspaceParts parts;
+  parts.motion = false;
+  parts.reference = export_out != nullptr;
+  parts.level_order = !parts.reference;
+  if (parts.level_order) parts.records = precision == NBB_PRECISION_MIXED ? kRecordsMixed : kRecordsFp64;
+  NBB_CUDA(alloc_workspace(sc.ws, sc.al, (int)n, parts), "allocate workspace");
   Workspace &ws = sc.ws;
   const cudaMemcpyKind in = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   const size_t bytes = n * sizeof(double);
@@ -1267,7 +1315,9 @@ int nbb_octree_from_keys(const uint32_t *sorted_keys, int n, nbb_tree_export *ou
   if (!sorted_keys || !out) return fail(NBB_ERR_INVALID_ARGUMENT, "d_sortedKeys must not be null");
   Scratch sc;
   NBB_CUDA(cudaStreamCreateWithFlags(&sc.s, cudaStreamNonBlocking), "create stream");
-  NBB_CUDA(alloc_workspace(sc.ws, sc.al, n, false), "allocate workspace");
+  WorkspaceParts parts;
+  parts.state = false;
+  NBB_CUDA(alloc_workspace(sc.ws, sc.al, n, parts), "allocate workspace");
   sc.ws.pack_shift = 32;  // caller keys may use all 32 bits (rejected by the plan)
   uint32_t *dk = nullptr;
   NBB_CUDA(sc.al.get(dk, (size_t)n), "allocate keys");
@@ -1694,19 +1744,25 @@ int nbb_sim_rollout(nbb_sim *sim, uint64_t steps, uint64_t checkpoint_every) {
   const uint64_t seg = std::min<uint64_t>(checkpoint_every, steps > 0 ? steps : 1) - 1;
   const double need = 8.0 * (double)n * (kStateArrays * (double)(slots + 1) + 3.0 * (double)seg + 7.0);
   if (need > 0x1p46) return fail(NBB_ERR_INVALID_ARGUMENT, "rollout checkpoints exceed device memory");
-  sim->rollout.reset();
-  auto rec = std::make_unique<RolloutRecord>();
-  Allocation &al = rec->al;
-  cudaError_t e = al.get(rec->ckpt, (size_t)slots * kStateArrays * n);
-  if (e == cudaSuccess) e = al.get(rec->final_state, kStateArrays * n);
-  if (e == cudaSuccess) e = al.get(rec->seg, (size_t)(seg > 0 ? seg : 1) * 3 * n);
-  if (e == cudaSuccess) e = al.get(rec->g, 7 * n);
-  if (e == cudaSuccess) e = al.get(rec->node_g, (size_t)ws.cap_nodes);
-  if (e == cudaSuccess) e = al.get(rec->part_g, n);
-  if (e == cudaSuccess) e = al.get(rec->tgt_g, n);
-  if (e == cudaSuccess) e = al.get(rec->pparent, (size_t)ws.cap_nodes);
-  if (e == cudaSuccess) e = al.get(rec->prange, (size_t)ws.cap_nodes);
-  if (e != cudaSuccess) return cuda_fail(e, "rollout checkpoint allocation");
+  // a rollout as long as the last one takes over its buffers
+  std::unique_ptr<RolloutRecord> rec = std::move(sim->rollout);
+  cudaError_t e = cudaSuccess;
+  if (!rec || rec->slots != slots || rec->seg_slots != seg) {
+    rec.reset();
+    rec = std::make_unique<RolloutRecord>();
+    Arena ar;
+    ar.add(rec->ckpt, (size_t)slots * kStateArrays * n);
+    ar.add(rec->final_state, kStateArrays * n);
+    ar.add(rec->seg, (size_t)(seg > 0 ? seg : 1) * 3 * n);
+    ar.add(rec->g, 7 * n);
+    ar.add(rec->node_g, (size_t)ws.cap_nodes);
+    ar.add(rec->part_g, n);
+    ar.add(rec->tgt_g, n);
+    ar.add(rec->pparent, (size_t)ws.cap_nodes);
+    ar.add(rec->prange, (size_t)ws.cap_nodes);
+    e = ar.take(rec->al);
+    if (e != cudaSuccess) return cuda_fail(e, "rollout checkpoint allocation");
+  }
   if (steps > 0 && sim->cfg.use_graph && !sim->step_graph) e = capture_step(sim);
   if (e == cudaSuccess) e = copy_state(sim, rec->ckpt, kStateArrays, true);
   for (uint64_t k = 0; k < steps && e == cudaSuccess; ++k) {
@@ -1727,6 +1783,7 @@ int nbb_sim_rollout(nbb_sim *sim, uint64_t steps, uint64_t checkpoint_every) {
   rec->steps = steps;
   rec->every = checkpoint_every;
   rec->slots = slots;
+  rec->seg_slots = seg;
   sim->rollout = std::move(rec);
   sim->time += sim->cfg.time_step * (double)steps;
   sim->steps += steps;
