@@ -22,9 +22,10 @@
 // over each node's particles.
 //
 //   adj_topology_kernel  preorder parent and Morton particle range per node
-//   adjoint_walk_kernel  the plain walk's visit order, vector-Jacobian products;
+//   adj_parent_kernel    preorder parents from a level-order build
+//   adjoint_walk_kernel  the plain walk's interactions, vector-Jacobian products;
 //                        node / particle cotangents reduced across the warp
-//                        (all lanes at a node share it) and added atomically
+//                        and added atomically
 //   adj_node_kernel      (gX, gM) -> (P, Q) per node
 //   adj_leaf_kernel      root-path sums, per-particle totals, velocity update
 //   frozen_*             the force on perturbed copies of the particles with
@@ -34,6 +35,7 @@
 //   direct_vjp_kernel    adjoint of the FP64 direct sum (all pairs)
 #include "nbb_internal.cuh"
 #include "walk_fp64.cuh"
+#include "walk_list.cuh"
 
 #include <climits>
 #include <cmath>
@@ -52,49 +54,26 @@ inline int grid_of_ws(const Workspace &ws, int per_sm) {
 
 // u and the mass term of one interaction (see the file comment).
 __device__ __forceinline__ bool vjp_pair(double dx, double dy, double dz, double d2, double mu, double g,
-                                         double soft2, double cx, double cy, double cz, double &ux,
-                                         double &uy, double &uz, double &uw) {
+                                         double soft2, double cx, double cy, double cz, double (&u)[4]) {
   const double r2 = d2 + soft2;
-  if (!(r2 > 0.0)) {
-    ux = uy = uz = uw = 0.0;
-    return false;
+  double inv = inv_sqrt_core(r2);
+  if (!inv_sqrt_in_range(r2)) {
+    if (!(r2 > 0.0)) {
+      u[0] = u[1] = u[2] = u[3] = 0.0;
+      return false;
+    }
+    inv = inv_sqrt_general(r2);
   }
-  const double inv = 1.0 / sqrt(r2);
   const double inv2 = inv * inv;
   const double gi3 = g * inv2 * inv;
   const double rc = dx * cx + dy * cy + dz * cz;
   const double f = gi3 * mu;
   const double h = 3.0 * f * inv2 * rc;
-  ux = f * cx - h * dx;
-  uy = f * cy - h * dy;
-  uz = f * cz - h * dz;
-  uw = gi3 * rc;
+  u[0] = f * cx - h * dx;
+  u[1] = f * cy - h * dy;
+  u[2] = f * cz - h * dz;
+  u[3] = gi3 * rc;
   return true;
-}
-
-// Add (ux, uy, uz, uw) of the lanes in `who` (warp-uniform ballot; other
-// lanes hold zeros) to dst: one lane's values directly, otherwise a butterfly
-// sum and lanes 0..3 each add one component.
-__device__ __forceinline__ void scatter4(double4 *dst, unsigned who, int lane, double ux, double uy,
-                                         double uz, double uw) {
-  double *d = reinterpret_cast<double *>(dst);
-  if (__popc(who) == 1) {
-    if (lane == __ffs(who) - 1) {
-      atomicAdd(d + 0, ux);
-      atomicAdd(d + 1, uy);
-      atomicAdd(d + 2, uz);
-      atomicAdd(d + 3, uw);
-    }
-    return;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    ux += __shfl_xor_sync(kFull, ux, o);
-    uy += __shfl_xor_sync(kFull, uy, o);
-    uz += __shfl_xor_sync(kFull, uz, o);
-    uw += __shfl_xor_sync(kFull, uw, o);
-  }
-  const double v = (lane == 0) ? ux : (lane == 1) ? uy : (lane == 2) ? uz : uw;
-  if (lane < 4) atomicAdd(d + lane, v);
 }
 
 __global__ void adj_reset_kernel(DevScalars *sc) {
@@ -128,126 +107,172 @@ __global__ void __launch_bounds__(kBlock) adj_topology_kernel(Workspace ws, int 
   }
 }
 
-// Vector-Jacobian product of the frozen-structure force: the plain walk's
-// node sequence per lane (same records, same acceptance test), with the
-// accelerations cotangent coef * gv of each target.
-__global__ void __launch_bounds__(256) adjoint_walk_kernel(Workspace ws, TraversalParams p, AdjointBuffers ab) {
+// The same parents from a level-order build: a cell's parent is an index of
+// the same numbering.
+__global__ void __launch_bounds__(kBlock) adj_parent_kernel(Workspace ws, int *pparent) {
   DevScalars *sc = ws.sc;
   if (sc->error) return;
-  const int lane = threadIdx.x & 31;
+  const int m = sc->n_nodes;
+  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < m; b += gridDim.x * blockDim.x) {
+    const int pre = ws.lo_node[b].pre, p = ws.lo_first[b].w;
+    if (pre < 0 || pre >= m || p >= m || (p < 0) != (b == 0)) {
+      record_error(sc, kStageLayout, 1);
+      continue;
+    }
+    pparent[pre] = p < 0 ? -1 : ws.lo_node[p].pre;
+  }
+}
+
+// Vector-Jacobian product of the frozen-structure force: the plain walk's
+// interactions (the ordered lists of walk_list.cuh, every target's own
+// decisions) with the accelerations cotangent coef * gv of each target.
+//
+// kTargets lanes hold one target each and 32 / kTargets lanes share a target,
+// so a block of four entries is four per lane or one.  A source's u is summed
+// over the warp's targets before it is added (FP64 atomics): the block's 16
+// components go to shared memory, a row per target, and each lane adds half a
+// column -- 12 instructions per entry, against 60 of a shuffle butterfly per
+// component.  The walk that took one node at a time was bound by that
+// reduction's latency after each node's; a vector-Jacobian product (rebuild
+// and walk) takes 1.2 ms at 16384 particles where that took 3.2, and 2.6 at
+// 65536 (4.3).
+constexpr int kAdjWarps = 2;
+constexpr int kAdjBlock = 4;   // entries reduced together
+constexpr int kAdjRow = 4 * kAdjBlock + 1;
+
+template <int kTargets>
+struct AdjShared {
+  ListShared list[kAdjWarps];
+  double sum[kAdjWarps][kTargets * kAdjRow];
+};
+
+template <int kTargets>
+__global__ void __launch_bounds__(kAdjWarps * 32, 7)
+    adjoint_walk_kernel(Workspace ws, TraversalParams p, AdjointBuffers ab) {
+  constexpr int kLanes = 32 / kTargets;            // lanes per target
+  constexpr int kPerLane = kAdjBlock / kLanes;     // entries of a block per lane
+  static_assert(kLanes * kPerLane == kAdjBlock, "a block of entries");
+  __shared__ AdjShared<kTargets> shared;
+  DevScalars *sc = ws.sc;
+  if (sc->error) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tl = lane & (kTargets - 1), el = lane / kTargets;
+  ListShared &sh = shared.list[warp];
+  double *sum = shared.sum[warp];
   const int n = ws.n;
   const int m = sc->n_nodes;
-  const int n_groups = sc->n_tgroups;
+  const int n_sets = sc->n_tgroups;
   const double g = p.g;
   bool singular = false;
   while (true) {
-    int grp = 0;
-    if (lane == 0) grp = (int)atomicAdd(&sc->work_counter, 1u);
-    grp = __shfl_sync(kFull, grp, 0);
-    if (grp >= n_groups) break;
-    const int g0 = ws.tstart[grp];
-    const int g1 = (grp + 1 < n_groups) ? ws.tstart[grp + 1] : n;
-    // a group larger than a warp is walked 32 targets at a time
-    for (int c0 = g0; c0 < g1; c0 += 32) {
-      const int c1 = min(c0 + 32, g1);
-      const int s = c0 + lane;
-      const bool valid = s < c1 && s < n;
-      double4 t = make_double4(0.0, 0.0, 0.0, 0.0);
-      double cx = 0.0, cy = 0.0, cz = 0.0;
-      if (valid) {
-        t = ws.pm4[s];
-        const uint32_t ti = ws.idx[s];
-        cx = ab.coef * ab.gvx[ti];
-        cy = ab.coef * ab.gvy[ti];
-        cz = ab.coef * ab.gvz[ti];
-      }
-      const int sys = ws.n_systems > 1 ? ws.psys[g0] : 0;
-      const int root = ws.root_pre[sys];
-      const int end = (root >= 0 && root < m) ? min(ws.node_meta[root].x, m) : 0;
-      const double soft = ws.sys_eps ? ws.sys_eps[sys] : p.soft;
-      const double soft2 = __dmul_rn(soft, soft);
-      double gtx = 0.0, gty = 0.0, gtz = 0.0;
-      int resume = valid ? root : INT_MAX;
-      int node = __reduce_min_sync(kFull, resume);
-      while (node < end) {
-        const int4 meta = ws.node_meta[node];
-        const double4 a = ws.node_a[node];
-        const bool here = resume == node;
-        if (meta.z > 0) {
-          // two particles at a time: both products are formed (independent
-          // square roots and divisions) before they are added and scattered
-          // in particle order
-          int k = 0;
-          for (; k + 1 < meta.z; k += 2) {
-            const int s0 = meta.y + k, s1 = s0 + 1;
-            const double4 q0 = ws.pm4[s0], q1 = ws.pm4[s1];
-            const bool act0 = here && s0 != s && q0.w != 0.0;
-            const bool act1 = here && s1 != s && q1.w != 0.0;
-            double u0x = 0.0, u0y = 0.0, u0z = 0.0, u0w = 0.0, u1x = 0.0, u1y = 0.0, u1z = 0.0, u1w = 0.0;
-            if (act0) {
-              const double dx = __dsub_rn(q0.x, t.x), dy = __dsub_rn(q0.y, t.y), dz = __dsub_rn(q0.z, t.z);
-              singular |= !vjp_pair(dx, dy, dz, sqdist(dx, dy, dz), q0.w, g, soft2, cx, cy, cz, u0x, u0y, u0z, u0w);
-            }
-            if (act1) {
-              const double dx = __dsub_rn(q1.x, t.x), dy = __dsub_rn(q1.y, t.y), dz = __dsub_rn(q1.z, t.z);
-              singular |= !vjp_pair(dx, dy, dz, sqdist(dx, dy, dz), q1.w, g, soft2, cx, cy, cz, u1x, u1y, u1z, u1w);
-            }
-            if (act0) {
-              gtx -= u0x;
-              gty -= u0y;
-              gtz -= u0z;
-            }
-            const unsigned who0 = __ballot_sync(kFull, act0);
-            if (who0) scatter4(ab.part_g + s0, who0, lane, u0x, u0y, u0z, u0w);
-            if (act1) {
-              gtx -= u1x;
-              gty -= u1y;
-              gtz -= u1z;
-            }
-            const unsigned who1 = __ballot_sync(kFull, act1);
-            if (who1) scatter4(ab.part_g + s1, who1, lane, u1x, u1y, u1z, u1w);
-          }
-          if (k < meta.z) {
-            const int sp = meta.y + k;
-            const double4 q = ws.pm4[sp];
-            const bool act = here && sp != s && q.w != 0.0;
-            double ux = 0.0, uy = 0.0, uz = 0.0, uw = 0.0;
-            if (act) {
-              const double dx = __dsub_rn(q.x, t.x), dy = __dsub_rn(q.y, t.y), dz = __dsub_rn(q.z, t.z);
-              singular |= !vjp_pair(dx, dy, dz, sqdist(dx, dy, dz), q.w, g, soft2, cx, cy, cz, ux, uy, uz, uw);
-              gtx -= ux;
-              gty -= uy;
-              gtz -= uz;
-            }
-            const unsigned who = __ballot_sync(kFull, act);
-            if (who) scatter4(ab.part_g + sp, who, lane, ux, uy, uz, uw);
-          }
-          if (here) resume = meta.x;
-        } else if (a.w == 0.0) {
-          if (here) resume = meta.x;
-        } else {
-          const double4 c = ws.node_c[node];
-          bool acc = false;
-          double ux = 0.0, uy = 0.0, uz = 0.0, uw = 0.0;
-          if (here) {
-            double dx, dy, dz, d2;
-            acc = accept_fp64(a, ws.node_b + node, c, t, dx, dy, dz, d2);
-            if (acc) {
-              singular |= !vjp_pair(dx, dy, dz, d2, a.w, g, soft2, cx, cy, cz, ux, uy, uz, uw);
-              gtx -= ux;
-              gty -= uy;
-              gtz -= uz;
-            }
-            resume = acc ? meta.x : node + 1;
-          }
-          const unsigned who = __ballot_sync(kFull, acc);
-          if (who) scatter4(ab.node_g + node, who, lane, ux, uy, uz, uw);
-        }
-        if (resume <= node) resume = node + 1;
-        node = __reduce_min_sync(kFull, resume);
-      }
-      if (valid) ab.tgt_g[s] = make_double4(gtx, gty, gtz, 0.0);
+    int set = 0;
+    if (lane == 0) set = (int)atomicAdd(&sc->work_counter, 1u);
+    set = __shfl_sync(kFull, set, 0);
+    if (set >= n_sets) break;
+    const int g0 = ws.tstart[set];
+    const int g1 = min(set + 1 < n_sets ? ws.tstart[set + 1] : n, g0 + kTargets);
+    const int s = g0 + tl;
+    const bool valid = s < g1;
+    const double4 t = ws.pm4[valid ? s : g0];
+    double cx = 0.0, cy = 0.0, cz = 0.0;
+    if (valid) {
+      const uint32_t ti = ws.idx[s];
+      cx = ab.coef * ab.gvx[ti];
+      cy = ab.coef * ab.gvy[ti];
+      cz = ab.coef * ab.gvz[ti];
     }
+    const int sys = ws.n_systems > 1 ? ws.psys[g0] : 0;
+    const int root = ws.root_pre[sys];
+    set_target_box(sh, t, ws.sys_box[4 * sys + 3]);
+    const double soft = ws.sys_eps ? ws.sys_eps[sys] : p.soft;
+    const double soft2 = __dmul_rn(soft, soft);
+    double gtx = 0.0, gty = 0.0, gtz = 0.0;
+    int resume = valid ? 0 : INT_MAX;
+    unsigned tests = 0;
+    auto eval = [&](int count) {
+      // (inactive entries fill the last block of four)
+      for (int j0 = 0; j0 < count; j0 += kAdjBlock) {
+        double dx[kPerLane], dy[kPerLane], dz[kPerLane], d2[kPerLane], mu[kPerLane];
+        int pre[kPerLane], aux[kPerLane];
+        bool act[kPerLane];
+#pragma unroll
+        for (int q = 0; q < kPerLane; ++q) {
+          const int j = j0 + el * kPerLane + q;
+          const double4 v = sh.src[j];
+          const int2 tag = sh.tag[j];
+          pre[q] = tag.x;
+          aux[q] = tag.y;
+          mu[q] = v.w;
+          dx[q] = __dsub_rn(v.x, t.x);
+          dy[q] = __dsub_rn(v.y, t.y);
+          dz[q] = __dsub_rn(v.z, t.z);
+          d2[q] = sqdist(dx[q], dy[q], dz[q]);
+        }
+        // the targets' decisions, entry by entry: an undecided cell that a
+        // target accepts moves its resume index past the cell
+        const int4 tag0 = *reinterpret_cast<const int4 *>(&sh.tag[j0]), tag1 = *reinterpret_cast<const int4 *>(&sh.tag[j0 + 2]);
+        const bool undecided = min(min(tag0.y, tag0.w), min(tag1.y, tag1.w)) < -1;
+#pragma unroll
+        for (int q = 0; q < kPerLane; ++q) act[q] = pre[q] >= resume && aux[q] != s;
+        if (undecided) {
+#pragma unroll
+          for (int e = 0; e < kLanes; ++e) {
+#pragma unroll
+            for (int q = 0; q < kPerLane; ++q) {
+              if (e == el) {
+                act[q] = act[q] && pre[q] >= resume;
+                if (aux[q] < -1) {
+                  act[q] = act[q] && accept_entry(sh, j0 + el * kPerLane + q, ws, pre[q], t, d2[q]);
+                  if (act[q]) resume = -aux[q];
+                }
+              }
+            }
+            if (kLanes > 1) resume = __shfl_sync(kFull, resume, e * kTargets + tl);
+          }
+        }
+        bool any = false;
+#pragma unroll
+        for (int q = 0; q < kPerLane; ++q) any |= act[q];
+        if (!__any_sync(kFull, any)) continue;
+#pragma unroll
+        for (int q = 0; q < kPerLane; ++q) {
+          double u[4] = {0.0, 0.0, 0.0, 0.0};
+          if (act[q]) {
+            singular |= !vjp_pair(dx[q], dy[q], dz[q], d2[q], mu[q], g, soft2, cx, cy, cz, u);
+            gtx -= u[0];
+            gty -= u[1];
+            gtz -= u[2];
+          }
+          double *row = sum + tl * kAdjRow + 4 * (el * kPerLane + q);
+          row[0] = u[0];
+          row[1] = u[1];
+          row[2] = u[2];
+          row[3] = u[3];
+        }
+        __syncwarp();
+        const int col = lane & 15, r0 = (lane >> 4) * (kTargets / 2);
+        double total = 0.0;
+#pragma unroll
+        for (int r = 0; r < kTargets / 2; ++r) total += sum[(r0 + r) * kAdjRow + col];
+        total += __shfl_xor_sync(kFull, total, 16);
+        if (lane < 16 && total != 0.0) {
+          const int2 tag = sh.tag[j0 + (col >> 2)];
+          double *dst = reinterpret_cast<double *>(tag.y >= 0 ? ab.part_g + tag.y : ab.node_g + tag.x);
+          atomicAdd(dst + (col & 3), total);
+        }
+        __syncwarp();
+      }
+      return __reduce_min_sync(kFull, resume);
+    };
+    ordered_walk(ws, m, root, 1.0, sh, tests, eval);
+#pragma unroll
+    for (int o = kTargets; o < 32; o <<= 1) {
+      gtx += __shfl_xor_sync(kFull, gtx, o);
+      gty += __shfl_xor_sync(kFull, gty, o);
+      gtz += __shfl_xor_sync(kFull, gtz, o);
+    }
+    if (valid && el == 0) ab.tgt_g[s] = make_double4(gtx, gty, gtz, 0.0);
+    __syncwarp();
   }
   if (__any_sync(kFull, singular) && lane == 0) record_error(sc, kStageTraversal, 6);
 }
@@ -539,12 +564,16 @@ cudaError_t launch_adjoint_force(Workspace &ws, const TraversalParams &p, const 
   if (e != cudaSuccess) return e;
   const int grid = grid_of_ws(ws, 8);
   adj_reset_kernel<<<1, 32, 0, s>>>(ws.sc);
-  adj_topology_kernel<<<grid, kBlock, 0, s>>>(ws, ab.pparent, ab.prange, nullptr);
+  adj_parent_kernel<<<grid, kBlock, 0, s>>>(ws, ab.pparent);
   if (p.precision == 1) {
     e = launch_adjoint_mixed(ws, p, ab, s);
     if (e != cudaSuccess) return e;
   } else {
-    adjoint_walk_kernel<<<grid_of_ws(ws, 8), 256, 0, s>>>(ws, p, ab);
+    // (7 blocks of two warps fit an SM)
+    if (p.targets > 8)
+      adjoint_walk_kernel<32><<<grid_of_ws(ws, 7), kAdjWarps * 32, 0, s>>>(ws, p, ab);
+    else
+      adjoint_walk_kernel<8><<<grid_of_ws(ws, 7), kAdjWarps * 32, 0, s>>>(ws, p, ab);
   }
   adj_node_kernel<<<grid, kBlock, 0, s>>>(ws, ab);
   adj_leaf_kernel<<<grid, kBlock, 0, s>>>(ws, ab);

@@ -288,6 +288,11 @@ bool finite_nonneg(double v) { return std::isfinite(v) && v >= 0.0; }
 // at 1000 particles, 208 / 400 at 4096, 1040 / 570 at 16384.
 int fp64_targets(int n) { return n < 8192 ? 1 : 32; }
 
+// Targets per warp of the FP64 adjoint walk: eight (four lanes to a target)
+// while 32 leave warps idle.  Backward pass of eight steps, 8 / 32 targets per
+// warp: 5.1 / 6.4 ms at 1000 particles, 13.4 / 16.7 at 16384, 30 / 27 at 65536.
+int adjoint_targets(int n) { return n < 32768 ? 8 : 32; }
+
 // The target groups a walk needs: their largest size and the pieces the plain
 // walk takes them in.  Groups of up to 128 cut into 32 fill the lanes better
 // than groups of up to 32 (27 targets per warp against 23 at 2^18 particles:
@@ -431,7 +436,6 @@ struct RolloutRecord {
   double *g = nullptr;            // 7 x n: gx gy gz gvx gvy gvz gm
   double4 *node_g = nullptr, *part_g = nullptr, *tgt_g = nullptr;
   int *pparent = nullptr;
-  int2 *prange = nullptr;
 };
 
 // Device buffers of frame capture, taken at the first capture.
@@ -1711,12 +1715,14 @@ cudaError_t enqueue_vjp(nbb_sim *sim, const TraversalParams &tpa, const AdjointB
   Workspace &ws = sim->ws;
   cudaStream_t s = sim->stream;
   const int group_max = ws.group_max, group_chunk = ws.group_chunk;
-  ws.group_max = 32;  // target groups of one warp (kernels take the workspace by value)
-  ws.group_chunk = 0;
+  set_groups(ws, tpa);  // (kernels take the workspace by value)
+  // the cotangents of the nodes are carried to the particles over the plain
+  // records, whichever walk forms them
+  ws.records = tpa.precision == NBB_PRECISION_MIXED ? (kRecordsFp64 | kRecordsMixed) : kRecordsFp64;
   cudaError_t e = launch_step_reset(ws, s);
   if (e == cudaSuccess) e = launch_kd_bbox(ws, 0.0, 0, s);
   if (e == cudaSuccess) e = launch_morton_sort_groups(ws, s);
-  if (e == cudaSuccess) e = launch_tree(ws, tpa.theta, s);
+  if (e == cudaSuccess) e = launch_level_order_tree(ws, tpa.theta, s);
   if (e == cudaSuccess) e = launch_adjoint_force(ws, tpa, ab, s);
   ws.group_max = group_max;
   ws.group_chunk = group_chunk;
@@ -1759,7 +1765,6 @@ int nbb_sim_rollout(nbb_sim *sim, uint64_t steps, uint64_t checkpoint_every) {
     ar.add(rec->part_g, n);
     ar.add(rec->tgt_g, n);
     ar.add(rec->pparent, (size_t)ws.cap_nodes);
-    ar.add(rec->prange, (size_t)ws.cap_nodes);
     e = ar.take(rec->al);
     if (e != cudaSuccess) return cuda_fail(e, "rollout checkpoint allocation");
   }
@@ -1830,13 +1835,13 @@ int nbb_sim_backward(nbb_sim *sim, const double *gx, const double *gy, const dou
   ab.part_g = rec.part_g;
   ab.tgt_g = rec.tgt_g;
   ab.pparent = rec.pparent;
-  ab.prange = rec.prange;
   // the VJP of the force the rollout ran: the plain form's, or the mixed
   // form's on its own interaction lists (32-target groups)
   TraversalParams tpa = traversal_params(sim, 0);
   tpa.precision = sim->cfg.precision == NBB_PRECISION_MIXED ? 1 : 0;
   tpa.kick = 0;
   tpa.group_size = 32;
+  tpa.targets = adjoint_targets(ws.n);
   tpa.cache_depth = 0;
   cudaError_t e = cudaSuccess;
   if (S > 0) {

@@ -432,7 +432,6 @@ struct AdjointBuffers {
   double4 *part_g = nullptr;  // per Morton slot
   double4 *tgt_g = nullptr;   // per Morton slot
   int *pparent = nullptr;     // per preorder node
-  int2 *prange = nullptr;     // per preorder node
 };
 // Perturbed copies of the particles: field arrays of copies * n values,
 // copy q at offset q * n (original order), plus per-copy scratch.
