@@ -277,14 +277,17 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 7)
   if (__any_sync(kFull, singular) && lane == 0) record_error(sc, kStageTraversal, 6);
 }
 
-// (gX, gM) of a node -> (P, Q) = (gX / M, gM - X . gX / M).
+// (gX, gM) of a node -> (P, Q) = (gX / M, gM - X . gX / M).  Node cotangents
+// are by preorder index (FP64 walk) or, with kLevel, by level-order index
+// (mixed walk).
+template <bool kLevel>
 __global__ void __launch_bounds__(kBlock) adj_node_kernel(Workspace ws, AdjointBuffers ab) {
   DevScalars *sc = ws.sc;
   if (sc->error) return;
   const int m = sc->n_nodes;
   for (int pre = blockIdx.x * blockDim.x + threadIdx.x; pre < m; pre += gridDim.x * blockDim.x) {
     const double4 gg = ab.node_g[pre];
-    const double4 a = ws.node_a[pre];
+    const double4 a = kLevel ? ws.lo_node[pre].a : ws.node_a[pre];
     double px = 0.0, py = 0.0, pz = 0.0, q = gg.w;
     if (a.w > 0.0) {
       const double inv = 1.0 / a.w;
@@ -301,12 +304,19 @@ __global__ void __launch_bounds__(kBlock) adj_node_kernel(Workspace ws, AdjointB
 // particles' total position / mass cotangent of this force evaluation; adds
 // them to the running cotangents and, when dt_v != 0, carries the position
 // cotangent into the velocity cotangent (gv += dt gx, the drift's adjoint).
+template <bool kLevel>
 __global__ void __launch_bounds__(kBlock) adj_leaf_kernel(Workspace ws, AdjointBuffers ab) {
   DevScalars *sc = ws.sc;
   if (sc->error) return;
   const int m = sc->n_nodes;
   for (int pre = blockIdx.x * blockDim.x + threadIdx.x; pre < m; pre += gridDim.x * blockDim.x) {
-    const int4 meta = ws.node_meta[pre];
+    int4 meta;  // (-, first particle, particles of a leaf, -)
+    if (kLevel) {
+      const int4 t = *reinterpret_cast<const int4 *>(&ws.lo_node[pre].pre);
+      meta = make_int4(0, t.z, t.w ? t.y : 0, 0);
+    } else {
+      meta = ws.node_meta[pre];
+    }
     if (meta.z <= 0) continue;
     double px = 0.0, py = 0.0, pz = 0.0, q = 0.0;
     int v = pre, guard = 0;
@@ -320,7 +330,7 @@ __global__ void __launch_bounds__(kBlock) adj_leaf_kernel(Workspace ws, AdjointB
       py += pq.y;
       pz += pq.z;
       q += pq.w;
-      v = ab.pparent[v];
+      v = kLevel ? ws.lo_first[v].w : ab.pparent[v];
     }
     for (int k = 0; k < meta.z; ++k) {
       const int sp = meta.y + k;
@@ -564,20 +574,22 @@ cudaError_t launch_adjoint_force(Workspace &ws, const TraversalParams &p, const 
   if (e != cudaSuccess) return e;
   const int grid = grid_of_ws(ws, 8);
   adj_reset_kernel<<<1, 32, 0, s>>>(ws.sc);
-  adj_parent_kernel<<<grid, kBlock, 0, s>>>(ws, ab.pparent);
   if (p.precision == 1) {
     e = launch_adjoint_mixed(ws, p, ab, s);
     if (e != cudaSuccess) return e;
+    adj_node_kernel<true><<<grid, kBlock, 0, s>>>(ws, ab);
+    adj_leaf_kernel<true><<<grid, kBlock, 0, s>>>(ws, ab);
   } else {
+    adj_parent_kernel<<<grid, kBlock, 0, s>>>(ws, ab.pparent);
     // (7 blocks of two warps fit an SM)
     if (p.targets > 8)
       adjoint_walk_kernel<32><<<grid_of_ws(ws, 7), kAdjWarps * 32, 0, s>>>(ws, p, ab);
     else
       adjoint_walk_kernel<8><<<grid_of_ws(ws, 7), kAdjWarps * 32, 0, s>>>(ws, p, ab);
+    adj_node_kernel<false><<<grid, kBlock, 0, s>>>(ws, ab);
+    adj_leaf_kernel<false><<<grid, kBlock, 0, s>>>(ws, ab);
   }
-  adj_node_kernel<<<grid, kBlock, 0, s>>>(ws, ab);
-  adj_leaf_kernel<<<grid, kBlock, 0, s>>>(ws, ab);
-  count_launches(p.precision == 1 ? 4 : 5);
+  count_launches(p.precision == 1 ? 3 : 5);
   return cudaGetLastError();
 }
 

@@ -1326,15 +1326,6 @@ __global__ void __launch_bounds__(kBlock) layout_kernel(Workspace ws, double the
       kids[j++] = pre + ws.preoff[c];
     }
     ws.node_meta[pre] = make_int4(pre + size, pc > 0 ? f : -1, pc > 0 ? pc : 0, j);
-    if (ws.node_m) {
-      MixedNode rec;
-      rec.a = rec_a;
-      rec.cr2 = __double2float_ru(cm * cm * (1.0 + 0x1p-18));
-      rec.first = pc > 0 ? f : -1;
-      rec.count = pc > 0 ? pc : 0;
-      rec.nchild = j;
-      ws.node_m[pre] = rec;
-    }
     for (; j < 8; ++j) kids[j] = -1;
   }
 }
@@ -1624,7 +1615,7 @@ __global__ void __launch_bounds__(32 * kLevelOrderChannels) lo_tile_scan_kernel(
 struct LoCell {
   double4 a;  // centre of mass, mass
   unsigned long long key;
-  int level, pre, skip, pf, pe, nk;
+  int level, b, pre, skip, pf, pe, c0, nk;  // b: level-order index; c0: first child
   bool leaf;
 };
 
@@ -1664,7 +1655,10 @@ __device__ __forceinline__ bool lo_emit_records(const Workspace &ws, double thet
   if (level >= ws.sys_levels) {
     const unsigned long long sys = c.key >> kSpatialBits;
     if (sys >= (unsigned long long)ws.n_systems) return false;
-    if (level == ws.sys_levels) ws.root_pre[sys] = pre;
+    if (level == ws.sys_levels) {
+      ws.root_pre[sys] = pre;
+      ws.root_lo[sys] = c.b;
+    }
   }
   if (level >= ws.sys_levels && !leaf) {
     const unsigned long long sys = c.key >> kSpatialBits;
@@ -1706,10 +1700,10 @@ __device__ __forceinline__ bool lo_emit_records(const Workspace &ws, double thet
     MixedNode mrec;
     mrec.a = a;
     mrec.cr2 = leaf ? 0.f : __double2float_ru(cm * cm * (1.0 + 0x1p-18));
-    mrec.first = leaf ? c.pf : -1;
+    mrec.first = leaf ? c.pf : c.c0;
     mrec.count = leaf ? c.pe - c.pf : 0;
     mrec.nchild = c.nk;
-    ws.node_m[pre] = mrec;
+    ws.node_m[c.b] = mrec;
   }
   return true;
 }
@@ -1922,8 +1916,10 @@ __device__ __forceinline__ bool lo_leaf_cell(const Workspace &ws, int g, int M, 
   bleaf = lf.x;
   c.skip = lf.y;
   c.pre = c.skip - 1;
+  c.b = bleaf;
   c.pf = pf;
   c.pe = pe;
+  c.c0 = 0;
   c.nk = 0;
   c.leaf = true;
   if (bleaf < 0 || bleaf >= M || c.pre < 0 || c.pre >= M || pf < 0 || pe <= pf || pe > ws.n || c.level < 1 ||
@@ -1971,6 +1967,7 @@ __device__ __forceinline__ LevelNode ld_level_node_cg(const LevelNode *p) {
 // the child list, the target-group marks and its LevelNode; the traversal
 // records are the caller's (lo_emit_records with c).  Returns false on
 // inconsistent input.
+template <int kRecords>
 __device__ __forceinline__ bool lo_level_cell(const Workspace &ws, int level, int b, int hi, int end, int M,
                                               const int4 &f, const int4 &q, int next_first_child, LoCell &c) {
   DevScalars *sc = ws.sc;
@@ -1988,11 +1985,13 @@ __device__ __forceinline__ bool lo_level_cell(const Workspace &ws, int level, in
   c.skip = skip;
   c.pf = pf;
   c.pe = pe;
+  c.b = b;
+  c.c0 = c0;
   c.nk = nk;
   c.leaf = false;
   c.key = (unsigned long long)(unsigned)q.z | ((unsigned long long)(unsigned)q.w << 32);
   // children in visit order: octant 7 -> 0, the children in descending key order
-  int *kids = ws.node_kids + (size_t)pre * 8;
+  int *kids = (kRecords & kRecordsFp64) ? ws.node_kids + (size_t)pre * 8 : nullptr;
   // target groups (group_mark_kernel's rule): a whole system that is one
   // group, else the starts of the children's runs
   const int np = pe - pf;
@@ -2012,7 +2011,7 @@ __device__ __forceinline__ bool lo_level_cell(const Workspace &ws, int level, in
       wx = __fma_rn(cm, ch.a.x, wx);
       wy = __fma_rn(cm, ch.a.y, wy);
       wz = __fma_rn(cm, ch.a.z, wz);
-      kids[nk - 1 - j] = ch.pre;
+      if (kRecords & kRecordsFp64) kids[nk - 1 - j] = ch.pre;
       if (!whole) {
         if (virt) run = 0;
         const int cp = ch.np;
@@ -2028,7 +2027,8 @@ __device__ __forceinline__ bool lo_level_cell(const Workspace &ws, int level, in
       }
     }
   }
-  for (int j = nk; j < 8; ++j) kids[j] = -1;
+  if (kRecords & kRecordsFp64)
+    for (int j = nk; j < 8; ++j) kids[j] = -1;
   lo_emit_node(ws, b, tm, wx, wy, wz, c);
   return true;
 }
@@ -2126,7 +2126,7 @@ __global__ void __launch_bounds__(kUpsweepBlock, 32) lo_upsweep_kernel(Workspace
         if (bad) record_error(sc, kStageLayout, 1);
         break;
       }
-      if (!lo_level_cell(ws, lv, p, hi, end, M, f, q, fr.y, c)) break;
+      if (!lo_level_cell<kRecords>(ws, lv, p, hi, end, M, f, q, fr.y, c)) break;
       cell = p;
       level = lv;
       p = f.w;
@@ -2192,39 +2192,6 @@ __global__ void __launch_bounds__(kBlock) lo_group_mark_kernel(Workspace ws) {
       }
       run += cp;
     }
-  }
-}
-
-// The node-cache table: the cells of levels 0..kTopDepth with their mixed
-// records and child lists (read back from the step's records).
-__global__ void __launch_bounds__(128) lo_top_kernel(Workspace ws) {
-  __shared__ int s_base[kTopDepth + 3];
-  __shared__ int s_ok;
-  DevScalars *sc = ws.sc;
-  if (threadIdx.x < kTopDepth + 3) s_base[threadIdx.x] = sc->level_base[threadIdx.x];
-  if (threadIdx.x == 0) {
-    const int m = sc->n_nodes;
-    s_ok = !sc->error && m > 0 && sc->level_base[kTopDepth + 2] <= m;
-  }
-  __syncthreads();
-  if (!s_ok) return;
-  const int count = min(s_base[kTopDepth + 1], kTopMax);
-  for (int q = threadIdx.x; q < count; q += blockDim.x) {
-    const int level = (q < s_base[1]) ? 0 : (q < s_base[2] ? 1 : 2);
-    const LevelNode nd = ws.lo_node[q];
-    const int c0 = ws.lo_first[q].y;
-    const int c1 = (q + 1 < s_base[level + 1]) ? ws.lo_first[q + 1].y : s_base[level + 2];
-    TopNode t;
-    t.rec = ws.node_m[nd.pre];
-    const int4 *k = reinterpret_cast<const int4 *>(ws.node_kids + (size_t)nd.pre * 8);
-    const int4 k0 = k[0], k1 = k[1];
-    t.kids[0] = k0.x; t.kids[1] = k0.y; t.kids[2] = k0.z; t.kids[3] = k0.w;
-    t.kids[4] = k1.x; t.kids[5] = k1.y; t.kids[6] = k1.z; t.kids[7] = k1.w;
-    t.first_child = c0;
-    t.nchild = nd.leaf ? 0 : min(max(c1 - c0, 0), 8);
-    t.level = level;
-    t.pad = 0;
-    ws.top[q] = t;
   }
 }
 
@@ -2427,10 +2394,8 @@ cudaError_t launch_level_order_tree(Workspace &ws, double theta, cudaStream_t s)
   lo_tile_scan_kernel<<<1, 32 * kLevelOrderChannels, 0, s>>>(ws);
   if (ws.records == kRecordsMixed)
     lo_rank_kernel<kRecordsMixed><<<ws.scan_tiles_n, kScanThreads, 0, s>>>(ws, theta);
-  else if (ws.records == kRecordsFp64)
-    lo_rank_kernel<kRecordsFp64><<<ws.scan_tiles_n, kScanThreads, 0, s>>>(ws, theta);
   else
-    lo_rank_kernel<kRecordsFp64 | kRecordsMixed><<<ws.scan_tiles_n, kScanThreads, 0, s>>>(ws, theta);
+    lo_rank_kernel<kRecordsFp64><<<ws.scan_tiles_n, kScanThreads, 0, s>>>(ws, theta);
   // leaves and every internal cell in one launch (arrival counters), one
   // thread per group in one-warp blocks (a resident grid taking groups
   // grid-stride measured slower: 267 against 174 us at 2^20 particles)
@@ -2438,14 +2403,8 @@ cudaError_t launch_level_order_tree(Workspace &ws, double theta, cudaStream_t s)
   const int up_grid = want > 0 ? want : 1;
   if (ws.records == kRecordsMixed)
     lo_upsweep_kernel<kRecordsMixed><<<up_grid, kUpsweepBlock, 0, s>>>(ws, theta);
-  else if (ws.records == kRecordsFp64)
-    lo_upsweep_kernel<kRecordsFp64><<<up_grid, kUpsweepBlock, 0, s>>>(ws, theta);
   else
-    lo_upsweep_kernel<kRecordsFp64 | kRecordsMixed><<<up_grid, kUpsweepBlock, 0, s>>>(ws, theta);
-  if (ws.top && (ws.records & kRecordsMixed) && ws.n_systems == 1) {
-    lo_top_kernel<<<1, 128, 0, s>>>(ws);
-    count_launches(1);
-  }
+    lo_upsweep_kernel<kRecordsFp64><<<up_grid, kUpsweepBlock, 0, s>>>(ws, theta);
   // target-group marks were set by the upward pass
   group_scan_kernel<<<ws.scan_tiles_n, kScanThreads, 0, s>>>(ws);
   count_launches(5);

@@ -197,7 +197,6 @@ struct WorkspaceParts {
   bool motion = true;        // their velocities and types
   bool reference = true;     // the reference-numbered build
   bool level_order = false;  // the level-order build
-  bool cache = false;        // the mixed walk's node-cache table
   int records = kRecordsFp64 | kRecordsMixed;
 };
 
@@ -235,7 +234,7 @@ cudaError_t alloc_workspace(Workspace &ws, Allocation &al, int n, const Workspac
     GET(ws.sys_eps, S);
   }
   GET(ws.sc, 1);
-  GET(ws.sys_bb, 6 * S); GET(ws.sys_box, 4 * S); GET(ws.root_pre, S);
+  GET(ws.sys_bb, 6 * S); GET(ws.sys_box, 4 * S); GET(ws.root_pre, S); GET(ws.root_lo, S);
   GET(ws.pairs_a, N); GET(ws.pairs_b, N);
   GET(ws.digit_hist, (size_t)kMaxSortPasses * 256);
   ws.sort_tiles = (n + kSortTile - 1) / kSortTile;
@@ -259,12 +258,12 @@ cudaError_t alloc_workspace(Workspace &ws, Allocation &al, int n, const Workspac
   }
   if (parts.records & kRecordsFp64) {
     GET(ws.node_a, C); GET(ws.node_b, C); GET(ws.node_c, C); GET(ws.node_meta, C);
+    GET(ws.node_kids, 8 * C);
   }
   if (parts.records & kRecordsMixed) {
     GET(ws.node_m, C);
     GET(ws.walk_ext, (size_t)ws.walk_warps * ws.walk_ext_cap);
   }
-  GET(ws.node_kids, 8 * C);
   if (parts.level_order) {
     ws.level_order = 1;
     GET(ws.gspan, N);
@@ -272,11 +271,11 @@ cudaError_t alloc_workspace(Workspace &ws, Allocation &al, int n, const Workspac
     GET(ws.pos4, N);
     GET(ws.lo_tiles, (size_t)ws.scan_tiles_n * kLevelOrderChannels);
   }
-  if (parts.cache) GET(ws.top, (size_t)kTopMax);
 #undef GET
   e = ar.take(al);
   if (e == cudaSuccess) e = cudaMemset(ws.sc, 0, sizeof(DevScalars));
   if (e == cudaSuccess) e = cudaMemset(ws.root_pre, 0, S * sizeof(int));
+  if (e == cudaSuccess) e = cudaMemset(ws.root_lo, 0, S * sizeof(int));
   return e;
 }
 
@@ -608,7 +607,7 @@ static int create_sim(const nbb_config *cfg, size_t n, int n_systems, const int6
   sim->min_softening = min_eps;
   cudaError_t e = cudaStreamCreateWithFlags(&sim->own_stream, cudaStreamNonBlocking);
   WorkspaceParts parts;
-  parts.level_order = parts.cache = true;
+  parts.level_order = true;
   if (e == cudaSuccess) e = alloc_workspace(sim->ws, sim->alloc, (int)n, parts, n_systems > 1 ? n_systems : 1);
   if (e != cudaSuccess) {
     if (sim->own_stream) cudaStreamDestroy(sim->own_stream);
@@ -672,7 +671,7 @@ static TraversalParams traversal_params(const nbb_sim *sim, int kick) {
   tp.group_size = sim->cfg.group_size > 0 ? sim->cfg.group_size
                                           : (sim->tuned_group_size > 0 ? sim->tuned_group_size : 32);
   tp.targets = sim->walk_targets > 0 ? sim->walk_targets : fp64_targets(sim->ws.n);
-  if (tp.precision == NBB_PRECISION_MIXED && sim->ws.top && sim->ws.n_systems == 1)
+  if (tp.precision == NBB_PRECISION_MIXED && sim->ws.n_systems == 1)
     tp.cache_depth = sim->cfg.cache_depth >= 0 ? sim->cfg.cache_depth
                                                : (sim->tuned_cache_depth > 0 ? sim->tuned_cache_depth : 0);
   if (sim->ws.n_systems > 1) tp.soft = sim->min_softening;
@@ -718,7 +717,7 @@ static int autotune_mixed_walk(nbb_sim *sim) {
     const int sizes[3] = {32, 64, 128};
     const int n_sizes = pinned ? 1 : 3;
     const int pinned_depth = sim->cfg.cache_depth;
-    const bool cacheable = ws.top && ws.n_systems == 1;
+    const bool cacheable = ws.n_systems == 1;
     const int n_depths = (pinned_depth >= 0 || !cacheable) ? 1 : kTopDepth + 1;
     // candidates timed round-robin (three rounds, best time of each) after
     // one untimed walk, so that clock ramp-up and cache warm-up fall on no
@@ -1137,12 +1136,13 @@ int nbb_accel(size_t n, const double *mass, const double *x, const double *y, co
   Scratch sc;
   NBB_CUDA(cudaStreamCreateWithFlags(&sc.s, cudaStreamNonBlocking), "create stream");
   // the octree in the reference's numbering only when it is exported; the
-  // level-order build gives the same records with fewer passes
+  // level-order build gives the same records with fewer passes (and is the
+  // mixed walk's only form: there its tree is exported as a simulation's is)
   WorkspaceParts parts;
   parts.motion = false;
   parts.reference = export_out != nullptr;
-  parts.level_order = !parts.reference;
-  if (parts.level_order) parts.records = precision == NBB_PRECISION_MIXED ? kRecordsMixed : kRecordsFp64;
+  parts.level_order = !parts.reference || precision == NBB_PRECISION_MIXED;
+  if (!parts.reference) parts.records = precision == NBB_PRECISION_MIXED ? kRecordsMixed : kRecordsFp64;
   NBB_CUDA(alloc_workspace(sc.ws, sc.al, (int)n, parts), "allocate workspace");
   Workspace &ws = sc.ws;
   const cudaMemcpyKind in = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
@@ -1179,6 +1179,11 @@ int nbb_accel(size_t n, const double *mass, const double *x, const double *y, co
     stats->cache_depth = 0;
   }
   if (export_out) {
+    if (ws.level_order) {
+      NBB_CUDA(launch_reference_octree(ws, theta, sc.s), "tree export");
+      st = check_device(ws, sc.s);
+      if (st) return st;
+    }
     st = export_workspace(ws, export_out, sc.s, true);
     if (st) return st;
   }
@@ -1716,9 +1721,7 @@ cudaError_t enqueue_vjp(nbb_sim *sim, const TraversalParams &tpa, const AdjointB
   cudaStream_t s = sim->stream;
   const int group_max = ws.group_max, group_chunk = ws.group_chunk;
   set_groups(ws, tpa);  // (kernels take the workspace by value)
-  // the cotangents of the nodes are carried to the particles over the plain
-  // records, whichever walk forms them
-  ws.records = tpa.precision == NBB_PRECISION_MIXED ? (kRecordsFp64 | kRecordsMixed) : kRecordsFp64;
+  ws.records = tpa.precision == NBB_PRECISION_MIXED ? kRecordsMixed : kRecordsFp64;
   cudaError_t e = launch_step_reset(ws, s);
   if (e == cudaSuccess) e = launch_kd_bbox(ws, 0.0, 0, s);
   if (e == cudaSuccess) e = launch_morton_sort_groups(ws, s);

@@ -86,13 +86,13 @@ constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
 
-// The mixed walk's record of one node (48 bytes, two 32-byte sectors):
-// centre of mass and mass, the squared acceptance radius for a target box
-// rounded up to FP32, and the node's particle range and child count.
+// The mixed walk's record of one node (48 bytes, two 32-byte sectors), at its
+// level-order index, where a node's children are consecutive: no child list
+// is loaded, and the records of siblings share cache lines.
 struct __align__(16) MixedNode {
   double4 a;   // com x, y, z, mass (an occupied leaf: its first particle)
   float cr2;   // (max(crit, sqrt(3) h + |com - centre|) (1 + 2^-40))^2 (1 + 2^-18), rounded up
-  int first;   // first particle of an occupied leaf, -1 otherwise
+  int first;   // first particle of an occupied leaf, else first child
   int count;   // particles of an occupied leaf, 0 otherwise
   int nchild;  // children
 };
@@ -111,21 +111,10 @@ struct __align__(16) LevelNode {
 static_assert(sizeof(LevelNode) == 48, "two 32-byte sectors per node");
 
 // The top levels of the level-order octree (levels 0..kTopDepth: at most
-// 1 + 8 + 64 cells, in level order), the table the mixed walk's shared-memory
-// node cache is loaded from: each cell's record, its children's preorder
-// indices (visit order) and, for a cell whose children are cached too, their
-// place in the table (first child, count).
+// 1 + 8 + 64 cells, the first entries of the numbering), which the mixed
+// walk's shared-memory node cache can hold.
 constexpr int kTopDepth = 2;
 constexpr int kTopMax = 73;
-struct __align__(16) TopNode {
-  MixedNode rec;
-  int kids[8];
-  int first_child;  // level-order index of the first child
-  int nchild;
-  int level;
-  int pad;
-};
-static_assert(sizeof(TopNode) == 96, "record, child list, child range");
 
 // Per-tile counts of the level-order build (tiles of kScanTile groups): the
 // cells started per octree level, then the cells ended (kMaxLevels); the
@@ -133,7 +122,7 @@ static_assert(sizeof(TopNode) == 96, "record, child list, child range");
 constexpr int kLevelOrderChannels = 32;
 
 // Traversal records a build writes: the plain FP64 walk's (node_a, node_b,
-// node_c, node_meta) and the mixed walk's (node_m); child lists always.
+// node_c, node_meta, node_kids) and the mixed walk's (node_m).
 constexpr int kRecordsFp64 = 1;
 constexpr int kRecordsMixed = 2;
 
@@ -172,6 +161,7 @@ struct Workspace {
   double *sys_box = nullptr;             // 4 per system: centre xyz, side
   double *sys_eps = nullptr;             // ensemble: softening per system
   int *root_pre = nullptr;               // preorder index of each system's root
+  int *root_lo = nullptr;                // its level-order index
 
   // sort
   unsigned long long *pairs_a = nullptr, *pairs_b = nullptr;  // n each
@@ -223,7 +213,7 @@ struct Workspace {
   double4 *node_c = nullptr;  // crit, crit^2 lower/upper band, mixed walk's squared box radius
   int4 *node_meta = nullptr;  // skip, first particle, particle count, nchild
   int *node_kids = nullptr;   // 8 per node, preorder ids in visit order
-  MixedNode *node_m = nullptr;  // the mixed walk's records, preorder
+  MixedNode *node_m = nullptr;  // the mixed walk's records, level-order
 
   // level-order build (simulation steps): the octree numbered level by level
   int level_order = 0;          // host: 1 when steps build the level-order octree
@@ -236,7 +226,6 @@ struct Workspace {
   LevelNode *lo_node = nullptr;  // cap: mass, centre of mass, preorder index, particles
   int *lo_tiles = nullptr;      // scan_tiles_n * kLevelOrderChannels: per-tile counts, then their prefixes
   int records = kRecordsFp64 | kRecordsMixed;  // host: the records the level-order build writes
-  TopNode *top = nullptr;       // kTopMax: the top levels, for the mixed walk's node cache
   int *walk_ext = nullptr;    // walk_warps x walk_ext_cap: the mixed walk's stack below shared memory
 };
 

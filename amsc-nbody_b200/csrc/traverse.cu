@@ -394,12 +394,6 @@ __device__ __forceinline__ bool eval_batch(const PairList &list, const int *src,
   return singular;
 }
 
-// A child entry the mixed walk may push: a node's children come after it in
-// preorder; a cached cell's children are cached cells after it or any node.
-__device__ __forceinline__ bool valid_child(int kid, int node, int m, int mc) {
-  return node < m ? (kid > node && kid < m) : ((kid > node && kid < mc) || (kid >= 0 && kid < m));
-}
-
 // Per-lane target state of the mixed walk: negated target offsets from the
 // group centre, each duplicated into both halves of a pair.
 template <int kTPL>
@@ -442,7 +436,7 @@ __device__ __forceinline__ bool eval_slots(const PairList &list, const int *src,
 // in FP32 with the hardware reciprocal square root.  A source's u is summed
 // over the warp's targets before it is added (FP64 atomics) to the cell's or
 // particle's cotangent; the list names each entry's source: a particle by its
-// Morton slot, a cell by -3 - its preorder index.
+// Morton slot, a cell by -3 - its level-order index.
 
 // Cotangent state of the adjoint walk's target (one per lane).
 struct LaneVjp {
@@ -631,11 +625,9 @@ __global__ void __launch_bounds__(kMixedWarps * 32,
     traverse_mixed_kernel(Workspace ws, TraversalParams p, AdjointBuffers ab) {
   static_assert(!kVjp || (kTrackSource && kTPL == 1), "the adjoint walk tracks sources, one target per lane");
   __shared__ MixedShared<kTrackSource> sh;
-  // node cache: the top cache_depth levels below the root, loaded once per
-  // block from the step's table; stack entry m + q names cached cell q
+  // node cache: the top cache_depth levels below the root (the first entries
+  // of the level order), loaded once per block
   __shared__ MixedNode c_rec[kTopMax];
-  __shared__ int4 c_kids[kTopMax][2];
-  __shared__ int s_ccount;
   DevScalars *sc = ws.sc;
   if (sc->error) return;
   const int lane = threadIdx.x & 31;
@@ -647,29 +639,12 @@ __global__ void __launch_bounds__(kMixedWarps * 32,
   const int m = sc->n_nodes;
   const int n_groups = sc->n_tgroups;
   const unsigned lt = lanemask_lt();
-  int ccount = 0;
-  if (p.cache_depth > 0 && ws.top && ws.n_systems == 1) {
-    if (threadIdx.x == 0) {
-      s_ccount = min(sc->level_base[min(p.cache_depth, kTopDepth) + 1], kTopMax);
-    }
-    __syncthreads();
-    ccount = s_ccount;
-    for (int q = threadIdx.x; q < ccount; q += blockDim.x) {
-      const TopNode &t = ws.top[q];
-      c_rec[q] = t.rec;
-      int kk[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        // children in visit order (descending level order); cached ones by slot
-        const int slot = t.first_child + t.nchild - 1 - j;
-        kk[j] = (t.level < p.cache_depth && j < t.nchild && slot < ccount) ? m + slot : t.kids[j];
-      }
-      c_kids[q][0] = make_int4(kk[0], kk[1], kk[2], kk[3]);
-      c_kids[q][1] = make_int4(kk[4], kk[5], kk[6], kk[7]);
-    }
+  int ccount = 0;  // nodes below this index are cached
+  if (p.cache_depth > 0 && ws.n_systems == 1) {
+    ccount = min(min(sc->level_base[min(p.cache_depth, kTopDepth) + 1], kTopMax), m);
+    for (int q = threadIdx.x; q < ccount; q += blockDim.x) c_rec[q] = ws.node_m[q];
     __syncthreads();
   }
-  const int mc = m + ccount;  // stack entries in [m, mc) are cached cells
   long long tests = 0;
   unsigned overflow = 0;
   long long inter_total = 0;
@@ -750,12 +725,12 @@ __global__ void __launch_bounds__(kMixedWarps * 32,
     }
     // a group's targets belong to one system: walk that system's subtree
     const int sys = ws.n_systems > 1 ? ws.psys[g0] : 0;
-    const int root = ws.root_pre[sys];
+    const int root = ws.root_lo[sys];
     const double soft = ws.sys_eps ? ws.sys_eps[sys] : p.soft;
     const float eps2f = (float)(soft * soft);
     const float2 eps2 = make_float2(eps2f, eps2f);
     int ls = 0;
-    if (lane == 0) stack[0] = ccount > 0 ? m : root;
+    if (lane == 0) stack[0] = root;
     int sp = (m > 0 && root >= 0 && root < m) ? 1 : 0;
     __syncwarp();
     // this warp's stack extension in global memory: when the shared part
@@ -795,36 +770,27 @@ __global__ void __launch_bounds__(kMixedWarps * 32,
       const int n1 = (lane + 32 < k) ? stack[sp - k + 32 + lane] : -1;
       sp -= k;
       __syncwarp();
-      int4 m0 = make_int4(0, 0, 0, 0), m1 = m0;
-      int4 k00 = make_int4(-1, -1, -1, -1), k01 = k00, k10 = k00, k11 = k00;
+      int4 m0 = make_int4(0, 0, 0, 0), m1 = m0;  // radius, first, count, nchild
       double4 a0 = make_double4(0.0, 0.0, 0.0, 0.0), a1 = a0;
-      float cr0 = 0.f, cr1 = 0.f;  // squared acceptance radius for a target box
-      if (n0 >= m) {
-        const MixedNode &rec = c_rec[n0 - m];
-        a0 = rec.a;
-        const int4 meta = *reinterpret_cast<const int4 *>(&rec.cr2);
-        cr0 = __int_as_float(meta.x);
-        m0 = make_int4(0, meta.y, meta.z, meta.w);
-      } else if (n0 >= 0) {
-        const MixedNode &rec = ws.node_m[n0];
-        a0 = rec.a;
-        const int4 meta = *reinterpret_cast<const int4 *>(&rec.cr2);
-        cr0 = __int_as_float(meta.x);
-        m0 = make_int4(0, meta.y, meta.z, meta.w);
+      if (n0 >= 0) {
+        if (n0 < ccount) {
+          a0 = c_rec[n0].a;
+          m0 = *reinterpret_cast<const int4 *>(&c_rec[n0].cr2);
+        } else {
+          a0 = ws.node_m[n0].a;
+          m0 = *reinterpret_cast<const int4 *>(&ws.node_m[n0].cr2);
+        }
       }
-      if (n1 >= m) {
-        const MixedNode &rec = c_rec[n1 - m];
-        a1 = rec.a;
-        const int4 meta = *reinterpret_cast<const int4 *>(&rec.cr2);
-        cr1 = __int_as_float(meta.x);
-        m1 = make_int4(0, meta.y, meta.z, meta.w);
-      } else if (n1 >= 0) {
-        const MixedNode &rec = ws.node_m[n1];
-        a1 = rec.a;
-        const int4 meta = *reinterpret_cast<const int4 *>(&rec.cr2);
-        cr1 = __int_as_float(meta.x);
-        m1 = make_int4(0, meta.y, meta.z, meta.w);
+      if (n1 >= 0) {
+        if (n1 < ccount) {
+          a1 = c_rec[n1].a;
+          m1 = *reinterpret_cast<const int4 *>(&c_rec[n1].cr2);
+        } else {
+          a1 = ws.node_m[n1].a;
+          m1 = *reinterpret_cast<const int4 *>(&ws.node_m[n1].cr2);
+        }
       }
+      const float cr0 = __int_as_float(m0.x), cr1 = __int_as_float(m1.x);  // squared acceptance radius for a target box
       // 0 nothing, 1 accepted cell, 2 leaf, 3 open; the cell's list entry
       // (centre of mass offset from the group centre, mass) in FP32
       int cat0 = 0, cat1 = 0;
@@ -851,32 +817,13 @@ __global__ void __launch_bounds__(kMixedWarps * 32,
           }
         }
       }
-      // opened nodes push their children (node 0's, then node 1's); a push
-      // that would end past the stack accepts the node instead
+      // opened nodes push their children (node 0's, then node 1's), which are
+      // consecutive and come after them in the level order; a push that would
+      // end past the stack accepts the node instead
       int nc0 = (cat0 == 3) ? min(max(m0.w, 0), 8) : 0;
       int nc1 = (cat1 == 3) ? min(max(m1.w, 0), 8) : 0;
-      // child lists only of the nodes that open; their loads overlap the
-      // prefix sums below
-      if (nc0 > 0) {
-        if (n0 >= m) {
-          k00 = c_kids[n0 - m][0];
-          k01 = c_kids[n0 - m][1];
-        } else {
-          const int4 *kids = reinterpret_cast<const int4 *>(ws.node_kids + (size_t)n0 * 8);
-          k00 = kids[0];
-          if (nc0 > 4) k01 = kids[1];
-        }
-      }
-      if (nc1 > 0) {
-        if (n1 >= m) {
-          k10 = c_kids[n1 - m][0];
-          k11 = c_kids[n1 - m][1];
-        } else {
-          const int4 *kids = reinterpret_cast<const int4 *>(ws.node_kids + (size_t)n1 * 8);
-          k10 = kids[0];
-          if (nc1 > 4) k11 = kids[1];
-        }
-      }
+      if (m0.y <= n0 || m0.y > m - nc0) nc0 = 0;
+      if (m1.y <= n1 || m1.y > m - nc1) nc1 = 0;
       int all_children;
       const int excl = warp_prefix_small<5>(nc0 + nc1, lt, all_children);
       int pushed = all_children;
@@ -893,18 +840,12 @@ __global__ void __launch_bounds__(kMixedWarps * 32,
         }
         pushed = __reduce_max_sync(kFull, (nc0 + nc1 > 0) ? excl + nc0 + nc1 : 0);
       }
-      {
-        const int kid[8] = {k00.x, k00.y, k00.z, k00.w, k01.x, k01.y, k01.z, k01.w};
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (j < nc0) stack[sp + excl + j] = valid_child(kid[j], n0, m, mc) ? kid[j] : -1;
-      }
-      {
-        const int kid[8] = {k10.x, k10.y, k10.z, k10.w, k11.x, k11.y, k11.z, k11.w};
+      for (int j = 0; j < 8; ++j)
+        if (j < nc0) stack[sp + excl + j] = m0.y + j;
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (j < nc1) stack[sp + excl + nc0 + j] = valid_child(kid[j], n1, m, mc) ? kid[j] : -1;
-      }
+      for (int j = 0; j < 8; ++j)
+        if (j < nc1) stack[sp + excl + nc0 + j] = m1.y + j;
       sp += pushed;
       // accepted cells -> interaction list (fewer than 32 entries before,
       // at most 64 more)
@@ -1422,7 +1363,7 @@ cudaError_t launch_adjoint_mixed(Workspace &ws, const TraversalParams &p, const 
   int grid = ws.vjp_grid > 0 ? ws.vjp_grid : 148;
   if (ws.walk_warps > 0 && grid * kMixedWarps > ws.walk_warps) grid = ws.walk_warps / kMixedWarps;
   TraversalParams q = p;
-  q.cache_depth = 0;  // cached cells carry no preorder index
+  q.cache_depth = 0;
   traverse_mixed_kernel<true, 1, true><<<grid, kMixedWarps * 32, 0, s>>>(ws, q, ab);
   count_launches(1);
   return cudaGetLastError();
