@@ -26,6 +26,8 @@
 // device memory and every later kernel bounds its grid-stride loop by them.
 #include "nbb_internal.cuh"
 
+#include <algorithm>
+
 #include <cfloat>
 #include <climits>
 #include <cmath>
@@ -58,8 +60,8 @@ __global__ void reset_sys_kernel(unsigned long long *bb, int n_systems) {
     bb[k] = (k % 6 < 3) ? ~0ull : 0ull;
 }
 
-__global__ void reset_scalars_kernel(DevScalars *sc) {
-  if (threadIdx.x == 0) {
+__device__ __forceinline__ void reset_scalars(DevScalars *sc) {
+  {
     for (int a = 0; a < 3; ++a) {
       sc->bb_min[a] = ~0ull;
       sc->bb_max[a] = 0ull;
@@ -77,6 +79,33 @@ __global__ void reset_scalars_kernel(DevScalars *sc) {
     sc->mac_tests = 0;
     for (int l = 0; l < kMaxLevels; ++l) sc->level_count[l] = 0;
     for (int l = 0; l < kMaxLevels + 2; ++l) sc->level_base[l] = 0;
+  }
+}
+
+__global__ void reset_scalars_kernel(DevScalars *sc) {
+  if (threadIdx.x == 0) reset_scalars(sc);
+}
+
+// Everything a step starts from, in one launch (two kernels and four memsets
+// took 12 us of a small system's step in launches): the scalars, the systems'
+// extrema, and zeroed digit histograms, look-back status words and group
+// marks.
+__global__ void __launch_bounds__(kBlock) step_reset_kernel(Workspace ws) {
+  const size_t i0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+  if (i0 == 0) reset_scalars(ws.sc);
+  for (size_t k = i0; k < 6 * (size_t)ws.n_systems; k += step) ws.sys_bb[k] = (k % 6 < 3) ? ~0ull : 0ull;
+  for (size_t k = i0; k < (size_t)kMaxSortPasses * 256; k += step) ws.digit_hist[k] = 0u;
+  // 16 bytes at a time (allocations start on 256 bytes); sort status words
+  // come in rows of 256, the others end in single elements
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  const size_t sort_words = (size_t)ws.sort_passes * ws.sort_tiles * 64;
+  for (size_t k = i0; k < sort_words; k += step) reinterpret_cast<uint4 *>(ws.sort_status)[k] = zero;
+  const size_t scan = 3 * (size_t)ws.scan_tiles_n + ws.scan_tiles_r;
+  for (size_t k = i0; k < scan; k += step) ws.scan_status[k] = 0ull;
+  if (ws.tflag) {
+    const size_t n = (size_t)ws.n;
+    for (size_t k = i0; k < n / 16; k += step) reinterpret_cast<uint4 *>(ws.tflag)[k] = zero;
+    for (size_t k = (n & ~(size_t)15) + i0; k < n; k += step) ws.tflag[k] = 0;
   }
 }
 
@@ -349,35 +378,37 @@ constexpr uint32_t kDigitMask = (1u << 30) - 1u;
 // out by consecutive threads: a digit's items of one tile land at consecutive
 // addresses, so the stores go out as runs instead of one scattered 8-byte
 // store per item.
+template <int kItems>
 __global__ void __launch_bounds__(kSortThreads)
     onesweep_kernel(const unsigned long long *__restrict__ in,
                     unsigned long long *__restrict__ out, int n, int pass, int shift,
                     const uint32_t *__restrict__ digit_offsets,
                     uint32_t *status, DevScalars *sc) {
   constexpr int kWarps = kSortThreads / 32;
+  constexpr int kTile = kSortThreads * kItems;
   static_assert(kSortThreads == 256, "one thread per digit");
   __shared__ uint32_t whist[kWarps][256];
   __shared__ uint32_t tile_excl[256];   // digit's first slot in the staged tile
   __shared__ uint32_t digit_base[256];  // digit's first output position of this tile
   __shared__ uint32_t warp_tot[kWarps];
-  __shared__ unsigned long long stage[kSortTile];
+  __shared__ unsigned long long stage[kTile];
   __shared__ int s_tile;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) s_tile = (int)atomicAdd(&sc->tile_counter[pass], 1u);
   for (int k = tid; k < kWarps * 256; k += kSortThreads) (&whist[0][0])[k] = 0;
   __syncthreads();
   const int tile = s_tile;
-  const int start = tile * kSortTile + warp * (32 * kSortItems);
-  unsigned long long key[kSortItems];
-  uint32_t rank[kSortItems];
+  const int start = tile * kTile + warp * (32 * kItems);
+  unsigned long long key[kItems];
+  uint32_t rank[kItems];
 #pragma unroll
-  for (int it = 0; it < kSortItems; ++it) {
+  for (int it = 0; it < kItems; ++it) {
     const int i = start + it * 32 + lane;
     key[it] = (i < n) ? in[i] : ~0ull;
   }
   const unsigned lt = lanemask_lt();
 #pragma unroll
-  for (int it = 0; it < kSortItems; ++it) {
+  for (int it = 0; it < kItems; ++it) {
     const int i = start + it * 32 + lane;
     const bool valid = i < n;
     const uint32_t dig = (uint32_t)(key[it] >> shift) & 255u;
@@ -426,12 +457,12 @@ __global__ void __launch_bounds__(kSortThreads)
   __syncthreads();
   // the tile in digit order in shared memory, while the predecessors publish
 #pragma unroll
-  for (int it = 0; it < kSortItems; ++it) {
+  for (int it = 0; it < kItems; ++it) {
     const int i = start + it * 32 + lane;
     if (i < n) {
       const uint32_t dig = (uint32_t)(key[it] >> shift) & 255u;
       const uint32_t local = tile_excl[dig] + whist[warp][dig] + rank[it];
-      if (local < (uint32_t)kSortTile) stage[local] = key[it];
+      if (local < (uint32_t)kTile) stage[local] = key[it];
     }
   }
   {
@@ -475,7 +506,7 @@ __global__ void __launch_bounds__(kSortThreads)
     digit_base[tid] = digit_offsets[pass * 256 + tid] + prefix;
   }
   __syncthreads();
-  const int count = min(kSortTile, n - tile * kSortTile);
+  const int count = min(kTile, n - tile * kTile);
   for (int j = tid; j < count; j += kSortThreads) {
     const unsigned long long k = stage[j];
     const uint32_t dig = (uint32_t)(k >> shift) & 255u;
@@ -1492,8 +1523,9 @@ __device__ __forceinline__ int common_levels(unsigned long long a, unsigned long
 }
 
 // Per group: the level span (delta, lambda, delta of the next group) and the
-// particle count; per tile of kScanTile groups: the cells its groups start at
+// particle count; per tile of kScanThreads * kItems groups: the cells its groups start at
 // each level and the cells they end.
+template <int kItems>
 __global__ void __launch_bounds__(kScanThreads) lo_span_kernel(Workspace ws) {
   __shared__ int s_cnt[kLevelOrderChannels];
   __shared__ int s_g;
@@ -1508,9 +1540,9 @@ __global__ void __launch_bounds__(kScanThreads) lo_span_kernel(Workspace ws) {
   if (threadIdx.x < kLevelOrderChannels) s_cnt[threadIdx.x] = 0;
   __syncthreads();
   const int G = s_g, kb = ws.key_bits;
-  const int base = blockIdx.x * kScanTile;
+  const int base = blockIdx.x * (kScanThreads * kItems);
 #pragma unroll 1
-  for (int k = 0; k < kScanItems; ++k) {
+  for (int k = 0; k < kItems; ++k) {
     const int g = base + k * kScanThreads + threadIdx.x;
     if (g >= G) break;
     ws.gcount[g] = ws.glast[g] - ws.gfirst[g] + 1;
@@ -1555,7 +1587,8 @@ __global__ void __launch_bounds__(32 * kLevelOrderChannels) lo_tile_scan_kernel(
   DevScalars *sc = ws.sc;
   const int g = sc->n_groups;
   const int G = (g > 0 && g <= ws.n) ? g : 0;
-  const int tiles = (G + kScanTile - 1) / kScanTile;
+  const int tile = kScanThreads * ws.lo_items;
+  const int tiles = (G + tile - 1) / tile;
   const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int inc = 0;  // running total of channel c
   for (int t0 = 0; t0 < tiles; t0 += kChunk) {
@@ -1715,15 +1748,15 @@ __device__ __forceinline__ bool lo_emit_records(const Workspace &ws, double thet
 // its particle end, preorder index and key (by its last group; every group of
 // a cell carries the cell's prefix), and per group its leaf's level-order
 // index and S(g) (the leaf sits at level lambda, preorder index S(g) - 1).
-template <int kRecords>
-__global__ void __launch_bounds__(kScanThreads) lo_rank_kernel(Workspace ws, double theta) {
+template <int kItems>
+__global__ void __launch_bounds__(kScanThreads) lo_rank_kernel(Workspace ws) {
   constexpr int kWarps = kScanThreads / 32;
   constexpr int kNodes = kMaxLevels;  // channel of the ended cells (the node count S)
   static_assert(kNodes < kLevelOrderChannels, "one warp holds every channel");
   __shared__ int s_warp[kWarps][kLevelOrderChannels];
   __shared__ int s_prefix[kLevelOrderChannels];
   __shared__ int s_base[kMaxLevels + 2];
-  __shared__ int s_span[kScanItems][kScanThreads];
+  __shared__ int s_span[kItems][kScanThreads];
   __shared__ int s_g, s_m;
   DevScalars *sc = ws.sc;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1739,12 +1772,12 @@ __global__ void __launch_bounds__(kScanThreads) lo_rank_kernel(Workspace ws, dou
   if (tid < kLevelOrderChannels) s_prefix[tid] = ws.lo_tiles[(size_t)tile * kLevelOrderChannels + tid];
   __syncthreads();
   const int G = s_g, M = s_m;
-  const int base = tile * kScanTile;
+  const int base = tile * (kScanThreads * kItems);
   if (G == 0 || base >= G) return;
   const int max_level = ws.max_level;
-  // each warp owns 32 * kScanItems consecutive groups, item k at g0 + 32 k;
+  // each warp owns 32 * kItems consecutive groups, item k at g0 + 32 k;
   // a group's cells: started at levels (delta, lambda], ended at (delta_next, lambda]
-  const int g0 = base + warp * (32 * kScanItems) + lane;
+  const int g0 = base + warp * (32 * kItems) + lane;
   auto masks = [&](int sp, unsigned &smask, unsigned &lmask, int &lam) {
     smask = lmask = 0u;
     lam = 0;
@@ -1761,9 +1794,9 @@ __global__ void __launch_bounds__(kScanThreads) lo_rank_kernel(Workspace ws, dou
   };
   // the spans, all loads in flight at once; kept in shared memory for the
   // second pass
-  int span[kScanItems];
+  int span[kItems];
 #pragma unroll
-  for (int k = 0; k < kScanItems; ++k) {
+  for (int k = 0; k < kItems; ++k) {
     const int g = g0 + 32 * k;
     span[k] = (g < G) ? ws.gspan[g] : -1;
   }
@@ -1773,7 +1806,7 @@ __global__ void __launch_bounds__(kScanThreads) lo_rank_kernel(Workspace ws, dou
   for (int l = 0; l < kMaxLevels; ++l) cnt[l] = 0;
   int e = 0;
 #pragma unroll
-  for (int k = 0; k < kScanItems; ++k) {
+  for (int k = 0; k < kItems; ++k) {
     s_span[k][tid] = span[k];
     unsigned sm, lm;
     int lam;
@@ -1786,7 +1819,7 @@ __global__ void __launch_bounds__(kScanThreads) lo_rank_kernel(Workspace ws, dou
   // cells, and at the level above (the parent of a group's shallowest cell)
   int wlo = kMaxLevels, whi = -1;
 #pragma unroll
-  for (int k = 0; k < kScanItems; ++k) {
+  for (int k = 0; k < kItems; ++k) {
     if (span[k] < 0) continue;
     const int d = (span[k] & 255) - 1, l = (span[k] >> 8) & 255, dn = ((span[k] >> 16) & 255) - 1;
     wlo = min(wlo, max(0, min(d, dn)));
@@ -1819,7 +1852,7 @@ __global__ void __launch_bounds__(kScanThreads) lo_rank_kernel(Workspace ws, dou
   for (int l = 0; l < kMaxLevels; ++l) run[l] = s_prefix[l] + s_warp[warp][l];
   int nrun = s_prefix[kNodes] + s_warp[warp][kNodes];
 #pragma unroll 1
-  for (int k = 0; k < kScanItems; ++k) {
+  for (int k = 0; k < kItems; ++k) {
     const int g = g0 + 32 * k;
     const int sp = s_span[k][tid];
     // the cell payloads (read before the ranks are formed)
@@ -1978,7 +2011,6 @@ __device__ __forceinline__ bool lo_leaf_cell(const Workspace &ws, int g, int M, 
       wz = __fma_rn(q.w, q.z, wz);
     }
   lo_emit_node(ws, bleaf, tm, wx, wy, wz, c);
-  c.a = ws.pm4[pf];  // the traversal records of a leaf carry its first particle
   const int np = pe - pf;
   if (lo_whole_group(ws, c.level, np, true)) {
     if (c.level == ws.sys_levels) ws.tflag[pf] = 1;
@@ -2009,7 +2041,6 @@ __device__ __forceinline__ LevelNode ld_level_node_cg(const LevelNode *p) {
 // the child list, the target-group marks and its LevelNode; the traversal
 // records are the caller's (lo_emit_records with c).  Returns false on
 // inconsistent input.
-template <int kRecords>
 __device__ __forceinline__ bool lo_level_cell(const Workspace &ws, int level, int b, int hi, int end, int M,
                                               const int4 &f, const int4 &q, int next_first_child, LoCell &c) {
   DevScalars *sc = ws.sc;
@@ -2032,8 +2063,6 @@ __device__ __forceinline__ bool lo_level_cell(const Workspace &ws, int level, in
   c.nk = nk;
   c.leaf = false;
   c.key = (unsigned long long)(unsigned)q.z | ((unsigned long long)(unsigned)q.w << 32);
-  // children in visit order: octant 7 -> 0, the children in descending key order
-  int *kids = (kRecords & kRecordsFp64) ? ws.node_kids + (size_t)pre * 8 : nullptr;
   // target groups (group_mark_kernel's rule): a whole system that is one
   // group, else the starts of the children's runs
   const int np = pe - pf;
@@ -2053,7 +2082,6 @@ __device__ __forceinline__ bool lo_level_cell(const Workspace &ws, int level, in
       wx = __fma_rn(cm, ch.a.x, wx);
       wy = __fma_rn(cm, ch.a.y, wy);
       wz = __fma_rn(cm, ch.a.z, wz);
-      if (kRecords & kRecordsFp64) kids[nk - 1 - j] = ch.pre;
       if (!whole) {
         if (virt) run = 0;
         const int cp = ch.np;
@@ -2069,8 +2097,6 @@ __device__ __forceinline__ bool lo_level_cell(const Workspace &ws, int level, in
       }
     }
   }
-  if (kRecords & kRecordsFp64)
-    for (int j = nk; j < 8; ++j) kids[j] = -1;
   lo_emit_node(ws, b, tm, wx, wy, wz, c);
   return true;
 }
@@ -2118,8 +2144,7 @@ __device__ __forceinline__ bool lo_arrive_last(const Workspace &ws, int c, int p
 // of 256: 170 us; one-warp blocks at 78 registers, 26 per SM: 163 us).
 constexpr int kUpsweepBlock = 32;
 
-template <int kRecords>
-__global__ void __launch_bounds__(kUpsweepBlock, 32) lo_upsweep_kernel(Workspace ws, double theta) {
+__global__ void __launch_bounds__(kUpsweepBlock, 32) lo_upsweep_kernel(Workspace ws) {
   __shared__ int s_g, s_m;
   __shared__ int s_base[kMaxLevels + 2];
   DevScalars *sc = ws.sc;
@@ -2157,7 +2182,6 @@ __global__ void __launch_bounds__(kUpsweepBlock, 32) lo_upsweep_kernel(Workspace
     int pr = cell + 1 < s_base[level + 1] ? ws.lo_first[cell + 1].w : -1;
     while (true) {
       if (level == 0) {
-        if (!lo_emit_records<kRecords>(ws, theta, c)) record_error(sc, kStageGeometry, 2);
         break;
       }
       const int lv = level - 1;
@@ -2174,18 +2198,76 @@ __global__ void __launch_bounds__(kUpsweepBlock, 32) lo_upsweep_kernel(Workspace
       const int npl = p > lo ? ws.lo_first[p - 1].w : -1;
       bool bad;
       const bool last = lo_arrive_last(ws, cell, p, pl, pr, bad);
-      if (!lo_emit_records<kRecords>(ws, theta, c)) record_error(sc, kStageGeometry, 2);
       if (!last) {
         if (bad) record_error(sc, kStageLayout, 1);
         break;
       }
-      if (!lo_level_cell<kRecords>(ws, lv, p, hi, end, M, f, q, fr.y, c)) break;
+      if (!lo_level_cell(ws, lv, p, hi, end, M, f, q, fr.y, c)) break;
       cell = p;
       level = lv;
       p = f.w;
       pl = npl;
       pr = fr.w;
     }
+  }
+}
+
+// The traversal records of every cell, once the upward pass has its mass and
+// centre of mass: a thread per cell, so that the geometry, the acceptance
+// radius and their divisions and square roots are on nobody's climb.
+template <int kRecords>
+__global__ void __launch_bounds__(kBlock) lo_records_kernel(Workspace ws, double theta) {
+  __shared__ int s_base[kMaxLevels + 2];
+  __shared__ int s_m;
+  DevScalars *sc = ws.sc;
+  if (threadIdx.x < kMaxLevels + 2) s_base[threadIdx.x] = sc->level_base[threadIdx.x];
+  if (threadIdx.x == 0) {
+    const int m = sc->n_nodes;
+    s_m = (sc->error || m != sc->level_base[kMaxLevels]) ? 0 : m;
+  }
+  __syncthreads();
+  const int M = s_m;
+  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < M; b += gridDim.x * blockDim.x) {
+    const LevelNode nd = ws.lo_node[b];
+    LoCell c;
+    c.level = 0;
+    while (c.level + 1 < kMaxLevels && b >= s_base[c.level + 1]) ++c.level;
+    c.b = b;
+    c.pre = nd.pre;
+    c.pf = nd.first;
+    c.pe = nd.first + nd.np;
+    c.leaf = nd.leaf != 0;
+    if (c.leaf) {
+      // a leaf's records carry its first particle; its system matters only
+      // where the leaf is a root
+      c.a = ws.pm4[c.pf];
+      c.key = (unsigned long long)(unsigned)(ws.n_systems > 1 ? ws.psys[c.pf] : 0) << kSpatialBits;
+      c.skip = nd.pre + 1;
+      c.c0 = 0;
+      c.nk = 0;
+    } else {
+      const int4 f = ws.lo_first[b], q = ws.lo_last[b];
+      const int hi = s_base[c.level + 1], end = s_base[c.level + 2];
+      c.a = nd.a;
+      c.key = (unsigned long long)(unsigned)q.z | ((unsigned long long)(unsigned)q.w << 32);
+      c.skip = f.z;
+      c.c0 = f.y;
+      c.nk = ((b + 1 < hi) ? ws.lo_first[b + 1].y : end) - c.c0;
+      if (c.c0 < hi || c.nk < 1 || c.nk > 8 || c.c0 + c.nk > end || c.pre < 0 || c.pre >= M) {
+        record_error(sc, kStageLayout, 1);
+        continue;
+      }
+      if (kRecords & kRecordsFp64) {
+        // children in visit order: octant 7 -> 0, in descending key order
+        int kids[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) kids[j] = j < c.nk ? ws.lo_node[c.c0 + c.nk - 1 - j].pre : -1;
+        int4 *dst = reinterpret_cast<int4 *>(ws.node_kids + (size_t)c.pre * 8);
+        dst[0] = make_int4(kids[0], kids[1], kids[2], kids[3]);
+        dst[1] = make_int4(kids[4], kids[5], kids[6], kids[7]);
+      }
+    }
+    if (!lo_emit_records<kRecords>(ws, theta, c)) record_error(sc, kStageGeometry, 2);
   }
 }
 
@@ -2348,21 +2430,25 @@ __global__ void __launch_bounds__(kBlock) pack_keys_kernel(Workspace ws, const u
 
 // ------------------------------------------------------------ launches ---
 
+static void launch_onesweep(const Workspace &ws, const unsigned long long *src, unsigned long long *dst, int pass,
+                            cudaStream_t s) {
+  uint32_t *status = ws.sort_status + (size_t)pass * ws.sort_tiles * 256;
+  const int shift = ws.pack_shift + 8 * pass;
+  if (ws.sort_items == kSortItemsSmall)
+    onesweep_kernel<kSortItemsSmall>
+        <<<ws.sort_tiles, kSortThreads, 0, s>>>(src, dst, ws.n, pass, shift, ws.digit_hist, status, ws.sc);
+  else
+    onesweep_kernel<kSortItems>
+        <<<ws.sort_tiles, kSortThreads, 0, s>>>(src, dst, ws.n, pass, shift, ws.digit_hist, status, ws.sc);
+}
+
 cudaError_t launch_step_reset(Workspace &ws, cudaStream_t s) {
-  reset_scalars_kernel<<<1, 32, 0, s>>>(ws.sc);
-  reset_sys_kernel<<<(6 * ws.n_systems + 255) / 256, 256, 0, s>>>(ws.sys_bb, ws.n_systems);
-  count_launches(2);
-  cudaError_t e = cudaMemsetAsync(ws.digit_hist, 0, sizeof(uint32_t) * kMaxSortPasses * 256, s);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(ws.sort_status, 0, sizeof(uint32_t) * (size_t)ws.sort_passes * ws.sort_tiles * 256, s);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(ws.scan_status, 0,
-                      sizeof(unsigned long long) * (size_t)(3 * ws.scan_tiles_n + ws.scan_tiles_r), s);
-  if (e != cudaSuccess) return e;
-  if (ws.tflag) {
-    e = cudaMemsetAsync(ws.tflag, 0, (size_t)ws.n, s);
-    if (e != cudaSuccess) return e;
-  }
+  // one 16-byte word per thread of the largest array, up to a full GPU
+  const size_t words = std::max((size_t)ws.n / 16, (size_t)ws.sort_passes * ws.sort_tiles * 64);
+  const int cap = grid_for(ws, 8);
+  const int blocks = (int)std::min((size_t)cap, words / kBlock + 1);
+  step_reset_kernel<<<blocks, kBlock, 0, s>>>(ws);
+  count_launches(1);
   return cudaGetLastError();
 }
 
@@ -2387,9 +2473,7 @@ cudaError_t launch_morton_sort_groups(Workspace &ws, cudaStream_t s, int part) {
     encode_kernel<<<blocks, kBlock, 0, s>>>(ws);
     unsigned long long *src = ws.pairs_a, *dst = ws.pairs_b;
     for (int p = 0; p < ws.sort_passes; ++p) {
-      onesweep_kernel<<<ws.sort_tiles, kSortThreads, 0, s>>>(
-          src, dst, ws.n, p, ws.pack_shift + 8 * p, ws.digit_hist,
-          ws.sort_status + (size_t)p * ws.sort_tiles * 256, ws.sc);
+      launch_onesweep(ws, src, dst, p, s);
       unsigned long long *t = src;
       src = dst;
       dst = t;
@@ -2443,24 +2527,30 @@ cudaError_t launch_tree(Workspace &ws, double theta, cudaStream_t s) {
 
 cudaError_t launch_level_order_tree(Workspace &ws, double theta, cudaStream_t s) {
   if (!ws.lo_tiles) return cudaErrorInvalidValue;
-  lo_span_kernel<<<ws.scan_tiles_n, kScanThreads, 0, s>>>(ws);
-  lo_tile_scan_kernel<<<1, 32 * kLevelOrderChannels, 0, s>>>(ws);
-  if (ws.records == kRecordsMixed)
-    lo_rank_kernel<kRecordsMixed><<<ws.scan_tiles_n, kScanThreads, 0, s>>>(ws, theta);
+  if (ws.lo_items == kScanItems)
+    lo_span_kernel<kScanItems><<<ws.lo_tile_count, kScanThreads, 0, s>>>(ws);
   else
-    lo_rank_kernel<kRecordsFp64><<<ws.scan_tiles_n, kScanThreads, 0, s>>>(ws, theta);
+    lo_span_kernel<1><<<ws.lo_tile_count, kScanThreads, 0, s>>>(ws);
+  lo_tile_scan_kernel<<<1, 32 * kLevelOrderChannels, 0, s>>>(ws);
+  if (ws.lo_items == kScanItems)
+    lo_rank_kernel<kScanItems><<<ws.lo_tile_count, kScanThreads, 0, s>>>(ws);
+  else
+    lo_rank_kernel<1><<<ws.lo_tile_count, kScanThreads, 0, s>>>(ws);
   // leaves and every internal cell in one launch (arrival counters), one
   // thread per group in one-warp blocks (a resident grid taking groups
   // grid-stride measured slower: 267 against 174 us at 2^20 particles)
   const int want = (ws.n + kUpsweepBlock - 1) / kUpsweepBlock;
   const int up_grid = want > 0 ? want : 1;
+  lo_upsweep_kernel<<<up_grid, kUpsweepBlock, 0, s>>>(ws);
+  int rec_grid = (ws.n + ws.n / 2 + kBlock - 1) / kBlock;  // about the cells there are
+  rec_grid = std::max(1, std::min(rec_grid, grid_for(ws, 8)));
   if (ws.records == kRecordsMixed)
-    lo_upsweep_kernel<kRecordsMixed><<<up_grid, kUpsweepBlock, 0, s>>>(ws, theta);
+    lo_records_kernel<kRecordsMixed><<<rec_grid, kBlock, 0, s>>>(ws, theta);
   else
-    lo_upsweep_kernel<kRecordsFp64><<<up_grid, kUpsweepBlock, 0, s>>>(ws, theta);
+    lo_records_kernel<kRecordsFp64><<<rec_grid, kBlock, 0, s>>>(ws, theta);
   // target-group marks were set by the upward pass
   group_scan_kernel<<<ws.scan_tiles_n, kScanThreads, 0, s>>>(ws);
-  count_launches(5);
+  count_launches(6);
   return cudaGetLastError();
 }
 
@@ -2495,9 +2585,7 @@ cudaError_t launch_morton_sort_only(Workspace &ws, uint32_t *keys, uint32_t *idx
   encode_kernel<<<blocks, kBlock, 0, s>>>(ws);
   unsigned long long *src = ws.pairs_a, *dst = ws.pairs_b;
   for (int p = 0; p < ws.sort_passes; ++p) {
-    onesweep_kernel<<<ws.sort_tiles, kSortThreads, 0, s>>>(
-        src, dst, ws.n, p, ws.pack_shift + 8 * p, ws.digit_hist,
-        ws.sort_status + (size_t)p * ws.sort_tiles * 256, ws.sc);
+    launch_onesweep(ws, src, dst, p, s);
     unsigned long long *t = src;
     src = dst;
     dst = t;

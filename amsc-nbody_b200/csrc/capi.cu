@@ -237,7 +237,8 @@ cudaError_t alloc_workspace(Workspace &ws, Allocation &al, int n, const Workspac
   GET(ws.sys_bb, 6 * S); GET(ws.sys_box, 4 * S); GET(ws.root_pre, S); GET(ws.root_lo, S);
   GET(ws.pairs_a, N); GET(ws.pairs_b, N);
   GET(ws.digit_hist, (size_t)kMaxSortPasses * 256);
-  ws.sort_tiles = (n + kSortTile - 1) / kSortTile;
+  ws.sort_items = n <= kSmallTiles ? kSortItemsSmall : kSortItems;
+  ws.sort_tiles = (n + kSortThreads * ws.sort_items - 1) / (kSortThreads * ws.sort_items);
   GET(ws.sort_status, (size_t)ws.sort_passes * ws.sort_tiles * 256);
   ws.scan_tiles_n = (n + kScanTile - 1) / kScanTile;
   ws.scan_tiles_r = (2 * n - 1 + kScanTile - 1) / kScanTile;
@@ -269,7 +270,9 @@ cudaError_t alloc_workspace(Workspace &ws, Allocation &al, int n, const Workspac
     GET(ws.gspan, N);
     GET(ws.lo_first, C); GET(ws.lo_arrive, C); GET(ws.lo_last, C); GET(ws.lo_node, C); GET(ws.lo_gleaf, N);
     GET(ws.pos4, N);
-    GET(ws.lo_tiles, (size_t)ws.scan_tiles_n * kLevelOrderChannels);
+    ws.lo_items = n <= kSmallTiles ? 1 : kScanItems;
+    ws.lo_tile_count = (n + kScanThreads * ws.lo_items - 1) / (kScanThreads * ws.lo_items);
+    GET(ws.lo_tiles, (size_t)ws.lo_tile_count * kLevelOrderChannels);
   }
 #undef GET
   e = ar.take(al);

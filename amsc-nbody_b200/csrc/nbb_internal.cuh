@@ -57,6 +57,14 @@ struct DevScalars {
 constexpr int kSortThreads = 256;
 constexpr int kSortItems = 16;
 constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 pairs
+// Small inputs are sorted in tiles of two pairs per thread and numbered in
+// tiles of one group per thread: a thread's items are worked off one after
+// another, which is all the time these kernels take while few tiles exist.
+// One pass / the numbering: 12.5 / 27 us in large tiles, 7 / 9 us in small
+// ones at 4096 particles, 14 / 27 and 9 / 11 at 65536; large tiles are the
+// faster from about 2^18 on.
+constexpr int kSortItemsSmall = 2;
+constexpr int kSmallTiles = 131072;  // particles up to which the small tiles are taken
 constexpr int kSortPasses = 4;     // 8-bit digits over a single system's 30-bit keys
 constexpr int kMaxSortPasses = 5;  // ensemble keys: up to 9 system bits + 30 Morton bits
 constexpr int kMaxLevels = 16;     // octree levels: 10 spatial + up to 3 above the system roots
@@ -116,7 +124,7 @@ static_assert(sizeof(LevelNode) == 48, "two 32-byte sectors per node");
 constexpr int kTopDepth = 2;
 constexpr int kTopMax = 73;
 
-// Per-tile counts of the level-order build (tiles of kScanTile groups): the
+// Per-tile counts of the level-order build (tiles of kScanThreads * lo_items groups): the
 // cells started per octree level, then the cells ended (kMaxLevels); the
 // rest pad a warp.
 constexpr int kLevelOrderChannels = 32;
@@ -168,6 +176,7 @@ struct Workspace {
   uint32_t *digit_hist = nullptr;    // kSortPasses * 256 (counts -> offsets)
   uint32_t *sort_status = nullptr;   // kSortPasses * tiles * 256
   int sort_tiles = 0;
+  int sort_items = kSortItems;       // pairs per thread of a tile: kSortItems or kSortItemsSmall
   unsigned long long *scan_status = nullptr;  // scan tiles: groups, plan, target groups
   int scan_tiles_n = 0;   // tiles over n
   int scan_tiles_r = 0;   // tiles over 2n-1
@@ -224,7 +233,9 @@ struct Workspace {
   int2 *lo_gleaf = nullptr;     // n: per group, its leaf's level-order index and S(g)
   double4 *pos4 = nullptr;      // n: {x, y, z, -} in original order, written by the kick-drift pass
   LevelNode *lo_node = nullptr;  // cap: mass, centre of mass, preorder index, particles
-  int *lo_tiles = nullptr;      // scan_tiles_n * kLevelOrderChannels: per-tile counts, then their prefixes
+  int lo_items = 0;             // groups per thread of a numbering tile: kScanItems or 1
+  int lo_tile_count = 0;        // numbering tiles over n
+  int *lo_tiles = nullptr;      // lo_tile_count * kLevelOrderChannels: per-tile counts, then their prefixes
   int records = kRecordsFp64 | kRecordsMixed;  // host: the records the level-order build writes
   int *walk_ext = nullptr;    // walk_warps x walk_ext_cap: the mixed walk's stack below shared memory
 };
