@@ -142,6 +142,7 @@ struct Workspace {
   int fp64_grid[2] = {0, 0};  // persistent traversal grids (blocks): 32 and 1 targets per warp
   int mixed_grid[2][3] = {{0, 0, 0}, {0, 0, 0}};  // [track source][1, 2 or 4 targets per lane]
   int vjp_grid = 0;     // the mixed walk's adjoint form
+  int split_grid[3] = {0, 0, 0};  // the mixed walk with a group per block: force [track source], adjoint
   int walk_warps = 0;     // warps of the largest mixed-walk grid
   int walk_ext_cap = 0;   // entries per warp of the mixed walk's stack extension
   int group_max = 32;   // largest octree target group: 32, 64 or 128 (32 x target slots per lane)

@@ -303,14 +303,19 @@ struct PairList {
   }
 };
 
-template <bool kTrackSource>
+// Warps of a block: kMixedWarps with a group each, or kSplit on one group.
+template <int kSplit>
+__host__ __device__ constexpr int mixed_warps() {
+  return kSplit > 1 ? kSplit : kMixedWarps;
+}
+template <bool kTrackSource, int kWarps>
 struct MixedShared {
-  double gbox[kMixedWarps][9];  // group box lo (3), hi (3), centre (3)
-  float ghalf[kMixedWarps][4];  // group box half extents, rounded up to FP32
-  int stack[kMixedWarps][kStackCap];
-  float4 la[kMixedWarps][list_cap_of<kTrackSource>() / 2];
-  float4 lb[kMixedWarps][list_cap_of<kTrackSource>() / 2];
-  int src[kMixedWarps][kTrackSource ? list_cap_of<kTrackSource>() : 1];
+  double gbox[kWarps][9];  // group box lo (3), hi (3), centre (3)
+  float ghalf[kWarps][4];  // group box half extents, rounded up to FP32
+  int stack[kWarps][kStackCap];
+  float4 la[kWarps][list_cap_of<kTrackSource>() / 2];
+  float4 lb[kWarps][list_cap_of<kTrackSource>() / 2];
+  int src[kWarps][kTrackSource ? list_cap_of<kTrackSource>() : 1];
 };
 
 // Hardware approximate reciprocal square root (MUFU), subnormal inputs and
@@ -619,17 +624,28 @@ __device__ __forceinline__ bool accept_box(const double4 &a, const double *gbox,
 // FP64, then rounded) and are evaluated by all lanes in batches of 32.
 // With kVjp (one target per lane, sources tracked) the same walk evaluates
 // the vector-Jacobian product above instead of the force.
-template <bool kTrackSource, int kTPL, bool kVjp = false>
-__global__ void __launch_bounds__(kMixedWarps * 32,
-                                   kTPL >= 4 ? NBB_MIXED_MINBLOCKS4 : (kTPL == 2 ? NBB_MIXED_MINBLOCKS2 : NBB_MIXED_MINBLOCKS))
+//
+// With kSplit > 1 the block's warps share one group: each walks from the root
+// until kDeal nodes are pending, then keeps every kSplit-th of them, and the
+// targets' sums are added at the end.  This is for systems with too few groups
+// to fill the GPU, where a walk is a chain of ~45 rounds of 2 us.
+constexpr int kDeal = 48;
+
+template <bool kTrackSource, int kTPL, bool kVjp = false, int kSplit = 1>
+__global__ void __launch_bounds__(mixed_warps<kSplit>() * 32,
+                                  kSplit > 1 ? 20 / kSplit
+                                             : (kTPL >= 4 ? NBB_MIXED_MINBLOCKS4 : (kTPL == 2 ? NBB_MIXED_MINBLOCKS2 : NBB_MIXED_MINBLOCKS)))
     traverse_mixed_kernel(Workspace ws, TraversalParams p, AdjointBuffers ab) {
   static_assert(!kVjp || (kTrackSource && kTPL == 1), "the adjoint walk tracks sources, one target per lane");
-  __shared__ MixedShared<kTrackSource> sh;
+  static_assert(kSplit == 1 || kTPL == 1, "a shared group has one target per lane");
+  __shared__ MixedShared<kTrackSource, mixed_warps<kSplit>()> sh;
+  __shared__ double s_part[kSplit > 1 ? kSplit - 1 : 1][3][kSplit > 1 ? 32 : 1];  // the other warps' sums
+  __shared__ int s_group;
   // node cache: the top cache_depth levels below the root (the first entries
   // of the level order), loaded once per block
   __shared__ MixedNode c_rec[kTopMax];
   DevScalars *sc = ws.sc;
-  if (sc->error) return;
+  if (kSplit > 1 ? __syncthreads_or(sc->error != 0) != 0 : sc->error != 0) return;
   const int lane = threadIdx.x & 31;
   const int wid = threadIdx.x >> 5;
   int *stack = sh.stack[wid];
@@ -651,11 +667,19 @@ __global__ void __launch_bounds__(kMixedWarps * 32,
   bool singular_any = false;
   while (true) {
     int grp = 0;
-    if (lane == 0) grp = (int)atomicAdd(&sc->work_counter, 1u);
-    grp = __shfl_sync(kFull, grp, 0);
+    if constexpr (kSplit > 1) {
+      if (threadIdx.x == 0) s_group = (int)atomicAdd(&sc->work_counter, 1u);
+      __syncthreads();
+      grp = s_group;
+    } else {
+      if (lane == 0) grp = (int)atomicAdd(&sc->work_counter, 1u);
+      grp = __shfl_sync(kFull, grp, 0);
+    }
     if (grp >= n_groups) break;
     const int g0 = ws.tstart[grp];
     const int g1 = (grp + 1 < n_groups) ? ws.tstart[grp + 1] : n;
+    bool dealt = kSplit == 1;
+    const long long tests_before = tests;
     const int nq = min(kTPL, max(1, (g1 - g0 + 31) >> 5));  // occupied target slots
     LaneTargets<kTPL> T;
     LaneVjp V;
@@ -739,10 +763,26 @@ __global__ void __launch_bounds__(kMixedWarps * 32,
     int *ext = nullptr;
     int esp = 0;
     {
-      const int gw = blockIdx.x * kMixedWarps + wid;
+      const int gw = blockIdx.x * mixed_warps<kSplit>() + wid;
       if (ws.walk_ext && gw < ws.walk_warps) ext = ws.walk_ext + (size_t)gw * ws.walk_ext_cap;
     }
     while (sp > 0 || esp > 0) {
+      if (kSplit > 1 && !dealt && sp >= kDeal) {
+        const int own = (sp - wid + kSplit - 1) / kSplit;
+        for (int c = 0; c < own; c += 32) {
+          // (the sources start at or after the destinations)
+          const int i = c + lane;
+          const int v = i < own ? stack[i * kSplit + wid] : 0;
+          __syncwarp();
+          if (i < own) stack[i] = v;
+          __syncwarp();
+        }
+        sp = own;
+        dealt = true;
+        if (wid > 0) tests = tests_before;
+      }
+      // until then every warp walks the same nodes, and only the first lists
+      const bool mute = kSplit > 1 && !dealt && wid > 0;
       if (sp > kStackCap - 7 * kWalkPop && ext && esp + kSpill <= ws.walk_ext_cap) {
         for (int i = lane; i < kSpill; i += 32) ext[esp + i] = stack[i];
         __syncwarp();
@@ -862,9 +902,10 @@ __global__ void __launch_bounds__(kMixedWarps * 32,
         if (kTrackSource) src[pos] = kVjp ? -3 - n1 : -1;
       }
       ls += __popc(cm0) + __popc(cm1);
+      if (mute) ls = 0;
       // reached leaves -> their particles: all at once when they fit
-      const int lc0 = (cat0 == 2) ? m0.z : 0;
-      const int lc1 = (cat1 == 2) ? m1.z : 0;
+      const int lc0 = (cat0 == 2 && !mute) ? m0.z : 0;
+      const int lc1 = (cat1 == 2 && !mute) ? m1.z : 0;
       int lexcl, ltotal;
       if (__all_sync(kFull, lc0 < 16 && lc1 < 16)) {
         lexcl = warp_prefix_small<5>(lc0 + lc1, lt, ltotal);
@@ -934,6 +975,7 @@ __global__ void __launch_bounds__(kMixedWarps * 32,
         }
       }
     }
+    if (kSplit > 1 && !dealt && wid > 0) tests = tests_before;
     if (ls > 0) {
       if (ls & 1) {
         // complete the last pair with a zero-mass entry far away (its
@@ -958,15 +1000,29 @@ __global__ void __launch_bounds__(kMixedWarps * 32,
         }
     }
     __syncwarp();
+    // the group's sums: the other warps' parts are added in warp order
+    double part[3] = {0.0, 0.0, 0.0};
+    if constexpr (kSplit > 1) {
+      if (wid > 0) {
+        s_part[wid - 1][0][lane] = kVjp ? V.gx : (double)T.sum[0].x - (double)T.comp[0].x;
+        s_part[wid - 1][1][lane] = kVjp ? V.gy : (double)T.sum[0].y - (double)T.comp[0].y;
+        s_part[wid - 1][2][lane] = kVjp ? V.gz : (double)T.sum[0].z - (double)T.comp[0].z;
+      }
+      __syncthreads();
+      if (wid == 0)
+        for (int w = 0; w < kSplit - 1; ++w)
+          for (int c = 0; c < 3; ++c) part[c] += s_part[w][c][lane];
+    }
     if constexpr (kVjp) {
-      if (T.valid[0]) ab.tgt_g[T.s[0]] = make_double4(V.gx, V.gy, V.gz, 0.0);
+      if (T.valid[0] && (kSplit == 1 || wid == 0))
+        ab.tgt_g[T.s[0]] = make_double4(V.gx + part[0], V.gy + part[1], V.gz + part[2], 0.0);
     }
 #pragma unroll
     for (int q = 0; q < kTPL; ++q) {
-      if (kVjp || !T.valid[q]) continue;
-      const double ax = p.g * ((double)T.sum[q].x - (double)T.comp[q].x);
-      const double ay = p.g * ((double)T.sum[q].y - (double)T.comp[q].y);
-      const double az = p.g * ((double)T.sum[q].z - (double)T.comp[q].z);
+      if (kVjp || !T.valid[q] || (kSplit > 1 && wid > 0)) continue;
+      const double ax = p.g * ((double)T.sum[q].x - (double)T.comp[q].x + part[0]);
+      const double ay = p.g * ((double)T.sum[q].y - (double)T.comp[q].y + part[1]);
+      const double az = p.g * ((double)T.sum[q].z - (double)T.comp[q].z + part[2]);
       const uint32_t ti = ws.idx[T.s[q]];
       ws.ax[ti] = ax;
       ws.ay[ti] = ay;
@@ -1309,6 +1365,13 @@ static cudaError_t grid_of(K kernel, int threads, int sms, int &grid) {
   return e;
 }
 
+// Whether the mixed walk of n particles in groups of at most 32 gives a group
+// to four warps: while one warp each leaves the GPU unfilled.  Walk of Plummer
+// spheres, one / four warps: 48 / 30 us at 1000 particles, 95 / 60 at 4096,
+// 165 / 103 at 16384, 208 / 165 at 32768, 232 / 337 at 65536.
+constexpr int kMixedSplit = 4;
+static bool split_group(int n) { return n < 40000; }
+
 cudaError_t configure_traversal(Workspace &ws) {
   const int sms = ws.num_sms > 0 ? ws.num_sms : 148;
   cudaError_t e = grid_of(traverse_fp64_kernel<32>, kFp64Warps * 32, sms, ws.fp64_grid[0]);
@@ -1320,6 +1383,10 @@ cudaError_t configure_traversal(Workspace &ws) {
   if (e == cudaSuccess) e = grid_of(traverse_mixed_kernel<false, 4>, kMixedWarps * 32, sms, ws.mixed_grid[0][2]);
   if (e == cudaSuccess) e = grid_of(traverse_mixed_kernel<true, 4>, kMixedWarps * 32, sms, ws.mixed_grid[1][2]);
   if (e == cudaSuccess) e = grid_of(traverse_mixed_kernel<true, 1, true>, kMixedWarps * 32, sms, ws.vjp_grid);
+  constexpr int kSplitThreads = 32 * kMixedSplit;
+  if (e == cudaSuccess) e = grid_of(traverse_mixed_kernel<false, 1, false, kMixedSplit>, kSplitThreads, sms, ws.split_grid[0]);
+  if (e == cudaSuccess) e = grid_of(traverse_mixed_kernel<true, 1, false, kMixedSplit>, kSplitThreads, sms, ws.split_grid[1]);
+  if (e == cudaSuccess) e = grid_of(traverse_mixed_kernel<true, 1, true, kMixedSplit>, kSplitThreads, sms, ws.split_grid[2]);
   // The stack extension holds a whole walk: the stack stays sorted by tree
   // level (a round pops the top and pushes children one level deeper), and
   // a level's entries are pushed only after every older entry of that level
@@ -1330,6 +1397,7 @@ cudaError_t configure_traversal(Workspace &ws) {
   for (int t = 0; t < 2; ++t)
     for (int q = 0; q < 3; ++q) blocks = std::max(blocks, ws.mixed_grid[t][q]);
   ws.walk_warps = blocks * kMixedWarps;
+  for (int t = 0; t < 3; ++t) ws.walk_warps = std::max(ws.walk_warps, ws.split_grid[t] * kMixedSplit);
   ws.walk_ext_cap = std::min(8 * kWalkPop * (ws.max_level + 1), std::max(ws.cap_nodes, 1));
   return e;
 }
@@ -1344,7 +1412,10 @@ cudaError_t launch_traversal(Workspace &ws, const TraversalParams &p, cudaStream
       traverse_fp64_kernel<32><<<ws.fp64_grid[0] > 0 ? ws.fp64_grid[0] : 148, kFp64Warps * 32, 0, s>>>(ws, p);
     else
       traverse_fp64_kernel<1><<<ws.fp64_grid[1] > 0 ? ws.fp64_grid[1] : 148, kFp64Warps * 32, 0, s>>>(ws, p);
-  } else if (slot == 0)
+  } else if (slot == 0 && split_group(ws.n))
+    (track ? traverse_mixed_kernel<true, 1, false, kMixedSplit> : traverse_mixed_kernel<false, 1, false, kMixedSplit>)
+        <<<ws.split_grid[track] > 0 ? ws.split_grid[track] : 148, 32 * kMixedSplit, 0, s>>>(ws, p, AdjointBuffers{});
+  else if (slot == 0)
     (track ? traverse_mixed_kernel<true, 1> : traverse_mixed_kernel<false, 1>)<<<grid, kMixedWarps * 32, 0, s>>>(
         ws, p, AdjointBuffers{});
   else if (slot == 1)
@@ -1364,7 +1435,11 @@ cudaError_t launch_adjoint_mixed(Workspace &ws, const TraversalParams &p, const 
   if (ws.walk_warps > 0 && grid * kMixedWarps > ws.walk_warps) grid = ws.walk_warps / kMixedWarps;
   TraversalParams q = p;
   q.cache_depth = 0;
-  traverse_mixed_kernel<true, 1, true><<<grid, kMixedWarps * 32, 0, s>>>(ws, q, ab);
+  if (split_group(ws.n))
+    traverse_mixed_kernel<true, 1, true, kMixedSplit>
+        <<<ws.split_grid[2] > 0 ? ws.split_grid[2] : 148, 32 * kMixedSplit, 0, s>>>(ws, q, ab);
+  else
+    traverse_mixed_kernel<true, 1, true><<<grid, kMixedWarps * 32, 0, s>>>(ws, q, ab);
   count_launches(1);
   return cudaGetLastError();
 }
