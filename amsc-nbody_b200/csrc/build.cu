@@ -2020,27 +2020,11 @@ __device__ __forceinline__ bool lo_leaf_cell(const Workspace &ws, int g, int M, 
   return true;
 }
 
-// A child's LevelNode, written earlier in the same kernel by another thread
-// of the upward pass: read from L2 (ld.global.cg), never from a stale L1 line.
-__device__ __forceinline__ LevelNode ld_level_node_cg(const LevelNode *p) {
-  const double2 *d = reinterpret_cast<const double2 *>(p);
-  const double2 lo = __ldcg(d), hi = __ldcg(d + 1);
-  const int4 t = __ldcg(reinterpret_cast<const int4 *>(p) + 2);
-  LevelNode r;
-  r.a = make_double4(lo.x, lo.y, hi.x, hi.y);
-  r.pre = t.x;
-  r.np = t.y;
-  r.first = t.z;
-  r.leaf = t.w;
-  return r;
-}
-
 // One internal cell b of a level (children in the next level's range
 // [hi, end); f, q its lo_first and lo_last entries): mass and centre of mass
 // from the children's records in octant order (octree_physics.cu:156-245),
-// the child list, the target-group marks and its LevelNode; the traversal
-// records are the caller's (lo_emit_records with c).  Returns false on
-// inconsistent input.
+// the target-group marks and its LevelNode.  Returns false on inconsistent
+// input.
 __device__ __forceinline__ bool lo_level_cell(const Workspace &ws, int level, int b, int hi, int end, int M,
                                               const int4 &f, const int4 &q, int next_first_child, LoCell &c) {
   DevScalars *sc = ws.sc;
@@ -2071,33 +2055,51 @@ __device__ __forceinline__ bool lo_level_cell(const Workspace &ws, int level, in
   const bool virt = level < ws.sys_levels;
   const bool merge = !virt && (np <= 1 || level - ws.sys_levels >= ws.group_depth);
   const bool child_compact_level = level + 1 - ws.sys_levels >= ws.group_depth;
-  int run = 0;
+  // the children first, the marks after: a store between two children's
+  // loads would keep them from being in flight together
   double tm = 0.0, wx = 0.0, wy = 0.0, wz = 0.0;
+  int4 kid[8];  // preorder index, particles, first particle, leaf
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    if (c0 + j < c1) {
-      const LevelNode ch = ld_level_node_cg(ws.lo_node + c0 + j);
-      const double cm = ch.a.w;
-      tm = __dadd_rn(tm, cm);
-      wx = __fma_rn(cm, ch.a.x, wx);
-      wy = __fma_rn(cm, ch.a.y, wy);
-      wz = __fma_rn(cm, ch.a.z, wz);
-      if (!whole) {
-        if (virt) run = 0;
-        const int cp = ch.np;
-        if (cp > ws.group_max || !(ch.leaf || cp <= 1 || child_compact_level)) {
-          run = 0;  // the child splits itself
-        } else {
-          if (!merge || run == 0 || run + cp > ws.group_max) {
-            if (ch.first >= 0 && ch.first < ws.n) ws.tflag[ch.first] = 1;
-            run = 0;
-          }
-          run += cp;
-        }
-      }
+  for (int h = 0; h < 8; h += 4) {
+    double2 lo[4], hi2[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      // (a cell past the last child is read in the last child's place)
+      const LevelNode *src = ws.lo_node + min(c0 + h + j, c1 - 1);
+      const double2 *d = reinterpret_cast<const double2 *>(src);
+      lo[j] = __ldcg(d);
+      hi2[j] = __ldcg(d + 1);
+      kid[h + j] = __ldcg(reinterpret_cast<const int4 *>(src) + 2);
     }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (c0 + h + j < c1) {
+        const double cm = hi2[j].y;
+        tm = __dadd_rn(tm, cm);
+        wx = __fma_rn(cm, lo[j].x, wx);
+        wy = __fma_rn(cm, lo[j].y, wy);
+        wz = __fma_rn(cm, hi2[j].x, wz);
+      }
+    if (c0 + h + 4 >= c1) break;
   }
   lo_emit_node(ws, b, tm, wx, wy, wz, c);
+  if (whole) return true;
+  int run = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    if (c0 + j >= c1) break;
+    if (virt) run = 0;
+    const int cp = kid[j].y;
+    if (cp > ws.group_max || !(kid[j].w || cp <= 1 || child_compact_level)) {
+      run = 0;  // the child splits itself
+    } else {
+      if (!merge || run == 0 || run + cp > ws.group_max) {
+        if (kid[j].z >= 0 && kid[j].z < ws.n) ws.tflag[kid[j].z] = 1;
+        run = 0;
+      }
+      run += cp;
+    }
+  }
   return true;
 }
 
@@ -2134,14 +2136,14 @@ __device__ __forceinline__ bool lo_arrive_last(const Workspace &ws, int c, int p
 // cell is finished exactly once, after all of its children, with the same
 // arithmetic in the same child order as a level-by-level pass.  No thread
 // ever waits: a climb ends at the root, at a parent that other children
-// still owe, or at the first inconsistency.  What keeps the climb short: a
-// cell's traversal records (geometry, acceptance radius, the scattered
-// writes at the preorder index) are written after its arrival, not before;
-// the parent's entries are read before the arrival; and a block is one warp
-// (32 resident per SM, 64 registers), so a warp whose lanes climb far holds
-// no other warp's slot.  Measured at 2^20 particles (kernel time, cold):
-// 174 us before these three changes, 152 us after (blocks of 64: 156 us,
-// of 256: 170 us; one-warp blocks at 78 registers, 26 per SM: 163 us).
+// still owe, or at the first inconsistency.  What keeps the climb short: the
+// parent's entries are read before the arrival, the traversal records are
+// lo_records_kernel's, and a block is one warp (32 resident per SM, 64
+// registers), so a warp whose lanes climb far holds no other warp's slot
+// (blocks of 64 and 256 measured 3 and 12 % slower).  Still a level costs the
+// climber about 3 us: two round trips to L2, a release that waits for its
+// writes, an atomic and the combination; 120 us at 2^20 particles, 30 at 4096
+// (a cluster of 8 blocks with a barrier per level took 44 there).
 constexpr int kUpsweepBlock = 32;
 
 __global__ void __launch_bounds__(kUpsweepBlock, 32) lo_upsweep_kernel(Workspace ws) {
