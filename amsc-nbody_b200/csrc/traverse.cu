@@ -570,40 +570,26 @@ __device__ __forceinline__ void flush_full(const PairList &list, int *src, int &
   }
 }
 
-// Exclusive prefix sum over the warp of a small count v in [0, 2^kBits):
-// one ballot per bit, no chain of dependent shuffles.  `total` receives the
-// warp's sum (one warp reduction instead of a population count per bit: the
-// XU pipe that counts bits also runs the walk's reciprocal square roots).
-template <int kBits>
-__device__ __forceinline__ int warp_prefix_small(int v, unsigned lt, int &total) {
-  int excl = 0;
-#pragma unroll
-  for (int b = 0; b < kBits; ++b) {
-    const unsigned m = __ballot_sync(kFull, (v >> b) & 1);
-    excl += __popc(m & lt) << b;
-  }
-  total = __reduce_add_sync(kFull, v);
-  return excl;
-}
-
-// The group-box acceptance test of the mixed walk, in FP32.  The node's
-// centre of mass is taken relative to the group centre in FP64 and rounded
-// (the list entry's offset, returned in e); the squared distance from the
+// The group-box acceptance test of the mixed walk, in FP32, of a node with
+// list entry e; the squared distance from the
 // box (half extents rounded up) to that point is computed in FP32 and shrunk
 // by 2^-20 so that it never exceeds the exact FP64 distance, and cr2 is the
 // exact squared radius rounded up with a 2^-18 margin.  An accepted node is
 // therefore accepted by the exact test for every target in the box; a node
 // within the margins is opened instead (more work, never less accuracy).
-__device__ __forceinline__ bool accept_box(const double4 &a, const double *gbox, const float *ghalf, float cr2,
-                                           float4 &e) {
-  const float ox = (float)(a.x - gbox[6]), oy = (float)(a.y - gbox[7]), oz = (float)(a.z - gbox[8]);
+__device__ __forceinline__ bool accept_box(const float4 &e, const float *ghalf, float cr2) {
   constexpr float kShrink = 1.0f - 0x1p-20f;
-  const float ex = fmaxf(0.f, fmaf(fabsf(ox), kShrink, -ghalf[0]));
-  const float ey = fmaxf(0.f, fmaf(fabsf(oy), kShrink, -ghalf[1]));
-  const float ez = fmaxf(0.f, fmaf(fabsf(oz), kShrink, -ghalf[2]));
+  const float ex = fmaxf(0.f, fmaf(fabsf(e.x), kShrink, -ghalf[0]));
+  const float ey = fmaxf(0.f, fmaf(fabsf(e.y), kShrink, -ghalf[1]));
+  const float ez = fmaxf(0.f, fmaf(fabsf(e.z), kShrink, -ghalf[2]));
   const float d2 = fmaf(ez, ez, fmaf(ey, ey, ex * ex)) * kShrink;
-  e = make_float4(ox, oy, oz, (float)a.w);
   return d2 > cr2;
+}
+
+// The list entry of a source: its offset from the group centre (formed in
+// FP64, then rounded) and its mass.
+__device__ __forceinline__ float4 list_entry(const double4 &a, const double *gbox) {
+  return make_float4((float)(a.x - gbox[6]), (float)(a.y - gbox[7]), (float)(a.z - gbox[8]), (float)a.w);
 }
 
 // Mixed-precision traversal, one warp per target group of at most 32 x kTPL
@@ -831,31 +817,16 @@ __global__ void __launch_bounds__(mixed_warps<kSplit>() * 32,
         }
       }
       const float cr0 = __int_as_float(m0.x), cr1 = __int_as_float(m1.x);  // squared acceptance radius for a target box
-      // 0 nothing, 1 accepted cell, 2 leaf, 3 open; the cell's list entry
-      // (centre of mass offset from the group centre, mass) in FP32
+      // 0 nothing, 1 accepted cell, 2 leaf, 3 open; a leaf's record carries
+      // its first particle, so every node has a list entry
       int cat0 = 0, cat1 = 0;
-      float4 e0 = make_float4(0.f, 0.f, 0.f, 0.f), e1 = e0;
+      const float4 e0 = list_entry(a0, gbox), e1 = list_entry(a1, gbox);
       {
-        const double4 a = a0;
-        if (n0 >= 0) {
-          if (m0.z > 0) {
-            cat0 = 2;
-          } else if (a.w != 0.0) {
-            ++tests;
-            cat0 = accept_box(a, gbox, sh.ghalf[wid], cr0, e0) ? 1 : 3;
-          }
-        }
-      }
-      {
-        const double4 a = a1;
-        if (n1 >= 0) {
-          if (m1.z > 0) {
-            cat1 = 2;
-          } else if (a.w != 0.0) {
-            ++tests;
-            cat1 = accept_box(a, gbox, sh.ghalf[wid], cr1, e1) ? 1 : 3;
-          }
-        }
+        const bool far0 = accept_box(e0, sh.ghalf[wid], cr0), far1 = accept_box(e1, sh.ghalf[wid], cr1);
+        const bool cell0 = m0.z <= 0 && a0.w != 0.0, cell1 = m1.z <= 0 && a1.w != 0.0;
+        if (n0 >= 0) cat0 = m0.z > 0 ? 2 : (cell0 ? (far0 ? 1 : 3) : 0);
+        if (n1 >= 0) cat1 = m1.z > 0 ? 2 : (cell1 ? (far1 ? 1 : 3) : 0);
+        tests += (n0 >= 0 && cell0 ? 1 : 0) + (n1 >= 0 && cell1 ? 1 : 0);
       }
       // opened nodes push their children (node 0's, then node 1's), which are
       // consecutive and come after them in the level order; a push that would
@@ -864,10 +835,26 @@ __global__ void __launch_bounds__(mixed_warps<kSplit>() * 32,
       int nc1 = (cat1 == 3) ? min(max(m1.w, 0), 8) : 0;
       if (m0.y <= n0 || m0.y > m - nc0) nc0 = 0;
       if (m1.y <= n1 || m1.y > m - nc1) nc1 = 0;
-      int all_children;
-      const int excl = warp_prefix_small<5>(nc0 + nc1, lt, all_children);
+      // list entries: a cell's, or a leaf's particles
+      int cnt0 = mute ? 0 : (cat0 == 1 ? 1 : (cat0 == 2 ? m0.z : 0));
+      int cnt1 = mute ? 0 : (cat1 == 1 ? 1 : (cat1 == 2 ? m1.z : 0));
+      // both prefix sums in one scan: children (at most 16 a lane) and list
+      // entries (capped: a round with that many takes the slow path)
+      constexpr int kCap = list_cap_of<kTrackSource>();
+      const int own = (nc0 + nc1) | (min(cnt0 + cnt1, 2 * kCap) << 16);
+      int scan = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(kFull, scan, o);
+        if (lane >= o) scan += v;
+      }
+      const int totals = __shfl_sync(kFull, scan, 31);
+      const int all_children = totals & 0xffff, entries = totals >> 16;
+      const int excl = (scan - own) & 0xffff;
       int pushed = all_children;
+      bool relisted = false;
       if (sp + all_children > kStackCap) {
+        relisted = true;  // the scan's list offsets may no longer hold
         if (nc0 > 0 && sp + excl + nc0 > kStackCap) {
           cat0 = 1;
           nc0 = 0;
@@ -887,69 +874,45 @@ __global__ void __launch_bounds__(mixed_warps<kSplit>() * 32,
       for (int j = 0; j < 8; ++j)
         if (j < nc1) stack[sp + excl + nc0 + j] = m1.y + j;
       sp += pushed;
-      // accepted cells -> interaction list (fewer than 32 entries before,
-      // at most 64 more)
-      const unsigned cm0 = __ballot_sync(kFull, cat0 == 1);
-      const unsigned cm1 = __ballot_sync(kFull, cat1 == 1);
-      if (cat0 == 1) {
-        const int pos = ls + __popc(cm0 & lt);
-        list.put(pos, e0.x, e0.y, e0.z, e0.w);
-        if (kTrackSource) src[pos] = kVjp ? -3 - n0 : -1;
-      }
-      if (cat1 == 1) {
-        const int pos = ls + __popc(cm0) + __popc(cm1 & lt);
-        list.put(pos, e1.x, e1.y, e1.z, e1.w);
-        if (kTrackSource) src[pos] = kVjp ? -3 - n1 : -1;
-      }
-      ls += __popc(cm0) + __popc(cm1);
-      if (mute) ls = 0;
-      // reached leaves -> their particles: all at once when they fit
-      const int lc0 = (cat0 == 2 && !mute) ? m0.z : 0;
-      const int lc1 = (cat1 == 2 && !mute) ? m1.z : 0;
-      int lexcl, ltotal;
-      if (__all_sync(kFull, lc0 < 16 && lc1 < 16)) {
-        lexcl = warp_prefix_small<5>(lc0 + lc1, lt, ltotal);
-      } else {
-        int linc = lc0 + lc1;
-        for (int o = 1; o < 32; o <<= 1) {
-          const int v = __shfl_up_sync(kFull, linc, o);
-          if (lane >= o) linc += v;
+      if (ls + entries <= kCap && !relisted) {
+        const int base = ls + ((scan - own) >> 16);
+        if (cnt0 > 0) {
+          list.put(base, e0.x, e0.y, e0.z, e0.w);
+          if (kTrackSource) src[base] = cat0 == 2 ? m0.y : (kVjp ? -3 - n0 : -1);
         }
-        ltotal = __shfl_sync(kFull, linc, 31);
-        lexcl = linc - lc0 - lc1;
-      }
-      if (ls + ltotal <= list_cap_of<kTrackSource>()) {
-        const int base = ls + lexcl;
-        double4 q0 = make_double4(0.0, 0.0, 0.0, 0.0), q1 = q0;
-        // a leaf's record carries its first particle
-        if (lc0 > 0) q0 = a0;
-        if (lc1 > 0) q1 = a1;
-        if (lc0 > 0) {
-          list.put(base, (float)(q0.x - gbox[6]), (float)(q0.y - gbox[7]), (float)(q0.z - gbox[8]), (float)q0.w);
-          if (kTrackSource) src[base] = m0.y;
+        if (cnt1 > 0) {
+          list.put(base + cnt0, e1.x, e1.y, e1.z, e1.w);
+          if (kTrackSource) src[base + cnt0] = cat1 == 2 ? m1.y : (kVjp ? -3 - n1 : -1);
         }
-        if (lc1 > 0) {
-          list.put(base + lc0, (float)(q1.x - gbox[6]), (float)(q1.y - gbox[7]), (float)(q1.z - gbox[8]),
-                   (float)q1.w);
-          if (kTrackSource) src[base + lc0] = m1.y;
-        }
-        for (int j = 1; j < lc0; ++j) {
-          const double4 q = ws.pm4[m0.y + j];
-          list.put(base + j, (float)(q.x - gbox[6]), (float)(q.y - gbox[7]), (float)(q.z - gbox[8]), (float)q.w);
+        for (int j = 1; j < cnt0; ++j) {
+          const float4 e = list_entry(ws.pm4[m0.y + j], gbox);
+          list.put(base + j, e.x, e.y, e.z, e.w);
           if (kTrackSource) src[base + j] = m0.y + j;
         }
-        for (int j = 1; j < lc1; ++j) {
-          const double4 q = ws.pm4[m1.y + j];
-          list.put(base + lc0 + j, (float)(q.x - gbox[6]), (float)(q.y - gbox[7]), (float)(q.z - gbox[8]),
-                   (float)q.w);
-          if (kTrackSource) src[base + lc0 + j] = m1.y + j;
+        for (int j = 1; j < cnt1; ++j) {
+          const float4 e = list_entry(ws.pm4[m1.y + j], gbox);
+          list.put(base + cnt0 + j, e.x, e.y, e.z, e.w);
+          if (kTrackSource) src[base + cnt0 + j] = m1.y + j;
         }
-        ls += ltotal;
+        ls += entries;
         __syncwarp();
         flush_full<kTrackSource, kTPL, kVjp>(list, src, ls, T, V, eps2, nq, (float)p.g, ab);
       } else {
-        // rare: the leaves' particles do not fit behind the list; their
-        // ranges stay in registers through the flush
+        // rare: the leaves' particles do not fit behind the list, or a node
+        // was accepted for want of stack; the cells first (at most 64)
+        const unsigned cm0 = __ballot_sync(kFull, cat0 == 1 && !mute), cm1 = __ballot_sync(kFull, cat1 == 1 && !mute);
+        if (cat0 == 1 && !mute) {
+          const int pos = ls + __popc(cm0 & lt);
+          list.put(pos, e0.x, e0.y, e0.z, e0.w);
+          if (kTrackSource) src[pos] = kVjp ? -3 - n0 : -1;
+        }
+        if (cat1 == 1 && !mute) {
+          const int pos = ls + __popc(cm0) + __popc(cm1 & lt);
+          list.put(pos, e1.x, e1.y, e1.z, e1.w);
+          if (kTrackSource) src[pos] = kVjp ? -3 - n1 : -1;
+        }
+        ls += __popc(cm0) + __popc(cm1);
+        const int lc0 = cat0 == 2 ? cnt0 : 0, lc1 = cat1 == 2 ? cnt1 : 0;
         __syncwarp();
         flush_full<kTrackSource, kTPL, kVjp>(list, src, ls, T, V, eps2, nq, (float)p.g, ab);
         for (int h = 0; h < 2; ++h) {
@@ -963,8 +926,8 @@ __global__ void __launch_bounds__(mixed_warps<kSplit>() * 32,
               const int j = b0 + lane;
               if (j < cnt) {
                 const double4 q = ws.pm4[first + j];
-                list.put(ls + lane, (float)(q.x - gbox[6]), (float)(q.y - gbox[7]), (float)(q.z - gbox[8]),
-                         (float)q.w);
+                const float4 e = list_entry(q, gbox);
+                list.put(ls + lane, e.x, e.y, e.z, e.w);
                 if (kTrackSource) src[ls + lane] = first + j;
               }
               ls += (cnt - b0 < 32) ? (cnt - b0) : 32;
@@ -1000,37 +963,38 @@ __global__ void __launch_bounds__(mixed_warps<kSplit>() * 32,
         }
     }
     __syncwarp();
-    // the group's sums: the other warps' parts are added in warp order
-    double part[3] = {0.0, 0.0, 0.0};
+    // the targets' sums; a shared group's are added in warp order
+    double own[kTPL][3];
+#pragma unroll
+    for (int q = 0; q < kTPL; ++q) {
+      own[q][0] = kVjp ? V.gx : (double)T.sum[q].x - (double)T.comp[q].x;
+      own[q][1] = kVjp ? V.gy : (double)T.sum[q].y - (double)T.comp[q].y;
+      own[q][2] = kVjp ? V.gz : (double)T.sum[q].z - (double)T.comp[q].z;
+    }
     if constexpr (kSplit > 1) {
-      if (wid > 0) {
-        s_part[wid - 1][0][lane] = kVjp ? V.gx : (double)T.sum[0].x - (double)T.comp[0].x;
-        s_part[wid - 1][1][lane] = kVjp ? V.gy : (double)T.sum[0].y - (double)T.comp[0].y;
-        s_part[wid - 1][2][lane] = kVjp ? V.gz : (double)T.sum[0].z - (double)T.comp[0].z;
-      }
+      if (wid > 0)
+        for (int c = 0; c < 3; ++c) s_part[wid - 1][c][lane] = own[0][c];
       __syncthreads();
       if (wid == 0)
         for (int w = 0; w < kSplit - 1; ++w)
-          for (int c = 0; c < 3; ++c) part[c] += s_part[w][c][lane];
-    }
-    if constexpr (kVjp) {
-      if (T.valid[0] && (kSplit == 1 || wid == 0))
-        ab.tgt_g[T.s[0]] = make_double4(V.gx + part[0], V.gy + part[1], V.gz + part[2], 0.0);
+          for (int c = 0; c < 3; ++c) own[0][c] += s_part[w][c][lane];
     }
 #pragma unroll
     for (int q = 0; q < kTPL; ++q) {
-      if (kVjp || !T.valid[q] || (kSplit > 1 && wid > 0)) continue;
-      const double ax = p.g * ((double)T.sum[q].x - (double)T.comp[q].x + part[0]);
-      const double ay = p.g * ((double)T.sum[q].y - (double)T.comp[q].y + part[1]);
-      const double az = p.g * ((double)T.sum[q].z - (double)T.comp[q].z + part[2]);
-      const uint32_t ti = ws.idx[T.s[q]];
-      ws.ax[ti] = ax;
-      ws.ay[ti] = ay;
-      ws.az[ti] = az;
-      if (p.kick) {
-        ws.vx[ti] = __fma_rn(p.half_dt, ax, ws.vx[ti]);
-        ws.vy[ti] = __fma_rn(p.half_dt, ay, ws.vy[ti]);
-        ws.vz[ti] = __fma_rn(p.half_dt, az, ws.vz[ti]);
+      if (!T.valid[q] || (kSplit > 1 && wid > 0)) continue;
+      if constexpr (kVjp) {
+        ab.tgt_g[T.s[q]] = make_double4(own[q][0], own[q][1], own[q][2], 0.0);
+      } else {
+        const double ax = p.g * own[q][0], ay = p.g * own[q][1], az = p.g * own[q][2];
+        const uint32_t ti = ws.idx[T.s[q]];
+        ws.ax[ti] = ax;
+        ws.ay[ti] = ay;
+        ws.az[ti] = az;
+        if (p.kick) {
+          ws.vx[ti] = __fma_rn(p.half_dt, ax, ws.vx[ti]);
+          ws.vy[ti] = __fma_rn(p.half_dt, ay, ws.vy[ti]);
+          ws.vz[ti] = __fma_rn(p.half_dt, az, ws.vz[ti]);
+        }
       }
     }
     inter_total += T.inter;
