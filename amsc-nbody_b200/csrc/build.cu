@@ -1643,8 +1643,7 @@ __global__ void __launch_bounds__(32 * kLevelOrderChannels) lo_tile_scan_kernel(
   }
 }
 
-// A finished cell of the upward pass whose traversal records are still to
-// be written: its mass and centre of mass and what the records need.
+// A cell whose traversal records are to be written.
 struct LoCell {
   double4 a;  // centre of mass, mass
   unsigned long long key;
@@ -1652,25 +1651,11 @@ struct LoCell {
   bool leaf;
 };
 
-// One cell's mass and centre of mass from its sums, and the LevelNode its
-// parent reads (the only record another thread of the upward pass needs).
-__device__ __forceinline__ void lo_emit_node(const Workspace &ws, int b, double tm, double wx, double wy, double wz,
-                                             LoCell &c) {
-  double comx = 0.0, comy = 0.0, comz = 0.0;
-  if (tm > 0.0) {
-    const double inv = __drcp_rn(tm);
-    comx = __dmul_rn(wx, inv);
-    comy = __dmul_rn(wy, inv);
-    comz = __dmul_rn(wz, inv);
-  }
-  c.a = make_double4(comx, comy, comz, tm);
-  LevelNode rec;
-  rec.a = c.a;
-  rec.pre = c.pre;
-  rec.np = c.pe - c.pf;
-  rec.first = c.pf;
-  rec.leaf = c.leaf ? 1 : 0;
-  ws.lo_node[b] = rec;
+// A cell's centre of mass and mass from its sums.
+__device__ __forceinline__ double4 lo_centre(double tm, double wx, double wy, double wz) {
+  if (!(tm > 0.0)) return make_double4(0.0, 0.0, 0.0, tm);
+  const double inv = __drcp_rn(tm);
+  return make_double4(__dmul_rn(wx, inv), __dmul_rn(wy, inv), __dmul_rn(wz, inv), tm);
 }
 
 // A finished cell's geometry from the key prefix (octree_geometry.cu:56-102)
@@ -1973,133 +1958,77 @@ __device__ __forceinline__ double4 lo_big_leaf(const Workspace &ws, int pf, int 
   return own;
 }
 
-// The occupied leaf of group g: mass and centre of mass of the group's
-// particles in sorted order (octree_physics.cu:95-154), its LevelNode and its
-// target-group marks; the traversal records (at preorder index S(g) - 1, no
-// child list: neither walk reads one for an occupied leaf) are the caller's
-// (lo_emit_records with c).  `big` holds the sums of a leaf of more than
-// kBigLeaf particles.  Returns the leaf's level-order index, or false on
-// inconsistent input.
-__device__ __forceinline__ bool lo_leaf_cell(const Workspace &ws, int g, int M, const double4 &big, int &bleaf,
-                                             LoCell &c) {
-  DevScalars *sc = ws.sc;
-  const int2 lf = ws.lo_gleaf[g];
-  const int pf = ws.gfirst[g], pe = ws.glast[g] + 1;
-  c.key = ws.ukey[g];
-  c.level = (ws.gspan[g] >> 8) & 255;
-  bleaf = lf.x;
-  c.skip = lf.y;
-  c.pre = c.skip - 1;
-  c.b = bleaf;
-  c.pf = pf;
-  c.pe = pe;
-  c.c0 = 0;
-  c.nk = 0;
-  c.leaf = true;
-  if (bleaf < 0 || bleaf >= M || c.pre < 0 || c.pre >= M || pf < 0 || pe <= pf || pe > ws.n || c.level < 1 ||
-      c.level > ws.max_level) {
-    record_error(sc, kStageLayout, 1);
+// The sums over a leaf's particles [pf, pe) in sorted order (octree_physics.cu:
+// 95-154), the first one given.
+__device__ __forceinline__ double4 lo_leaf_sums(const Workspace &ws, int pf, int pe, double4 q) {
+  double tm = 0.0, wx = 0.0, wy = 0.0, wz = 0.0;
+  for (int i = pf; i < pe;) {
+    tm = __dadd_rn(tm, q.w);
+    wx = __fma_rn(q.w, q.x, wx);
+    wy = __fma_rn(q.w, q.y, wy);
+    wz = __fma_rn(q.w, q.z, wz);
+    if (++i < pe) q = ws.pm4[i];
+  }
+  return make_double4(wx, wy, wz, tm);
+}
+
+// The occupied leaf lf (level-order index, S of its group) from the sums over
+// its particles: its LevelNode, and its mass and centre of mass in a.  Returns
+// false on inconsistent input.
+__device__ __forceinline__ bool lo_leaf_cell(const Workspace &ws, int M, const double4 &sums, const int2 &lf, int level,
+                                             int pf, int pe, double4 &a) {
+  if (lf.x < 0 || lf.x >= M || lf.y < 1 || lf.y > M || pf < 0 || pe <= pf || pe > ws.n || level < 1 ||
+      level > ws.max_level) {
+    record_error(ws.sc, kStageLayout, 1);
     return false;
   }
-  double tm = big.w, wx = big.x, wy = big.y, wz = big.z;
-  if (pe - pf <= kBigLeaf)
-    for (int i = pf; i < pe; ++i) {
-      const double4 q = ws.pm4[i];
-      tm = __dadd_rn(tm, q.w);
-      wx = __fma_rn(q.w, q.x, wx);
-      wy = __fma_rn(q.w, q.y, wy);
-      wz = __fma_rn(q.w, q.z, wz);
-    }
-  lo_emit_node(ws, bleaf, tm, wx, wy, wz, c);
-  const int np = pe - pf;
-  if (lo_whole_group(ws, c.level, np, true)) {
-    if (c.level == ws.sys_levels) ws.tflag[pf] = 1;
-  } else {
-    for (int k = 0; k < np; k += ws.group_max) ws.tflag[pf + k] = 1;
-  }
+  LevelNode rec;
+  rec.a = a = lo_centre(sums.w, sums.x, sums.y, sums.z);
+  rec.pre = lf.y - 1;
+  rec.np = pe - pf;
+  rec.first = pf;
+  rec.leaf = 1;
+  ws.lo_node[lf.x] = rec;
   return true;
 }
 
-// One internal cell b of a level (children in the next level's range
-// [hi, end); f, q its lo_first and lo_last entries): mass and centre of mass
-// from the children's records in octant order (octree_physics.cu:156-245),
-// the target-group marks and its LevelNode.  Returns false on inconsistent
-// input.
-__device__ __forceinline__ bool lo_level_cell(const Workspace &ws, int level, int b, int hi, int end, int M,
-                                              const int4 &f, const int4 &q, int next_first_child, LoCell &c) {
-  DevScalars *sc = ws.sc;
-  const int c0 = f.y;
-  const int c1 = (b + 1 < hi) ? next_first_child : end;
-  const int pf = f.x, skip = f.z, pe = q.x, pre = q.y;
+// One internal cell b of a level (f, q its lo_first and lo_last entries, its
+// children [f.y, c1) in the next level's range [hi, end)): mass and centre of
+// mass from the children's (load(child)) in octant order (octree_physics.cu:
+// 156-245), and its LevelNode.  Returns false on inconsistent input.
+template <class Load>
+__device__ __forceinline__ bool lo_level_cell(const Workspace &ws, int b, int hi, int end, int M, const int4 &f,
+                                              const int4 &q, int c1, double4 &a, Load &&load) {
+  const int c0 = f.y, pf = f.x, skip = f.z, pe = q.x, pre = q.y;
   if (pre < 0 || pre >= M || skip <= pre + 1 || skip > M || c0 < hi || c1 <= c0 || c1 > end || c1 - c0 > 8 ||
       pf < 0 || pe <= pf || pe > ws.n) {
-    record_error(sc, kStageLayout, 1);
+    record_error(ws.sc, kStageLayout, 1);
     return false;
   }
-  const int nk = c1 - c0;
-  c.level = level;
-  c.pre = pre;
-  c.skip = skip;
-  c.pf = pf;
-  c.pe = pe;
-  c.b = b;
-  c.c0 = c0;
-  c.nk = nk;
-  c.leaf = false;
-  c.key = (unsigned long long)(unsigned)q.z | ((unsigned long long)(unsigned)q.w << 32);
-  // target groups (group_mark_kernel's rule): a whole system that is one
-  // group, else the starts of the children's runs
-  const int np = pe - pf;
-  const bool whole = lo_whole_group(ws, level, np, false);
-  if (whole && level == ws.sys_levels) ws.tflag[pf] = 1;
-  const bool virt = level < ws.sys_levels;
-  const bool merge = !virt && (np <= 1 || level - ws.sys_levels >= ws.group_depth);
-  const bool child_compact_level = level + 1 - ws.sys_levels >= ws.group_depth;
-  // the children first, the marks after: a store between two children's
-  // loads would keep them from being in flight together
   double tm = 0.0, wx = 0.0, wy = 0.0, wz = 0.0;
-  int4 kid[8];  // preorder index, particles, first particle, leaf
 #pragma unroll
   for (int h = 0; h < 8; h += 4) {
-    double2 lo[4], hi2[4];
+    // (a cell past the last child is read in the last child's place)
+    double4 child[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      // (a cell past the last child is read in the last child's place)
-      const LevelNode *src = ws.lo_node + min(c0 + h + j, c1 - 1);
-      const double2 *d = reinterpret_cast<const double2 *>(src);
-      lo[j] = __ldcg(d);
-      hi2[j] = __ldcg(d + 1);
-      kid[h + j] = __ldcg(reinterpret_cast<const int4 *>(src) + 2);
-    }
+    for (int j = 0; j < 4; ++j) child[j] = load(min(c0 + h + j, c1 - 1));
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (c0 + h + j < c1) {
-        const double cm = hi2[j].y;
-        tm = __dadd_rn(tm, cm);
-        wx = __fma_rn(cm, lo[j].x, wx);
-        wy = __fma_rn(cm, lo[j].y, wy);
-        wz = __fma_rn(cm, hi2[j].x, wz);
+        tm = __dadd_rn(tm, child[j].w);
+        wx = __fma_rn(child[j].w, child[j].x, wx);
+        wy = __fma_rn(child[j].w, child[j].y, wy);
+        wz = __fma_rn(child[j].w, child[j].z, wz);
       }
     if (c0 + h + 4 >= c1) break;
   }
-  lo_emit_node(ws, b, tm, wx, wy, wz, c);
-  if (whole) return true;
-  int run = 0;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    if (c0 + j >= c1) break;
-    if (virt) run = 0;
-    const int cp = kid[j].y;
-    if (cp > ws.group_max || !(kid[j].w || cp <= 1 || child_compact_level)) {
-      run = 0;  // the child splits itself
-    } else {
-      if (!merge || run == 0 || run + cp > ws.group_max) {
-        if (kid[j].z >= 0 && kid[j].z < ws.n) ws.tflag[kid[j].z] = 1;
-        run = 0;
-      }
-      run += cp;
-    }
-  }
+  LevelNode rec;
+  rec.a = a = lo_centre(tm, wx, wy, wz);
+  rec.pre = pre;
+  rec.np = pe - pf;
+  rec.first = pf;
+  rec.leaf = 0;
+  ws.lo_node[b] = rec;
   return true;
 }
 
@@ -2137,13 +2066,15 @@ __device__ __forceinline__ bool lo_arrive_last(const Workspace &ws, int c, int p
 // arithmetic in the same child order as a level-by-level pass.  No thread
 // ever waits: a climb ends at the root, at a parent that other children
 // still owe, or at the first inconsistency.  What keeps the climb short: the
-// parent's entries are read before the arrival, the traversal records are
-// lo_records_kernel's, and a block is one warp (32 resident per SM, 64
-// registers), so a warp whose lanes climb far holds no other warp's slot
-// (blocks of 64 and 256 measured 3 and 12 % slower).  Still a level costs the
-// climber about 3 us: two round trips to L2, a release that waits for its
-// writes, an atomic and the combination; 120 us at 2^20 particles, 30 at 4096
-// (a cluster of 8 blocks with a barrier per level took 44 there).
+// parent's entries are read before the arrival, the traversal records and the
+// target-group marks are lo_records_kernel's (the marks alone, written on the
+// climb before its release, took 9 of the tree stage's 66 us at 8192
+// particles), and a block is one warp (32 resident per SM, 64 registers), so a
+// warp whose lanes climb far holds no other warp's slot (blocks of 64 and 256
+// measured 3 and 12 % slower).  Still a level costs the climber about 2.5 us:
+// two round trips to L2, a release that waits for its writes, an atomic and
+// the combination (a cluster of 8 blocks with a barrier per level took 1.3
+// times as long at 4096).
 constexpr int kUpsweepBlock = 32;
 
 __global__ void __launch_bounds__(kUpsweepBlock, 32) lo_upsweep_kernel(Workspace ws) {
@@ -2174,11 +2105,13 @@ __global__ void __launch_bounds__(kUpsweepBlock, 32) lo_upsweep_kernel(Workspace
     }
     const double4 big = lo_big_leaf(ws, pf, np, s_leaf);
     if (g >= G) continue;
-    int cell;
-    LoCell c;
-    if (!lo_leaf_cell(ws, g, M, big, cell, c)) continue;
+    const int2 lf = ws.lo_gleaf[g];
+    int level = (ws.gspan[g] >> 8) & 255;
+    double4 sums = big, a;
+    if (np > 0 && np <= kBigLeaf) sums = lo_leaf_sums(ws, pf, pf + np, ws.pm4[pf]);
+    if (!lo_leaf_cell(ws, M, sums, lf, level, pf, pf + np, a)) continue;
+    int cell = lf.x;
     // the cell's parent and its neighbours' (which children are first and last)
-    int level = c.level;
     int p = ws.lo_first[cell].w;
     int pl = cell > s_base[level] ? ws.lo_first[cell - 1].w : -1;
     int pr = cell + 1 < s_base[level + 1] ? ws.lo_first[cell + 1].w : -1;
@@ -2204,7 +2137,12 @@ __global__ void __launch_bounds__(kUpsweepBlock, 32) lo_upsweep_kernel(Workspace
         if (bad) record_error(sc, kStageLayout, 1);
         break;
       }
-      if (!lo_level_cell(ws, lv, p, hi, end, M, f, q, fr.y, c)) break;
+      const auto load = [&](int k) {
+        const double2 *d = reinterpret_cast<const double2 *>(ws.lo_node + k);
+        const double2 u = __ldcg(d), v = __ldcg(d + 1);
+        return make_double4(u.x, u.y, v.x, v.y);
+      };
+      if (!lo_level_cell(ws, p, hi, end, M, f, q, fr.y, a, load)) break;
       cell = p;
       level = lv;
       p = f.w;
@@ -2214,9 +2152,488 @@ __global__ void __launch_bounds__(kUpsweepBlock, 32) lo_upsweep_kernel(Workspace
   }
 }
 
+// ------------------------------------------------------ small systems ----
+//
+// Up to kSmallSort particles the sort, and up to kSmallTree the numbering and
+// the upward pass, are one block's work: the general kernels spend their time
+// on launch gaps, tickets, look-backs and round trips to L2 (a dozen kernels of
+// 4-8 us each and a climb of 3 us a level, whatever the size), one block on
+// barriers of a few hundred cycles and shared memory.  Same arrays, same bits.
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallWarps = kSmallThreads / 32;
+constexpr int kSmallItems = kSmallSort / kSmallThreads;
+static_assert(kSmallItems % 2 == 0, "items are gathered in pairs");
+// digit counts of a warp: rows eight apart start eight banks apart
+constexpr int kSmallRow = 257;
+constexpr size_t kSmallSortBytes = 8 * (size_t)kSmallSort + 4 * (size_t)kSmallWarps * kSmallRow;
+
+// Keys, sort, leaf groups and the Morton-order gather: encode_kernel, the
+// onesweep passes, groups_kernel and gather_pos4_kernel for one block.  Each
+// warp holds 32 * items consecutive pairs in registers; a pass ranks them by
+// 8-bit digit within the warp (a ballot per bit finds the lanes with the same
+// digit; __match_any_sync made the stage 5 us longer at 4096 particles), scans the
+// warps' digit counts and scatters through shared memory.  Of the 65000 cycles at
+// 4096 particles the passes take half, the FP64 divisions of the keys 9000.
+__global__ void __launch_bounds__(kSmallThreads) small_sort_kernel(Workspace ws) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  unsigned long long *s_pair = reinterpret_cast<unsigned long long *>(smem);
+  unsigned(*s_hist)[kSmallRow] = reinterpret_cast<unsigned(*)[kSmallRow]>(smem + 8 * (size_t)kSmallSort);
+  __shared__ unsigned s_base[256], s_tot[kSmallWarps];
+  DevScalars *sc = ws.sc;
+  const int n = ws.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned lt = lanemask_lt();
+  const int shift = ws.pack_shift, passes = ws.sort_passes;
+  const int items = (n + kSmallThreads - 1) / kSmallThreads;
+  const int p0 = warp * items * 32 + lane;  // item k is pair p0 + 32 k
+  const bool multi = ws.n_systems > 1;
+  for (int sys = tid; sys < ws.n_systems; sys += kSmallThreads) {
+    // morton.cu:167-170, every system's box
+    const double *b = ws.sys_box + 4 * (size_t)sys;
+    if (!isfinite(b[0]) || !isfinite(b[1]) || !isfinite(b[2]) || !isfinite(b[3]) || b[3] <= 0.0)
+      record_error(sc, kStageBbox, 2);
+  }
+  unsigned long long pair[kSmallItems];
+#pragma unroll
+  for (int k = 0; k < kSmallItems; ++k) {
+    const int i = p0 + 32 * k;
+    pair[k] = ~0ull;  // past the end: after every pair, in every pass
+    if (k >= items || i >= n) continue;
+    const int sys = multi ? ws.sys_of[i] : 0;
+    const double *b = ws.sys_box + 4 * (size_t)sys;
+    const double side = b[3], half_side = __dmul_rn(side, 0.5);
+    const uint32_t qx = quantise(ws.x[i], __dsub_rn(b[0], half_side), side);
+    const uint32_t qy = quantise(ws.y[i], __dsub_rn(b[1], half_side), side);
+    const uint32_t qz = quantise(ws.z[i], __dsub_rn(b[2], half_side), side);
+    const unsigned long long key = ((unsigned long long)sys << kSpatialBits) |
+                                   ((expand_bits(qx) << 2) | (expand_bits(qy) << 1) | expand_bits(qz));
+    pair[k] = (key << shift) | (unsigned long long)i;
+  }
+  for (int pass = 0; pass < passes; ++pass) {
+    const int at = shift + 8 * pass;
+    for (int j = lane; j < 256; j += 32) s_hist[warp][j] = 0u;
+    __syncwarp();
+    unsigned rank[kSmallItems];
+#pragma unroll
+    for (int k = 0; k < kSmallItems; ++k) {
+      if (k >= items) break;
+      const unsigned d = (unsigned)(pair[k] >> at) & 255u;
+      unsigned peers = 0xffffffffu;
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        const bool bit = (d >> b) & 1u;
+        const unsigned on = __ballot_sync(0xffffffffu, bit);
+        peers &= bit ? on : ~on;
+      }
+      const unsigned before = s_hist[warp][d];
+      rank[k] = before + __popc(peers & lt);
+      __syncwarp();
+      if ((peers & lt) == 0u) s_hist[warp][d] = before + __popc(peers);
+      __syncwarp();
+    }
+    __syncthreads();
+    // digit d = tid / 4, a quarter of the warps each
+    {
+      const int d = tid >> 2, w0 = (tid & 3) * (kSmallWarps / 4);
+      unsigned v[kSmallWarps / 4], sum = 0;
+#pragma unroll
+      for (int w = 0; w < kSmallWarps / 4; ++w) {
+        v[w] = s_hist[w0 + w][d];
+        sum += v[w];
+      }
+      unsigned inc = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += u;
+      }
+      // the counts before it: other digits of the warp's eight, then the digit's earlier warps
+      unsigned acc = inc - sum;
+      if (lane == 31) s_tot[warp] = inc;
+#pragma unroll
+      for (int w = 0; w < kSmallWarps / 4; ++w) {
+        s_hist[w0 + w][d] = acc;
+        acc += v[w];
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const unsigned v = s_tot[lane];
+      unsigned inc = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += u;
+      }
+      s_tot[lane] = inc - v;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kSmallItems; ++k) {
+      if (k >= items) break;
+      const unsigned d = (unsigned)(pair[k] >> at) & 255u;
+      s_pair[s_tot[d >> 3] + s_hist[warp][d] + rank[k]] = pair[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kSmallItems; ++k) {
+      if (k >= items) break;
+      pair[k] = s_pair[p0 + 32 * k];
+    }
+  }
+  // runs of equal keys
+  const unsigned long long imask = (1ull << shift) - 1ull;
+  unsigned starts[kSmallItems];
+  int count = 0;
+#pragma unroll
+  for (int k = 0; k < kSmallItems; ++k) {
+    if (k >= items) break;
+    const int i = p0 + 32 * k;
+    const bool flag = i < n && (i == 0 || (pair[k] >> shift) != (s_pair[i - 1] >> shift));
+    starts[k] = __ballot_sync(0xffffffffu, flag);
+    count += __popc(starts[k]);
+  }
+  if (lane == 0) s_base[warp] = (unsigned)count;
+  __syncthreads();
+  int run = 0, total = 0;
+  {
+    const int v = (int)s_base[lane];
+    int inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += u;
+    }
+    run = __shfl_sync(0xffffffffu, inc - v, warp);
+    total = __shfl_sync(0xffffffffu, inc, 31);
+  }
+#pragma unroll
+  for (int k = 0; k < kSmallItems; ++k) {
+    if (k >= items) break;
+    const int i = p0 + 32 * k;
+    const int g = run + __popc(starts[k] & lt) + (int)((starts[k] >> lane) & 1u) - 1;
+    run += __popc(starts[k]);
+    if (i >= n) continue;
+    const unsigned long long key = pair[k] >> shift, id = pair[k] & imask;
+    if (g < 0 || g >= n || id >= (unsigned long long)n) {
+      record_error(sc, kStageGroups, 1);
+      continue;
+    }
+    if ((starts[k] >> lane) & 1u) {
+      ws.ukey[g] = key;
+      ws.uniq[g] = (uint32_t)key;
+      ws.gfirst[g] = i;
+    }
+    if (i == n - 1 || (s_pair[i + 1] >> shift) != key) ws.glast[g] = i;
+    ws.keys[i] = (uint32_t)key;
+    ws.idx[i] = (uint32_t)id;
+    ws.psys[i] = (int)(key >> kSpatialBits);
+  }
+  if (tid == 0) sc->n_groups = total;
+  // the particles in Morton order, two items' reads in flight at once
+#pragma unroll
+  for (int h = 0; h < kSmallItems; h += 2) {
+    if (h >= items) break;
+    double4 v[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const unsigned long long id = pair[h + j] & imask;
+      if (h + j >= items || p0 + 32 * (h + j) >= n || id >= (unsigned long long)n) continue;
+      v[j] = ws.pos4 ? ws.pos4[id] : make_double4(ws.x[id], ws.y[id], ws.z[id], 0.0);
+      v[j].w = ws.m[id];
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      if (h + j < items && p0 + 32 * (h + j) < n && (pair[h + j] & imask) < (unsigned long long)n)
+        ws.pm4[p0 + 32 * (h + j)] = v[j];
+  }
+}
+
+// The level-order numbering and the upward pass: lo_span_kernel,
+// lo_tile_scan_kernel, lo_rank_kernel and lo_upsweep_kernel for one block,
+// which takes 32 groups a warp at a time and then the cells of a level at a
+// time, deepest level first, with the masses and centres of mass of the first
+// kSmallCells cells in shared memory (the numbering goes by levels: the upper
+// ones).  A level is a barrier and the sums here, where the climb of
+// lo_upsweep_kernel pays a release, an atomic and two round trips to L2.  What
+// bounds it is one SM's rate of scattered 16-byte writes (80 bytes a cell); 35000
+// cycles at 1000 particles, half of them the ten levels of the upward pass.
+constexpr int kSmallChunks = kSmallTree / 32;
+constexpr int kSmallCells =
+    (224 * 1024 - 4 * kSmallChunks * (kLevelOrderChannels + 1) - 32 * 32 * kSmallWarps) / 32;
+constexpr size_t kSmallTreeBytes =
+    4 * (size_t)kSmallChunks * (kLevelOrderChannels + 1) + 32 * 32 * (size_t)kSmallWarps + 32 * (size_t)kSmallCells;
+static_assert(kSmallWarps == kLevelOrderChannels, "a warp scans a channel");
+
+__global__ void __launch_bounds__(kSmallThreads) small_tree_kernel(Workspace ws) {
+  constexpr int kEnded = kMaxLevels;  // channel of the ended cells
+  extern __shared__ __align__(16) unsigned char smem[];
+  double4 *s_a = reinterpret_cast<double4 *>(smem);
+  double4 *s_leaf = s_a + kSmallCells;
+  int(*s_cnt)[kLevelOrderChannels + 1] = reinterpret_cast<int(*)[kLevelOrderChannels + 1]>(s_leaf + 32 * kSmallWarps);
+  __shared__ int s_total[kLevelOrderChannels], s_base[kMaxLevels + 2], s_m;
+  DevScalars *sc = ws.sc;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned lt = lanemask_lt();
+  const int kb = ws.key_bits, max_level = ws.max_level;
+  int G = sc->n_groups;
+  if (G <= 0 || G > ws.n) {
+    if (tid == 0) record_error(sc, kStageGroups, 2);
+    G = 0;
+  }
+  const int chunks = (G + 31) >> 5;
+  // started levels (delta, lambda] and ended levels (delta_next, lambda] of a span
+  auto masks = [&](int sp, unsigned &smask, unsigned &lmask, int &lam) {
+    smask = lmask = 0u;
+    lam = 0;
+    if (sp < 0) return;
+    const int d = (sp & 255) - 1, l = (sp >> 8) & 255, dn = ((sp >> 16) & 255) - 1;
+    const unsigned upto = (2u << l) - 1u;  // levels 0..lambda
+    smask = upto & ~((1u << (d + 1)) - 1u);
+    lmask = upto & ~((1u << (dn + 1)) - 1u);
+    lam = l;
+  };
+  for (int c = warp; c < chunks; c += kSmallWarps) {
+    const int g = 32 * c + lane;
+    int sp = -1;
+    if (g < G) {
+      const unsigned long long key = ws.ukey[g];
+      int d = -1, dn = -1;
+      bool bad = (key >> kb) != 0ull;
+      if (g > 0) {
+        const unsigned long long kp = ws.ukey[g - 1];
+        if (kp >= key) bad = true;
+        else d = common_levels(kp, key, kb);
+      }
+      if (g + 1 < G) {
+        const unsigned long long kn = ws.ukey[g + 1];
+        if (kn <= key) bad = true;
+        else dn = common_levels(key, kn, kb);
+      }
+      ws.gcount[g] = ws.glast[g] - ws.gfirst[g] + 1;
+      const int lam = 1 + max(0, max(d, dn));
+      if (bad || lam > max_level) {
+        record_error(sc, kStagePlan, bad ? 1 : 3);
+      } else {
+        sp = (d + 1) | (lam << 8) | ((dn + 1) << 16);
+      }
+      ws.gspan[g] = sp;
+    }
+    unsigned sm, lm;
+    int lam, mine = 0;
+    masks(sp, sm, lm, lam);
+    const unsigned any = __reduce_or_sync(0xffffffffu, sm);
+    for (int l = any ? __ffs(any) - 1 : kMaxLevels; l < kMaxLevels && (any >> l) != 0u; ++l) {
+      const int v = __popc(__ballot_sync(0xffffffffu, (sm >> l) & 1u));
+      if (lane == l) mine = v;
+    }
+    const int ended = __reduce_add_sync(0xffffffffu, __popc(lm));
+    s_cnt[c][lane] = lane == kEnded ? ended : mine;
+  }
+  __syncthreads();
+  {
+    // exclusive prefixes over the chunks, a warp per channel
+    int carry = 0;
+    for (int c0 = 0; c0 < chunks; c0 += 32) {
+      const int v = c0 + lane < chunks ? s_cnt[c0 + lane][warp] : 0;
+      int inc = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += u;
+      }
+      if (c0 + lane < chunks) s_cnt[c0 + lane][warp] = carry + inc - v;
+      carry += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (lane == 0) s_total[warp] = carry;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const int v = lane < kMaxLevels ? s_total[lane] : 0;
+    int inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += u;
+    }
+    const int m = __shfl_sync(0xffffffffu, inc, 31);
+    if (lane < kMaxLevels) {
+      sc->level_count[lane] = v;
+      sc->level_base[lane] = s_base[lane] = inc - v;
+    } else if (lane < kMaxLevels + 2) {
+      sc->level_base[lane] = s_base[lane] = m;
+    }
+    if (lane == 0) {
+      const bool ok = G > 0 && m == s_total[kEnded] && m <= ws.cap_nodes;
+      if (G > 0 && !ok) record_error(sc, m > ws.cap_nodes ? kStagePlan : kStageLayout, m > ws.cap_nodes ? kCodeOverflow : 1);
+      sc->n_nodes = s_m = ok ? m : 0;
+    }
+  }
+  __syncthreads();
+  const int M = s_m;
+  if (M == 0) return;
+  const auto keep = [&](int b, const double4 &a) {
+    if (b < kSmallCells) s_a[b] = a;
+  };
+  const auto sum_of = [&](int b) {
+    if (b < kSmallCells) return s_a[b];
+    const double2 *d = reinterpret_cast<const double2 *>(ws.lo_node + b);
+    const double2 u = __ldcg(d), v = __ldcg(d + 1);
+    return make_double4(u.x, u.y, v.x, v.y);
+  };
+  // the cells' entries (as lo_rank_kernel writes them) and the leaves
+  for (int c = warp; c < chunks; c += kSmallWarps) {
+    const int g = 32 * c + lane;
+    int sp = -1, pf = 0, pe = 0;
+    unsigned long long key = 0ull;
+    if (g < G) {
+      sp = ws.gspan[g];
+      pf = ws.gfirst[g];
+      pe = ws.glast[g] + 1;
+      key = ws.ukey[g];
+    }
+    if (pf < 0 || pe > ws.n) pe = pf;
+    double4 sums = make_double4(0.0, 0.0, 0.0, 0.0);  // the leaf's first particle until the end
+    if (pe > pf) sums = ws.pm4[pf];
+    unsigned sm, lm;
+    int lam;
+    masks(sp, sm, lm, lam);
+    const double4 big = lo_big_leaf(ws, pf, pe - pf, s_leaf + 32 * warp);
+    const int ek = __popc(lm);
+    int inc = ek;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += t;
+    }
+    const int s_from = M - (s_cnt[c][kEnded] + inc - ek);
+    const int delta = (sp & 255) - 1;
+    // the cells started at a level by the groups before this one
+    const auto before = [&](int l) {
+      return s_cnt[c][l] + __popc(__ballot_sync(0xffffffffu, (sm >> l) & 1u) & lt);
+    };
+    // the levels where the warp's groups start or end cells, and the one above
+    // (the parent of a group's shallowest cell)
+    const unsigned any = __reduce_or_sync(0xffffffffu, sm | lm);
+    const int l0 = max(0, (any ? __ffs(any) - 1 : 0) - 1);
+    int above = 0, here = before(l0), bleaf = -1;
+    for (int l = l0; (any >> l) != 0u; ++l) {
+      const int below = l + 1 < kMaxLevels ? before(l + 1) : 0;
+      if (sp >= 0 && l <= lam) {
+        const int started = (int)((sm >> l) & 1u);
+        if (started) {
+          const int b = s_base[l] + here;
+          const int parent = (l == 0) ? -1 : s_base[l - 1] + above - (l - 1 == delta ? 1 : 0);
+          if (b < s_base[l + 1]) {
+            ws.lo_first[b] = make_int4(pf, s_base[l + 1] + below, s_from, parent);
+          } else {
+            record_error(sc, kStageLayout, 1);
+          }
+          if (l == lam) bleaf = b;
+        }
+        if (((lm >> l) & 1u) && l < lam) {
+          const int b = s_base[l] + here + started - 1;
+          const int pre = s_from - lam + l - 1;
+          if (b >= s_base[l] && b < s_base[l + 1] && pre >= 0 && pre < M)
+            ws.lo_last[b] = make_int4(pe, pre, (int)(unsigned)key, (int)(unsigned)(key >> 32));
+          else
+            record_error(sc, kStageLayout, 1);
+        }
+      }
+      above = here;
+      here = below;
+    }
+    if (sp < 0) continue;
+    if (bleaf < 0 || s_from < 1 || s_from > M) {
+      record_error(sc, kStageLayout, 1);
+      continue;
+    }
+    const int2 lf = make_int2(bleaf, s_from);
+    ws.lo_gleaf[g] = lf;
+    sums = pe - pf > kBigLeaf ? big : lo_leaf_sums(ws, pf, pe, sums);
+    double4 a;
+    if (lo_leaf_cell(ws, M, sums, lf, lam, pf, pe, a)) keep(bleaf, a);
+  }
+  // a level's entries are on their way while the level below it is finished
+  __syncthreads();
+  int4 f = make_int4(0, 0, 0, 0), q = f;
+  int next = 0;
+  const auto entries = [&](int b, int hi, int end) {
+    if (b < hi) {
+      f = ws.lo_first[b];
+      q = ws.lo_last[b];
+      next = b + 1 < hi ? ws.lo_first[b + 1].y : end;
+    }
+  };
+  entries(s_base[max_level - 1] + tid, s_base[max_level], s_base[max_level + 1]);
+  for (int lv = max_level - 1; lv >= 0; --lv) {
+    const int hi = s_base[lv + 1], end = s_base[lv + 2];
+    for (int b = s_base[lv] + tid; b < hi; b += kSmallThreads) {
+      // (a cell without children is a leaf, and finished)
+      double4 a;
+      if (f.y != next && lo_level_cell(ws, b, hi, end, M, f, q, next, a, sum_of)) keep(b, a);
+      entries(b + kSmallThreads, hi, end);
+    }
+    if (lv > 0) entries(s_base[lv - 1] + tid, s_base[lv], s_base[lv + 1]);
+    __syncthreads();
+  }
+}
+
+// The target groups that cell b (level-order index, children in the next
+// level's range [hi, end), up to next_first_child) starts, group_mark_kernel's
+// rule: nothing inside a cell that is one group by itself, unless it is a
+// whole system; slices of group_max of an occupied leaf; else the starts of
+// the children's runs.
+__device__ __forceinline__ void lo_mark_groups(const Workspace &ws, int b, int level, int hi, int end,
+                                               const LevelNode &nd, int next_first_child) {
+  const int gmax = ws.group_max, n = ws.n, np = nd.np;
+  const bool leaf = nd.leaf != 0;
+  if (lo_whole_group(ws, level, np, leaf)) {
+    if (level == ws.sys_levels && np > 0 && nd.first >= 0 && nd.first < n) ws.tflag[nd.first] = 1;
+    return;
+  }
+  if (leaf) {
+    // an occupied leaf with more than group_max coincident-key particles
+    for (int k = 0; k < np; k += gmax)
+      if (nd.first + k >= 0 && nd.first + k < n) ws.tflag[nd.first + k] = 1;
+    return;
+  }
+  const int c0 = ws.lo_first[b].y, c1 = next_first_child;
+  if (c0 < hi || c1 < c0 || c1 > end || c1 - c0 > 8) {
+    record_error(ws.sc, kStageLayout, 1);
+    return;
+  }
+  const bool virt = level < ws.sys_levels;  // children are other systems
+  const bool merge = !virt && (np <= 1 || level - ws.sys_levels >= ws.group_depth);  // split for its count only
+  const bool child_compact_level = level + 1 - ws.sys_levels >= ws.group_depth;
+  int run = 0;
+#pragma unroll
+  for (int h = 0; h < 8; h += 4) {
+    int4 kid[4];  // preorder index, particles, first particle, leaf
+#pragma unroll
+    for (int j = 0; j < 4; ++j) kid[j] = reinterpret_cast<const int4 *>(ws.lo_node + min(c0 + h + j, c1 - 1))[2];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (c0 + h + j >= c1) break;
+      if (virt) run = 0;
+      const int cp = kid[j].y;
+      if (cp > gmax || !(kid[j].w || cp <= 1 || child_compact_level)) {
+        run = 0;  // the child splits itself
+        continue;
+      }
+      if (!merge || run == 0 || run + cp > gmax) {
+        if (kid[j].z >= 0 && kid[j].z < n) ws.tflag[kid[j].z] = 1;
+        run = 0;
+      }
+      run += cp;
+    }
+    if (c0 + h + 4 >= c1) break;
+  }
+}
+
 // The traversal records of every cell, once the upward pass has its mass and
-// centre of mass: a thread per cell, so that the geometry, the acceptance
-// radius and their divisions and square roots are on nobody's climb.
+// centre of mass, and its target-group marks: a thread per cell, so that the
+// geometry, the acceptance radius with its divisions and square roots and the
+// marks are on nobody's climb.
 template <int kRecords>
 __global__ void __launch_bounds__(kBlock) lo_records_kernel(Workspace ws, double theta) {
   __shared__ int s_base[kMaxLevels + 2];
@@ -2270,11 +2687,11 @@ __global__ void __launch_bounds__(kBlock) lo_records_kernel(Workspace ws, double
       }
     }
     if (!lo_emit_records<kRecords>(ws, theta, c)) record_error(sc, kStageGeometry, 2);
+    lo_mark_groups(ws, b, c.level, s_base[c.level + 1], s_base[c.level + 2], nd, c.c0 + c.nk);
   }
 }
 
-// Target-group starts on the level-order octree: group_mark_kernel's rule
-// with the children read as consecutive entries of the next level.
+// Target-group starts on the level-order octree.
 __global__ void __launch_bounds__(kBlock) lo_group_mark_kernel(Workspace ws) {
   __shared__ int s_base[kMaxLevels + 2];
   __shared__ int s_m;
@@ -2285,50 +2702,12 @@ __global__ void __launch_bounds__(kBlock) lo_group_mark_kernel(Workspace ws) {
     s_m = (sc->error || m != sc->level_base[kMaxLevels]) ? 0 : m;
   }
   __syncthreads();
-  const int M = s_m, gmax = ws.group_max, n = ws.n;
+  const int M = s_m;
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < M; b += gridDim.x * blockDim.x) {
     int level = 0;
     while (level + 1 < kMaxLevels && b >= s_base[level + 1]) ++level;
-    const LevelNode nd = ws.lo_node[b];
-    const int np = nd.np;
-    const bool virt = level < ws.sys_levels;  // children are other systems
-    const bool compact = !virt && (nd.leaf || np <= 1 || level - ws.sys_levels >= ws.group_depth);
-    if (!virt && np <= gmax && compact) {
-      // a whole system that is one group
-      if (level == ws.sys_levels && np > 0 && nd.first >= 0 && nd.first < n) ws.tflag[nd.first] = 1;
-      continue;
-    }
-    if (nd.leaf) {
-      // an occupied leaf with more than group_max coincident-key particles
-      for (int k = 0; k < np; k += gmax)
-        if (nd.first + k >= 0 && nd.first + k < n) ws.tflag[nd.first + k] = 1;
-      continue;
-    }
     const int hi = s_base[level + 1], end = s_base[level + 2];
-    const int c0 = ws.lo_first[b].y;
-    const int c1 = (b + 1 < hi) ? ws.lo_first[b + 1].y : end;
-    if (c0 < hi || c1 < c0 || c1 > end || c1 - c0 > 8) {
-      record_error(sc, kStageLayout, 1);
-      continue;
-    }
-    const bool merge = compact;  // split for its count only
-    int run = 0;
-    for (int c = c0; c < c1; ++c) {
-      const LevelNode ch = ws.lo_node[c];
-      const int cp = ch.np;
-      if (virt) run = 0;
-      const bool ccompact = ch.leaf || cp <= 1 || level + 1 - ws.sys_levels >= ws.group_depth;
-      if (cp > gmax || !ccompact) {
-        // the child splits itself
-        run = 0;
-        continue;
-      }
-      if (!merge || run == 0 || run + cp > gmax) {
-        if (ch.first >= 0 && ch.first < n) ws.tflag[ch.first] = 1;
-        run = 0;
-      }
-      run += cp;
-    }
+    lo_mark_groups(ws, b, level, hi, end, ws.lo_node[b], (b + 1 < hi) ? ws.lo_first[b + 1].y : end);
   }
 }
 
@@ -2432,6 +2811,15 @@ __global__ void __launch_bounds__(kBlock) pack_keys_kernel(Workspace ws, const u
 
 // ------------------------------------------------------------ launches ---
 
+// Leave for the one-block kernels' shared memory, above the 48 KB a launch may
+// take unasked.
+cudaError_t configure_build() {
+  cudaError_t e = cudaFuncSetAttribute(small_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSortBytes);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(small_tree_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallTreeBytes);
+  return e;
+}
+
 static void launch_onesweep(const Workspace &ws, const unsigned long long *src, unsigned long long *dst, int pass,
                             cudaStream_t s) {
   uint32_t *status = ws.sort_status + (size_t)pass * ws.sort_tiles * 256;
@@ -2467,6 +2855,11 @@ cudaError_t launch_kd_bbox(Workspace &ws, double dt, int do_kd, cudaStream_t s) 
 cudaError_t launch_morton_sort_groups(Workspace &ws, cudaStream_t s, int part) {
   // the passes alternate between the two pair buffers
   unsigned long long *sorted = (ws.sort_passes & 1) ? ws.pairs_b : ws.pairs_a;
+  if (part == 0 && ws.lo_tiles && ws.n <= kSmallSort) {
+    small_sort_kernel<<<1, kSmallThreads, kSmallSortBytes, s>>>(ws);
+    count_launches(1);
+    return cudaGetLastError();
+  }
   if (part != 2) {
     int blocks = (ws.n + kBlock - 1) / kBlock;
     const int cap = grid_for(ws, 4);
@@ -2527,8 +2920,8 @@ cudaError_t launch_tree(Workspace &ws, double theta, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_level_order_tree(Workspace &ws, double theta, cudaStream_t s) {
-  if (!ws.lo_tiles) return cudaErrorInvalidValue;
+// Numbering and upward pass of the level-order octree.
+static void launch_level_order_cells(Workspace &ws, cudaStream_t s) {
   if (ws.lo_items == kScanItems)
     lo_span_kernel<kScanItems><<<ws.lo_tile_count, kScanThreads, 0, s>>>(ws);
   else
@@ -2544,15 +2937,25 @@ cudaError_t launch_level_order_tree(Workspace &ws, double theta, cudaStream_t s)
   const int want = (ws.n + kUpsweepBlock - 1) / kUpsweepBlock;
   const int up_grid = want > 0 ? want : 1;
   lo_upsweep_kernel<<<up_grid, kUpsweepBlock, 0, s>>>(ws);
+  count_launches(4);
+}
+
+cudaError_t launch_level_order_tree(Workspace &ws, double theta, cudaStream_t s) {
+  if (!ws.lo_tiles) return cudaErrorInvalidValue;
+  if (ws.n <= kSmallTree) {
+    small_tree_kernel<<<1, kSmallThreads, kSmallTreeBytes, s>>>(ws);
+    count_launches(1);
+  } else {
+    launch_level_order_cells(ws, s);
+  }
   int rec_grid = (ws.n + ws.n / 2 + kBlock - 1) / kBlock;  // about the cells there are
   rec_grid = std::max(1, std::min(rec_grid, grid_for(ws, 8)));
   if (ws.records == kRecordsMixed)
     lo_records_kernel<kRecordsMixed><<<rec_grid, kBlock, 0, s>>>(ws, theta);
   else
     lo_records_kernel<kRecordsFp64><<<rec_grid, kBlock, 0, s>>>(ws, theta);
-  // target-group marks were set by the upward pass
   group_scan_kernel<<<ws.scan_tiles_n, kScanThreads, 0, s>>>(ws);
-  count_launches(6);
+  count_launches(2);
   return cudaGetLastError();
 }
 

@@ -217,6 +217,7 @@ cudaError_t alloc_workspace(Workspace &ws, Allocation &al, int n, const Workspac
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&ws.num_sms, cudaDevAttrMultiProcessorCount, dev);
   cudaError_t e = configure_traversal(ws);
+  if (e == cudaSuccess) e = configure_build();
   if (e != cudaSuccess) return e;
   const size_t N = (size_t)n, C = (size_t)ws.cap_nodes, S = (size_t)n_systems;
   Arena ar;

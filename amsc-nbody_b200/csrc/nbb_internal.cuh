@@ -65,6 +65,12 @@ constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 pairs
 // faster from about 2^18 on.
 constexpr int kSortItemsSmall = 2;
 constexpr int kSmallTiles = 131072;  // particles up to which the small tiles are taken
+// Particles up to which one block makes the keys, sorts and finds the groups,
+// and up to which one block numbers the cells and does the upward pass.  Morton
+// stage, one block / many: 16 / 46 us at 1000 particles, 34 / 50 at 4096, 62 /
+// 57 at 8192; tree stage: 32 / 53 at 1000, 42 / 50 at 2048, 60 / 52 at 4096.
+constexpr int kSmallSort = 4096;
+constexpr int kSmallTree = 2048;
 constexpr int kSortPasses = 4;     // 8-bit digits over a single system's 30-bit keys
 constexpr int kMaxSortPasses = 5;  // ensemble keys: up to 9 system bits + 30 Morton bits
 constexpr int kMaxLevels = 16;     // octree levels: 10 spatial + up to 3 above the system roots
@@ -335,6 +341,8 @@ cudaError_t launch_step_reset(Workspace &ws, cudaStream_t s);
 cudaError_t launch_kd_bbox(Workspace &ws, double dt, int do_kd, cudaStream_t s);
 // Morton encode + digit histograms, onesweep sort, groups + gather.
 // part: 0 all, 1 Morton encode + sort only, 2 leaf groups + gather only
+// Once per workspace, before the launches below.
+cudaError_t configure_build();
 cudaError_t launch_morton_sort_groups(Workspace &ws, cudaStream_t s, int part = 0);
 // Karras tree, plan + scan, octree materialisation, geometry, physics,
 // preorder layout.

@@ -1,0 +1,74 @@
+"""Both sides of the size rules of the mixed walk, the FP64 adjoint and the
+rollout's buffers, against direct summation or a fresh simulation."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [33, 39999, 40000])
+def test_mixed_walk_split(nbb_mod, n):
+    """Four warps to a target group below 40000 particles, one above.  With
+    theta = 0 the list holds every particle; an FP32 sum of at most 96 terms,
+    each with a relative error of at most 16 roundings, is within (96 + 16)
+    2^-24 of the terms' magnitudes."""
+    from nbb import ics
+
+    p = ics.plummer(n, seed=4)
+    soft = 0.02
+    sim = nbb_mod.Simulation(p, nbb_mod.SimulationConfig(1e-3, 0.0, soft, 1.0, group_size=32,
+                                                         precision=nbb_mod.PRECISION_MIXED))
+    sim.initialize()
+    acc = np.stack(sim.accelerations())
+    sim.close()
+    x = np.stack([p.x, p.y, p.z])
+    for i in np.random.default_rng(1).choice(n, min(n, 128), replace=False):
+        d = x - x[:, i:i + 1]
+        term = p.mass * (np.sum(d * d, axis=0) + soft * soft) ** -1.5 * d
+        assert np.all(np.abs(acc[:, i] - term.sum(axis=1)) <= 112 * 2.0 ** -24 * np.abs(term).sum(axis=1).max())
+
+
+@pytest.mark.parametrize("n", [7, 32767, 32768])
+def test_fp64_adjoint_targets(nbb_mod, n):
+    """Eight targets to a warp below 32768 particles, 32 above: theta = 0
+    against the direct-summation adjoint; the two add n terms in different
+    orders (n 2^-52 of the largest, with a factor of 16)."""
+    from nbb import ics
+
+    p = ics.plummer(n, seed=6)
+    gp = np.random.default_rng(2).standard_normal((3, n)) / n
+    cfg = nbb_mod.SimulationConfig(1e-3, 0.0, 0.05, 1.0)
+    sim = nbb_mod.Simulation(p, cfg)
+    sim.initialize()
+    sim.rollout(1, 1)
+    got = sim.backward(gp, gp)
+    sim.close()
+    ref = nbb_mod.direct_rollout_adjoint(p, cfg, 1, gp, gp)[1:]
+    for a, b in zip(got, ref):
+        assert np.max(np.abs(a - b)) <= 16 * n * 2.0 ** -52 * np.max(np.abs(b)) + 1e-18
+
+
+@pytest.mark.parametrize("lengths", [(3, 7), (7, 3), (4, 4)])
+def test_rollout_buffers(nbb_mod, lengths):
+    """A second rollout, shorter, longer or alike, in the first one's buffers
+    gives what it gives in new ones (the adjoint's atomics may add in another
+    order)."""
+    from nbb import ics
+
+    n = 3000
+    p = ics.plummer(n, seed=7)
+    gp = np.random.default_rng(3).standard_normal((3, n)) / n
+    cfg = nbb_mod.SimulationConfig(1e-3, 0.5, 0.05, 1.0)
+    used, fresh = nbb_mod.Simulation(p, cfg), nbb_mod.Simulation(p, cfg)
+    used.initialize()
+    fresh.initialize()
+    used.rollout(lengths[0], 2)
+    used.backward(gp, gp)
+    fresh.run(lengths[0])
+    for sim in (used, fresh):
+        sim.rollout(lengths[1], 2)
+    got, ref = used.backward(gp, gp), fresh.backward(gp, gp)
+    used.close()
+    fresh.close()
+    for a, b in zip(got, ref):
+        assert np.max(np.abs(a - b)) <= 16 * n * 2.0 ** -52 * np.max(np.abs(b))
