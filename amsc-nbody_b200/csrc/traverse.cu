@@ -449,86 +449,93 @@ struct LaneVjp {
   double gx = 0.0, gy = 0.0, gz = 0.0;  // position cotangent (running)
 };
 
-// Sum over the warp of 8 per-lane values, transposed: lane l ends with the
-// total of value ((l >> 4) & 1) * 4 + ((l >> 3) & 1) * 2 + ((l >> 2) & 1)
-// (the four lanes of a quad hold the same total) -- 9 shuffles for 8 sums.
-__device__ __forceinline__ float warp_sum8_transposed(float (&v)[8], int lane) {
-  const bool u16 = lane & 16, u8 = lane & 8, u4 = lane & 4;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float send = u16 ? v[i] : v[i + 4];
-    const float keep = u16 ? v[i + 4] : v[i];
-    v[i] = keep + __shfl_xor_sync(kFull, send, 16);
-  }
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const float send = u8 ? v[i] : v[i + 2];
-    const float keep = u8 ? v[i + 2] : v[i];
-    v[i] = keep + __shfl_xor_sync(kFull, send, 8);
-  }
-  const float send = u4 ? v[0] : v[1];
-  float x = (u4 ? v[1] : v[0]) + __shfl_xor_sync(kFull, send, 4);
-  x += __shfl_xor_sync(kFull, x, 2);
-  x += __shfl_xor_sync(kFull, x, 1);
-  return x;
-}
-
-// VJP of `count` list entries (zero-mass pads contribute nothing) for the
+// VJP of `count` list entries (a multiple of 8; pads have no mass) for the
 // lane's target; returns true on a singular pair.
-__device__ bool vjp_entries(const PairList &list, const int *src, int count, int self, bool valid, float ntx,
-                            float nty, float ntz, LaneVjp &v, float eps2, float g, const AdjointBuffers &ab) {
-  const int lane = threadIdx.x & 31;
-  bool singular = false;
-  float gx = 0.f, gy = 0.f, gz = 0.f;
+//
+// Entries go two to a packed instruction, eight to a reduction over the warp.
+// A lane takes the block's four pairs in an order permuted by its bits 4 and 3,
+// so that in the butterfly's first two rounds every lane keeps its first
+// registers and sends the others, without selects; then it ends with component
+// lane & 3 of entry 2 * (lane >> 3) + (lane >> 2 & 1).  Bound by instruction issue
+// (61 % of the slots, ~38 instructions per entry, 8 of them the reduction): the
+// walk of 65536 particles takes 646 us, 876 with single entries and a
+// reduction by selects.  Blocks of 8 to 10 per SM and batches of 32 to 96
+// entries measured alike.
+__device__ __forceinline__ bool vjp_entries(const PairList &list, const int *src, int count, int self, bool valid,
+                                            float2 ntx, float2 nty, float2 ntz, LaneVjp &v, float2 eps2, float g,
+                                            const AdjointBuffers &ab) {
+  const int lane = threadIdx.x & 31, perm = lane >> 3;
+  const bool b4 = lane & 4, b2 = lane & 2, b1 = lane & 1;
+  const float2 cx = make_float2(v.cx, v.cx), cy = make_float2(v.cy, v.cy), cz = make_float2(v.cz, v.cz);
+  const float2 g2 = make_float2(g, g), m3 = make_float2(-3.f, -3.f);
+  float2 sx = make_float2(0.f, 0.f), sy = sx, sz = sx;
+  bool zero = false;
+#pragma unroll 1
   for (int e0 = 0; e0 < count; e0 += 8) {
-    float ux[8], uy[8], uz[8], uw[8];
+    float2 ux[4], uy[4], uz[4], uw[4];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      ux[k] = uy[k] = uz[k] = uw[k] = 0.f;
-      const int e = e0 + k;
-      if (e >= count) continue;  // warp-uniform
-      const float4 ea = list.a[e >> 1], eb = list.b[e >> 1];
-      const bool hi = e & 1;
-      const float ex = hi ? ea.y : ea.x, ey = hi ? ea.w : ea.z, ez = hi ? eb.y : eb.x, mu = hi ? eb.w : eb.z;
-      const float dx = ex + ntx, dy = ey + nty, dz = ez + ntz;
-      const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2)));
-      if (!valid || src[e] == self || mu == 0.f) continue;
-      if (!(r2 > 0.f)) {
-        singular = true;
-        continue;
-      }
-      const float r = rsqrt_approx(r2);
-      const float rr = r * r;
-      const float gi3 = g * rr * r;
-      const float rc = fmaf(dx, v.cx, fmaf(dy, v.cy, dz * v.cz));
-      const float f = gi3 * mu;
-      const float h = 3.f * f * rr * rc;
-      ux[k] = fmaf(f, v.cx, -h * dx);
-      uy[k] = fmaf(f, v.cy, -h * dy);
-      uz[k] = fmaf(f, v.cz, -h * dz);
-      uw[k] = gi3 * rc;
-      gx -= ux[k];
-      gy -= uy[k];
-      gz -= uz[k];
+    for (int k = 0; k < 4; ++k) {
+      const int pr = (e0 >> 1) + (k ^ perm);
+      const float4 ea = list.a[pr], eb = list.b[pr];
+      const int2 sr = *reinterpret_cast<const int2 *>(src + 2 * pr);
+      const float2 dx = __fadd2_rn(make_float2(ea.x, ea.y), ntx), dy = __fadd2_rn(make_float2(ea.z, ea.w), nty),
+                   dz = __fadd2_rn(make_float2(eb.x, eb.y), ntz);
+      const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, eps2)));
+      zero = zero || !(r2.x > 0.f) || !(r2.y > 0.f);
+      // a factor of 0 takes an entry out of every sum
+      float2 r = make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
+      r.x = sr.x != self && r2.x > 0.f ? r.x : 0.f;
+      r.y = sr.y != self && r2.y > 0.f ? r.y : 0.f;
+      const float2 rr = __fmul2_rn(r, r);
+      const float2 gi3 = __fmul2_rn(__fmul2_rn(g2, rr), r);
+      const float2 rc = __ffma2_rn(dx, cx, __ffma2_rn(dy, cy, __fmul2_rn(dz, cz)));
+      const float2 f = __fmul2_rn(gi3, make_float2(eb.z, eb.w));
+      const float2 h = __fmul2_rn(__fmul2_rn(__fmul2_rn(f, m3), rr), rc);
+      ux[k] = __ffma2_rn(f, cx, __fmul2_rn(h, dx));
+      uy[k] = __ffma2_rn(f, cy, __fmul2_rn(h, dy));
+      uz[k] = __ffma2_rn(f, cz, __fmul2_rn(h, dz));
+      uw[k] = __fmul2_rn(gi3, rc);
+      sx = __fadd2_rn(sx, ux[k]);
+      sy = __fadd2_rn(sy, uy[k]);
+      sz = __fadd2_rn(sz, uz[k]);
     }
-    const float sx = warp_sum8_transposed(ux, lane);
-    const float sy = warp_sum8_transposed(uy, lane);
-    const float sz = warp_sum8_transposed(uz, lane);
-    const float sw = warp_sum8_transposed(uw, lane);
-    const int e = e0 + ((((lane >> 4) & 1) << 2) | (((lane >> 3) & 1) << 1) | ((lane >> 2) & 1));
-    const int comp = lane & 3;
-    const float val = comp == 0 ? sx : (comp == 1 ? sy : (comp == 2 ? sz : sw));
-    if (e < count && val != 0.f) {
+    const auto halves = [&](float2 (&u)[4]) {
+      const auto from = [](float2 t, int o) {
+        return make_float2(__shfl_xor_sync(kFull, t.x, o), __shfl_xor_sync(kFull, t.y, o));
+      };
+      u[0] = __fadd2_rn(u[0], from(u[2], 16));
+      u[1] = __fadd2_rn(u[1], from(u[3], 16));
+      u[0] = __fadd2_rn(u[0], from(u[1], 8));
+      return (b4 ? u[0].y : u[0].x) + __shfl_xor_sync(kFull, b4 ? u[0].x : u[0].y, 4);
+    };
+    const float tx = halves(ux), ty = halves(uy), tz = halves(uz), tw = halves(uw);
+    const float ta = (b2 ? tz : tx) + __shfl_xor_sync(kFull, b2 ? tx : tz, 2);
+    const float tb = (b2 ? tw : ty) + __shfl_xor_sync(kFull, b2 ? ty : tw, 2);
+    const float val = (b1 ? tb : ta) + __shfl_xor_sync(kFull, b1 ? ta : tb, 1);
+    const int e = e0 + 2 * perm + (b4 ? 1 : 0);
+    const float4 eb = list.b[e >> 1];
+    if (val != 0.f && (b4 ? eb.w : eb.z) != 0.f) {
       const int sr = src[e];
       double *dst = nullptr;
       if (sr >= 0) dst = reinterpret_cast<double *>(ab.part_g + sr);
       else if (sr <= -3) dst = reinterpret_cast<double *>(ab.node_g + (-3 - sr));
-      if (dst) atomicAdd(dst + comp, (double)val);
+      if (dst) atomicAdd(dst + (lane & 3), (double)val);
     }
   }
-  v.gx += gx;
-  v.gy += gy;
-  v.gz += gz;
+  v.gx -= sx.x + sx.y;
+  v.gy -= sy.x + sy.y;
+  v.gz -= sz.x + sz.y;
+  bool singular = false;
+  if (valid && zero)  // (the target's own entry, or a singular one)
+#pragma unroll 1
+    for (int e = 0; e < count; ++e) {
+      const float4 ea = list.a[e >> 1], eb = list.b[e >> 1];
+      const bool hi = e & 1;
+      const float dx = (hi ? ea.y : ea.x) + ntx.x, dy = (hi ? ea.w : ea.z) + nty.x, dz = (hi ? eb.y : eb.x) + ntz.x;
+      const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2.x)));
+      singular |= src[e] != self && (hi ? eb.w : eb.z) != 0.f && !(r2 > 0.f);
+    }
+  __syncwarp();
   return singular;
 }
 
@@ -542,8 +549,8 @@ __device__ __forceinline__ void flush_full(const PairList &list, int *src, int &
     const PairList part{list.a + done / 2, list.b + done / 2};
     bool sg;
     if constexpr (kVjp)
-      sg = vjp_entries(part, src + done, kBatch, lt_.s[0], lt_.valid[0], lt_.ntx[0].x, lt_.nty[0].x, lt_.ntz[0].x,
-                       vj, eps2.x, g, ab);
+      sg = vjp_entries(part, src + done, kBatch, lt_.s[0], lt_.valid[0], lt_.ntx[0], lt_.nty[0], lt_.ntz[0],
+                       vj, eps2, g, ab);
     else
       sg = eval_slots<kTrackSource, kTPL>(part, src + (kTrackSource ? done : 0), kBatch, nq, lt_, eps2);
 #pragma unroll
@@ -940,7 +947,14 @@ __global__ void __launch_bounds__(mixed_warps<kSplit>() * 32,
     }
     if (kSplit > 1 && !dealt && wid > 0) tests = tests_before;
     if (ls > 0) {
-      if (ls & 1) {
+      if (kVjp && (ls & 7)) {
+        // complete the last block of eight, as below
+        if (lane < (-ls & 7)) {
+          list.put(ls + lane, 1.0e18f, 1.0e18f, 1.0e18f, 0.f);
+          src[ls + lane] = -2;
+        }
+        __syncwarp();
+      } else if (ls & 1) {
         // complete the last pair with a zero-mass entry far away (its
         // offset squared stays finite in FP32 and it contributes exactly 0)
         if (lane == 0) {
@@ -951,7 +965,7 @@ __global__ void __launch_bounds__(mixed_warps<kSplit>() * 32,
       }
       bool sg;
       if constexpr (kVjp)
-        sg = vjp_entries(list, src, ls + (ls & 1), T.s[0], T.valid[0], T.ntx[0].x, T.nty[0].x, T.ntz[0].x, V, eps2.x,
+        sg = vjp_entries(list, src, (ls + 7) & ~7, T.s[0], T.valid[0], T.ntx[0], T.nty[0], T.ntz[0], V, eps2,
                          (float)p.g, ab);
       else
         sg = eval_slots<kTrackSource, kTPL>(list, src, ls, nq, T, eps2);

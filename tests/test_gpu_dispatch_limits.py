@@ -72,3 +72,28 @@ def test_rollout_buffers(nbb_mod, lengths):
     fresh.close()
     for a, b in zip(got, ref):
         assert np.max(np.abs(a - b)) <= 16 * n * 2.0 ** -52 * np.max(np.abs(b))
+
+
+@pytest.mark.parametrize("n", [2, 7, 8, 9, 31, 33, 65])
+@pytest.mark.parametrize("soft", [0.0, 0.05])
+def test_mixed_adjoint_blocks(nbb_mod, n, soft):
+    """Lists that end inside a block of eight entries, without softening and
+    with zero masses: theta = 0 against the direct-summation adjoint in FP64.
+    64 roundings of FP32 in each of n terms; a lost or doubled entry is of the
+    order of the gradient itself."""
+    from nbb import ics
+
+    p = ics.plummer(n, seed=8)
+    p.mass[n // 2:n // 2 + n // 5] = 0.0
+    gp = np.random.default_rng(5).standard_normal((3, n)) / n
+    cfg = nbb_mod.SimulationConfig(1e-3, 0.0, soft, 1.0, precision=nbb_mod.PRECISION_MIXED, group_size=32)
+    sim = nbb_mod.Simulation(p, cfg)
+    sim.initialize()
+    sim.rollout(1, 1)
+    got = sim.backward(gp, gp)
+    sim.close()
+    ref = nbb_mod.direct_rollout_adjoint(p, nbb_mod.SimulationConfig(1e-3, 0.0, soft, 1.0), 1, gp, gp)[1:]
+    heavy = p.mass > 0.0
+    for a, b in zip(got, ref):
+        a, b = a[..., heavy], b[..., heavy]
+        assert np.max(np.abs(a - b)) <= 64 * n * 2.0 ** -24 * np.max(np.abs(b))
