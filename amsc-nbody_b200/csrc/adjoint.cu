@@ -136,13 +136,15 @@ __global__ void __launch_bounds__(kBlock) adj_parent_kernel(Workspace ws, int *p
 // reduction's latency after each node's; a vector-Jacobian product (rebuild
 // and walk) takes 1.2 ms at 16384 particles where that took 3.2, and 2.6 at
 // 65536 (4.3).
+constexpr int kAdjList = 96;
 constexpr int kAdjWarps = 2;
 constexpr int kAdjBlock = 4;   // entries reduced together
 constexpr int kAdjRow = 4 * kAdjBlock + 1;
 
 template <int kTargets>
 struct AdjShared {
-  ListShared list[kAdjWarps];
+  Frontier walk[kAdjWarps];
+  ListBuffer<kAdjList> list[kAdjWarps];
   double sum[kAdjWarps][kTargets * kAdjRow];
 };
 
@@ -157,7 +159,8 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 7)
   if (sc->error) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tl = lane & (kTargets - 1), el = lane / kTargets;
-  ListShared &sh = shared.list[warp];
+  Frontier &sh = shared.walk[warp];
+  ListBuffer<kAdjList> *list = &shared.list[warp];
   double *sum = shared.sum[warp];
   const int n = ws.n;
   const int m = sc->n_nodes;
@@ -189,7 +192,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 7)
     double gtx = 0.0, gty = 0.0, gtz = 0.0;
     int resume = valid ? 0 : INT_MAX;
     unsigned tests = 0;
-    auto eval = [&](int count) {
+    auto eval = [&](int count, bool) {
       // (inactive entries fill the last block of four)
       for (int j0 = 0; j0 < count; j0 += kAdjBlock) {
         double dx[kPerLane], dy[kPerLane], dz[kPerLane], d2[kPerLane], mu[kPerLane];
@@ -198,8 +201,8 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 7)
 #pragma unroll
         for (int q = 0; q < kPerLane; ++q) {
           const int j = j0 + el * kPerLane + q;
-          const double4 v = sh.src[j];
-          const int2 tag = sh.tag[j];
+          const double4 v = list->src[j];
+          const int2 tag = list->tag[j];
           pre[q] = tag.x;
           aux[q] = tag.y;
           mu[q] = v.w;
@@ -210,7 +213,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 7)
         }
         // the targets' decisions, entry by entry: an undecided cell that a
         // target accepts moves its resume index past the cell
-        const int4 tag0 = *reinterpret_cast<const int4 *>(&sh.tag[j0]), tag1 = *reinterpret_cast<const int4 *>(&sh.tag[j0 + 2]);
+        const int4 tag0 = *reinterpret_cast<const int4 *>(&list->tag[j0]), tag1 = *reinterpret_cast<const int4 *>(&list->tag[j0 + 2]);
         const bool undecided = min(min(tag0.y, tag0.w), min(tag1.y, tag1.w)) < -1;
 #pragma unroll
         for (int q = 0; q < kPerLane; ++q) act[q] = pre[q] >= resume && aux[q] != s;
@@ -222,7 +225,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 7)
               if (e == el) {
                 act[q] = act[q] && pre[q] >= resume;
                 if (aux[q] < -1) {
-                  act[q] = act[q] && accept_entry(sh, j0 + el * kPerLane + q, ws, pre[q], t, d2[q]);
+                  act[q] = act[q] && accept_entry(*list, j0 + el * kPerLane + q, ws, pre[q], t, d2[q]);
                   if (act[q]) resume = -aux[q];
                 }
               }
@@ -256,7 +259,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 7)
         for (int r = 0; r < kTargets / 2; ++r) total += sum[(r0 + r) * kAdjRow + col];
         total += __shfl_xor_sync(kFull, total, 16);
         if (lane < 16 && total != 0.0) {
-          const int2 tag = sh.tag[j0 + (col >> 2)];
+          const int2 tag = list->tag[j0 + (col >> 2)];
           double *dst = reinterpret_cast<double *>(tag.y >= 0 ? ab.part_g + tag.y : ab.node_g + tag.x);
           atomicAdd(dst + (col & 3), total);
         }
@@ -264,7 +267,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, 7)
       }
       return __reduce_min_sync(kFull, resume);
     };
-    ordered_walk(ws, m, root, 1.0, sh, tests, eval);
+    ordered_walk(ws, m, root, 1.0, sh, list, tests, eval);
 #pragma unroll
     for (int o = kTargets; o < 32; o <<= 1) {
       gtx += __shfl_xor_sync(kFull, gtx, o);

@@ -285,11 +285,11 @@ cudaError_t alloc_workspace(Workspace &ws, Allocation &al, int n, const Workspac
 
 bool finite_nonneg(double v) { return std::isfinite(v) && v >= 0.0; }
 
-// Targets per warp of the plain FP64 walk.  A walk costs a warp hardly less
-// for one target than for 32, so one is taken only while that leaves the GPU
-// unfilled: traversal of Plummer spheres, 1 / 32 targets per warp, 60 / 156 us
-// at 1000 particles, 208 / 400 at 4096, 1040 / 570 at 16384.
-int fp64_targets(int n) { return n < 8192 ? 1 : 32; }
+// Targets of a set of the plain FP64 walk.  A walk costs hardly less for one
+// target than for 32, so one is taken only while that leaves the GPU unfilled:
+// traversal of Plummer spheres, 1 / 32 targets to a set, 203 / 232 us at 4096
+// particles, 260 / 264 at 5000, 326 / 287 at 6000, 472 / 294 at 8191.
+int fp64_targets(int n) { return n < 5000 ? 1 : 32; }
 
 // Targets per warp of the FP64 adjoint walk: eight (four lanes to a target)
 // while 32 leave warps idle.  Backward pass of eight steps, 8 / 32 targets per

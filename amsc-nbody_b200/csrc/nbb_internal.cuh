@@ -145,7 +145,7 @@ struct Workspace {
   int n = 0;            // particle count
   int cap_nodes = 0;    // octree node capacity (sum over levels of min(8^L, n))
   int num_sms = 0;
-  int fp64_grid[2] = {0, 0};  // persistent traversal grids (blocks): 32 and 1 targets per warp
+  int fp64_grid[3] = {0, 0, 0};  // persistent traversal grids (blocks): 32 targets to a warp, to two, 1 target to two
   int mixed_grid[2][3] = {{0, 0, 0}, {0, 0, 0}};  // [track source][1, 2 or 4 targets per lane]
   int vjp_grid = 0;     // the mixed walk's adjoint form
   int split_grid[3] = {0, 0, 0};  // the mixed walk with a group per block: force [track source], adjoint

@@ -29,214 +29,328 @@ __device__ __forceinline__ long long warp_sum_ll(long long v) {
   return v;
 }
 
-// Plain FP64 traversal: one warp per set of at most kTargets Morton-consecutive
-// targets, on the ordered interaction list of walk_list.cuh.  Every target
-// sees its own node sequence of the reference's stackless walk
-// (barnes_hut.cu:90-162): a list entry counts for a target when its preorder
-// index has reached the target's resume index, and an undecided cell that the
-// target accepts moves that index past the cell's subtree.
+// Plain FP64 traversal on the ordered interaction lists of walk_list.cuh, for
+// sets of at most kTargets Morton-consecutive targets.  Every target sees its
+// own node sequence of the reference's stackless walk (barnes_hut.cu:90-162):
+// a list entry counts for a target when its preorder index has reached the
+// target's resume index, and an undecided cell that the target accepts moves
+// that index past the cell's subtree.
 //
 // With 32 targets a lane holds one target and the warp takes the entries in
 // order, four in flight.  With one target the 32 lanes form the terms of 32
 // consecutive entries at once; the terms are then added in entry order, each
 // component's sum by one lane, so the result has the same bits.  One target
-// per warp wastes the walk on a single target but fills the GPU from small
+// per set wastes the walk on a single target but fills the GPU from small
 // systems (see fp64_targets).
 //
+// With kPair a set is two warps' work: one walks and fills the list, the other
+// evaluates it, with two buffers between them.  That is for systems whose sets
+// all run at once, where the time is that of one set: its round trips and its
+// FP64 chains then overlap (walk at 2000, 12000, 24000 particles 120, 540, 582
+// us by one warp, 86, 348, 390 by two; alike at 65536).  Where sets wait for
+// warps, a warp for each has the FP64 pipe busier: 10.7 against 11.9 ms at 2^20
+// (see pair_sets).
+//
 // Bound at 2^20 particles: instruction issue and FP64 latency (FP64 pipe 49 %,
-// issue 61 % busy at 16 warps per SM; an entry takes 25 FP64 operations of
+// issue 61 % busy at 16 warps per SM; an entry takes 23 FP64 operations of
 // 2.2 cycles).  16 warps with 128 registers, four entries in flight, beat 20
 // warps of 96 registers and 24 of 80 (10.7, 11.8 and 12.4 ms).
-constexpr int kFp64Warps = 2;
+constexpr int kFp64Warps = 2;  // sets of a block, one warp each
+constexpr int kFp64Pairs = 4;  // sets of a block, two warps each: w walks, w + 4 evaluates (one of each per SM quarter)
+template <bool kPair>
+__host__ __device__ constexpr int fp64_threads() {
+  return kPair ? 64 * kFp64Pairs : 32 * kFp64Warps;
+}
 
+// One warp's targets and their sums.
 template <int kTargets>
-struct Fp64Shared {
-  ListShared list[kFp64Warps];
-  double4 term[kTargets < 32 ? kFp64Warps : 1][kTargets < 32 ? 32 : 1];  // offset and factor of each lane's entry
+struct Fp64Targets {
+  int s, resume;
+  unsigned count;  // interactions
+  bool valid, in_range, singular = false;
+  double4 t;
+  double soft2, ax, ay, az;
+
+  // set g0 .. g1 - 1
+  __device__ __forceinline__ void load(const Workspace &ws, const TraversalParams &p, int g0, int g1, int sys) {
+    s = g0 + ((threadIdx.x & 31) & (kTargets - 1));
+    valid = s < g1;
+    t = ws.pm4[valid ? s : g0];
+    const double soft = ws.sys_eps ? ws.sys_eps[sys] : p.soft;
+    soft2 = __dmul_rn(soft, soft);
+    // no squared distance of the system leaves inv_sqrt_core's range
+    in_range = soft2 > 0x1p-900 && soft2 < 0x1p900 && ws.sys_box[4 * sys + 3] < 0x1p400;
+    resume = valid ? 0 : INT_MAX;
+    ax = ay = az = 0.0;
+    count = 0;
+  }
+
+  // Entries [0, n) of the list; returns the smallest resume index.  term:
+  // room for each lane's offset and factor (one target only).
+  template <int kCap>
+  __device__ __forceinline__ int eval(const Workspace &ws, const ListBuffer<kCap> &list, int n, double4 *term) {
+    const int lane = threadIdx.x & 31;
+    if constexpr (kTargets == 32) {
+      for (int j = 0; j < n; j += 4) {
+        double dx[4], dy[4], dz[4], r2[4], f[4];
+        int pre[4], aux[4];
+        bool act[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const double4 v = list.src[j + q];
+          const int2 tag = list.tag[j + q];
+          pre[q] = tag.x;
+          aux[q] = tag.y;
+          dx[q] = __dsub_rn(v.x, t.x);
+          dy[q] = __dsub_rn(v.y, t.y);
+          dz[q] = __dsub_rn(v.z, t.z);
+          f[q] = v.w;
+          r2[q] = sqdist(dx[q], dy[q], dz[q]);
+          act[q] = pre[q] >= resume && aux[q] != s;
+        }
+        if (min(min(aux[0], aux[1]), min(aux[2], aux[3])) < -1) {
+          // undecided cells: a target that accepts one resumes past it
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            act[q] = act[q] && pre[q] >= resume;
+            if (aux[q] < -1) {
+              act[q] = act[q] && accept_entry(list, j + q, ws, pre[q], t, r2[q]);
+              if (act[q]) resume = -aux[q];
+            }
+          }
+        }
+        // all terms are formed before any is added; the sums take them in
+        // the reference's order
+        bool plain = in_range;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          r2[q] = __dadd_rn(r2[q], soft2);
+          plain = plain && __double2loint(r2[q]) != -1;
+        }
+        double inv[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) inv[q] = inv_sqrt_core(r2[q]);
+        if (!plain) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            inv[q] = inv_sqrt_general(r2[q]);
+            if (act[q] && r2[q] <= 0.0) {
+              singular = true;
+              act[q] = false;
+              ++count;
+            }
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) f[q] = __dmul_rn(f[q], __dmul_rn(__dmul_rn(inv[q], inv[q]), inv[q]));
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (act[q]) {
+            ax = __fma_rn(f[q], dx[q], ax);
+            ay = __fma_rn(f[q], dy[q], ay);
+            az = __fma_rn(f[q], dz[q], az);
+            ++count;
+          }
+      }
+    } else {
+      // lane (el, tl): entry el of each block of kLanes, target tl; lanes
+      // el = 0, 1, 2 sum the x, y, z component (in ax)
+      constexpr int kLanes = 32 / kTargets;  // lanes per target
+      const int tl = lane & (kTargets - 1), el = lane / kTargets, comp = min(el, 2);
+      for (int e0 = 0; e0 < n; e0 += kLanes) {
+        const bool has = e0 + el < n;
+        const int j = has ? e0 + el : e0;
+        const double4 q = list.src[j];
+        const int2 tg = list.tag[j];
+        const double dx = __dsub_rn(q.x, t.x), dy = __dsub_rn(q.y, t.y), dz = __dsub_rn(q.z, t.z);
+        const double d2 = sqdist(dx, dy, dz);
+        const bool undecided = has && tg.y < -1;
+        bool act = has && tg.x >= resume && tg.y != s;
+        if (__any_sync(kFull, undecided)) {
+          // the entries' decisions in order: each may move the resume
+          // index of the target's later entries
+          const bool take = act && (!undecided || accept_entry(list, j, ws, tg.x, t, d2));
+          act = false;
+          for (int e = 0; e < kLanes; ++e) {
+            if (e == el) act = take && tg.x >= resume;
+            const int moved = (act && undecided) ? -tg.y : resume;
+            resume = __shfl_sync(kFull, moved, e * kTargets + tl);
+          }
+        }
+        const double r2 = __dadd_rn(d2, soft2);
+        double inv = inv_sqrt_core(r2);
+        if (!inv_sqrt_in_range(r2)) inv = inv_sqrt_general(r2);
+        const double f = __dmul_rn(q.w, __dmul_rn(__dmul_rn(inv, inv), inv));
+        const bool zero = r2 <= 0.0;
+        singular |= act && zero;
+        count += act ? 1 : 0;
+        // an idle lane's term is 0, which leaves a sum's bits alone
+        const bool on = act && !zero;
+        term[lane] = make_double4(on ? dx : 0.0, on ? dy : 0.0, on ? dz : 0.0, on ? f : 0.0);
+        __syncwarp();
+#pragma unroll
+        for (int e = 0; e < kLanes; ++e) {
+          const double *v = reinterpret_cast<const double *>(term + e * kTargets + tl);
+          ax = __fma_rn(v[3], v[comp], ax);
+        }
+        __syncwarp();
+      }
+    }
+    return __reduce_min_sync(kFull, resume);
+  }
+
+  // The accelerations, and the second half kick (integrator.cu:86-106).
+  __device__ __forceinline__ void store(const Workspace &ws, const TraversalParams &p) const {
+    if (!valid) return;
+    const uint32_t ti = ws.idx[s];
+    if constexpr (kTargets == 32) {
+      ws.ax[ti] = ax;
+      ws.ay[ti] = ay;
+      ws.az[ti] = az;
+      if (p.kick) {
+        ws.vx[ti] = __fma_rn(p.half_dt, ax, ws.vx[ti]);
+        ws.vy[ti] = __fma_rn(p.half_dt, ay, ws.vy[ti]);
+        ws.vz[ti] = __fma_rn(p.half_dt, az, ws.vz[ti]);
+      }
+    } else {
+      const int el = (threadIdx.x & 31) / kTargets;
+      if (el >= 3) return;
+      double *a = el == 0 ? ws.ax : (el == 1 ? ws.ay : ws.az);
+      a[ti] = ax;
+      if (p.kick) {
+        double *v = el == 0 ? ws.vx : (el == 1 ? ws.vy : ws.vz);
+        v[ti] = __fma_rn(p.half_dt, ax, v[ti]);
+      }
+    }
+  }
 };
 
-template <int kTargets>
-__global__ void __launch_bounds__(kFp64Warps * 32, kTargets == 32 ? 8 : 10)
+// What a set's warp or pair of warps keeps in shared memory.
+template <int kTargets, bool kPair>
+struct Fp64Shared {
+  static constexpr int kCap = kPair ? 64 : 96;
+  Frontier walk;
+  ListBuffer<kCap> list[kPair ? 2 : 1];
+  double4 term[kTargets < 32 ? 32 : 1];
+  int set[2], count[2], last[2], done[2];  // per buffer of a pair: see the kernel
+};
+
+// Named barriers of a pair: buffer b filled (kFilled + b), buffer b free (kFree
+// + b); the two warps use each in turn, one arriving and one waiting.
+constexpr int kFilled = 0, kFree = 2, kPairBarriers = 4;
+static_assert(kFp64Pairs * kPairBarriers <= 16, "named barriers of a block");
+__device__ __forceinline__ void pair_arrive(int id) {
+  __syncwarp();
+  asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory");
+}
+__device__ __forceinline__ void pair_wait(int id) {
+  __syncwarp();
+  asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
+}
+
+template <int kTargets, bool kPair>
+__global__ void __launch_bounds__(fp64_threads<kPair>(), kPair ? 2 : 8)
     traverse_fp64_kernel(Workspace ws, TraversalParams p) {
-  constexpr int kLanes = 32 / kTargets;  // lanes per target
-  __shared__ Fp64Shared<kTargets> shared;
+  using Shared = Fp64Shared<kTargets, kPair>;
+  constexpr int kSets = kPair ? kFp64Pairs : kFp64Warps;
+  __shared__ Shared shared[kSets];
   DevScalars *sc = ws.sc;
-  if (sc->error) return;
+  // (one decision for the block: a pair's warps leave together)
+  if (__syncthreads_or(sc->error != 0)) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int tl = lane & (kTargets - 1), el = lane / kTargets;
-  ListShared &sh = shared.list[warp];
+  Shared &sh = shared[warp % kSets];
   const int n = ws.n;
   const int m = sc->n_nodes;
   const int n_sets = sc->n_tgroups;
   long long inter = 0, tests = 0;
-  bool singular = false;
-  while (true) {
+  Fp64Targets<kTargets> targets;
+  const auto bounds = [&](int set, int &g0, int &g1, int &sys) {
+    g0 = ws.tstart[set];
+    g1 = min(set + 1 < n_sets ? ws.tstart[set + 1] : n, g0 + kTargets);
+    // a set's targets belong to one system: walk that system's subtree
+    sys = ws.n_systems > 1 ? ws.psys[g0] : 0;
+  };
+  const auto next_set = [&]() {
     int set = 0;
     if (lane == 0) set = (int)atomicAdd(&sc->work_counter, 1u);
-    set = __shfl_sync(kFull, set, 0);
-    if (set >= n_sets) break;
-    const int g0 = ws.tstart[set];
-    const int g1 = min(set + 1 < n_sets ? ws.tstart[set + 1] : n, g0 + kTargets);
-    const int s = g0 + tl;
-    const bool valid = s < g1;
-    const double4 t = ws.pm4[valid ? s : g0];
-    // a warp's targets belong to one system: walk that system's subtree
-    const int sys = ws.n_systems > 1 ? ws.psys[g0] : 0;
-    const int root = ws.root_pre[sys];
-    set_target_box(sh, t, ws.sys_box[4 * sys + 3]);
-    const double soft = ws.sys_eps ? ws.sys_eps[sys] : p.soft;
-    const double soft2 = __dmul_rn(soft, soft);
-    // no squared distance of the system leaves inv_sqrt_core's range
-    const bool in_range = soft2 > 0x1p-900 && soft2 < 0x1p900 && ws.sys_box[4 * sys + 3] < 0x1p400;
-    int resume = valid ? 0 : INT_MAX;
-    unsigned count_inter = 0, count_tests = 0;
-    if constexpr (kTargets == 32) {
-      double ax = 0.0, ay = 0.0, az = 0.0;
-      auto eval = [&](int count) {
-        for (int j = 0; j < count; j += 4) {
-          double dx[4], dy[4], dz[4], r2[4], f[4];
-          int pre[4], aux[4];
-          bool act[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const double4 v = sh.src[j + q];
-            const int2 tag = sh.tag[j + q];
-            pre[q] = tag.x;
-            aux[q] = tag.y;
-            dx[q] = __dsub_rn(v.x, t.x);
-            dy[q] = __dsub_rn(v.y, t.y);
-            dz[q] = __dsub_rn(v.z, t.z);
-            f[q] = v.w;
-            r2[q] = sqdist(dx[q], dy[q], dz[q]);
-            act[q] = pre[q] >= resume && aux[q] != s;
-          }
-          if (min(min(aux[0], aux[1]), min(aux[2], aux[3])) < -1) {
-            // undecided cells: a target that accepts one resumes past it
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              act[q] = act[q] && pre[q] >= resume;
-              if (aux[q] < -1) {
-                act[q] = act[q] && accept_entry(sh, j + q, ws, pre[q], t, r2[q]);
-                if (act[q]) resume = -aux[q];
-              }
-            }
-          }
-          // all terms are formed before any is added; the sums take them in
-          // the reference's order
-          bool plain = in_range;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            r2[q] = __dadd_rn(r2[q], soft2);
-            plain = plain && __double2loint(r2[q]) != -1;
-          }
-          double inv[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) inv[q] = inv_sqrt_core(r2[q]);
-          if (!plain) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              inv[q] = inv_sqrt_general(r2[q]);
-              if (act[q] && r2[q] <= 0.0) {
-                singular = true;
-                act[q] = false;
-                ++count_inter;
-              }
-            }
-          }
-#pragma unroll
-          for (int q = 0; q < 4; ++q) f[q] = __dmul_rn(f[q], __dmul_rn(__dmul_rn(inv[q], inv[q]), inv[q]));
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            if (act[q]) {
-              ax = __fma_rn(f[q], dx[q], ax);
-              ay = __fma_rn(f[q], dy[q], ay);
-              az = __fma_rn(f[q], dz[q], az);
-              ++count_inter;
-            }
-        }
-        return __reduce_min_sync(kFull, resume);
-      };
-      ordered_walk(ws, m, root, p.g, sh, count_tests, eval);
-      if (valid) {
-        const uint32_t ti = ws.idx[s];
-        ws.ax[ti] = ax;
-        ws.ay[ti] = ay;
-        ws.az[ti] = az;
-        if (p.kick) {
-          // second half kick, integrator.cu:86-106
-          ws.vx[ti] = __fma_rn(p.half_dt, ax, ws.vx[ti]);
-          ws.vy[ti] = __fma_rn(p.half_dt, ay, ws.vy[ti]);
-          ws.vz[ti] = __fma_rn(p.half_dt, az, ws.vz[ti]);
-        }
-      }
-    } else {
-      // lane (el, tl): entry el of each block of kLanes, target tl; lanes
-      // el = 0, 1, 2 sum the x, y, z component
-      double acc = 0.0;
-      double4 *term = shared.term[warp];
-      const int comp = min(el, 2);
-      auto eval = [&](int count) {
-        for (int e0 = 0; e0 < count; e0 += kLanes) {
-          const bool has = e0 + el < count;
-          const int j = has ? e0 + el : e0;
-          const double4 q = sh.src[j];
-          const int2 tg = sh.tag[j];
-          const double dx = __dsub_rn(q.x, t.x), dy = __dsub_rn(q.y, t.y), dz = __dsub_rn(q.z, t.z);
-          const double d2 = sqdist(dx, dy, dz);
-          const bool undecided = has && tg.y < -1;
-          bool act = has && tg.x >= resume && tg.y != s;
-          if (__any_sync(kFull, undecided)) {
-            // the entries' decisions in order: each may move the resume
-            // index of the target's later entries
-            const bool take = act && (!undecided || accept_entry(sh, j, ws, tg.x, t, d2));
-            act = false;
-            for (int e = 0; e < kLanes; ++e) {
-              if (e == el) act = take && tg.x >= resume;
-              const int moved = (act && undecided) ? -tg.y : resume;
-              resume = __shfl_sync(kFull, moved, e * kTargets + tl);
-            }
-          }
-          const double r2 = __dadd_rn(d2, soft2);
-          double inv = inv_sqrt_core(r2);
-          if (!inv_sqrt_in_range(r2)) inv = inv_sqrt_general(r2);
-          const double f = __dmul_rn(q.w, __dmul_rn(__dmul_rn(inv, inv), inv));
-          const bool zero = r2 <= 0.0;
-          singular |= act && zero;
-          count_inter += act ? 1 : 0;
-          // an idle lane's term is 0, which leaves a sum's bits alone
-          const bool on = act && !zero;
-          term[lane] = make_double4(on ? dx : 0.0, on ? dy : 0.0, on ? dz : 0.0, on ? f : 0.0);
-          __syncwarp();
-#pragma unroll
-          for (int e = 0; e < kLanes; ++e) {
-            const double *v = reinterpret_cast<const double *>(term + e * kTargets + tl);
-            acc = __fma_rn(v[3], v[comp], acc);
-          }
-          __syncwarp();
-        }
-        return __reduce_min_sync(kFull, resume);
-      };
-      ordered_walk(ws, m, root, p.g, sh, count_tests, eval);
-      if (valid && el < 3) {
-        const uint32_t ti = ws.idx[s];
-        double *a = el == 0 ? ws.ax : (el == 1 ? ws.ay : ws.az);
-        a[ti] = acc;
-        if (p.kick) {
-          double *v = el == 0 ? ws.vx : (el == 1 ? ws.vy : ws.vz);
-          v[ti] = __fma_rn(p.half_dt, acc, v[ti]);
-        }
-      }
+    return __shfl_sync(kFull, set, 0);
+  };
+  int g0, g1, sys;
+  if constexpr (!kPair) {
+    for (int set = next_set(); set < n_sets; set = next_set()) {
+      bounds(set, g0, g1, sys);
+      targets.load(ws, p, g0, g1, sys);
+      set_target_box(sh.walk, targets.t, ws.sys_box[4 * sys + 3]);
+      unsigned set_tests = 0;
+      auto *list = &sh.list[0];
+      ordered_walk(ws, m, ws.root_pre[sys], p.g, sh.walk, list, set_tests,
+                   [&](int count, bool) { return targets.eval(ws, *list, count, sh.term); });
+      tests += set_tests;
+      inter += targets.count;
+      targets.store(ws, p);
     }
-    inter += count_inter;
-    tests += count_tests;
-    __syncwarp();
+  } else if (warp < kSets) {
+    // the walking warp: a buffer is its own once the other warp has freed it
+    const int filled = warp * kPairBarriers + kFilled, free = warp * kPairBarriers + kFree;
+    int b = 0;
+    auto *list = &sh.list[0];
+    pair_wait(free);
+    for (int set = next_set(); set < n_sets; set = next_set()) {
+      bounds(set, g0, g1, sys);
+      const int s = g0 + (lane & (kTargets - 1));
+      set_target_box(sh.walk, ws.pm4[s < g1 ? s : g0], ws.sys_box[4 * sys + 3]);
+      unsigned set_tests = 0;
+      bool first = true;  // the other buffer holds no entries of this set yet
+      const auto hand = [&](int count, bool last) {
+        if (lane == 0) {
+          sh.set[b] = set;
+          sh.count[b] = count;
+          sh.last[b] = last ? 1 : 0;
+        }
+        pair_arrive(filled + b);
+        b ^= 1;
+        list = &sh.list[b];
+        pair_wait(free + b);
+        const int done = first ? 0 : sh.done[b];
+        first = false;
+        return done;
+      };
+      ordered_walk(ws, m, ws.root_pre[sys], p.g, sh.walk, list, set_tests, hand);
+      tests += set_tests;
+    }
+    if (lane == 0) sh.set[b] = -1;  // no more
+    pair_arrive(filled + b);
+    pair_wait(free + (b ^ 1));  // every arrival is met
+  } else {
+    // the evaluating warp
+    const int filled = (warp - kSets) * kPairBarriers + kFilled, free = (warp - kSets) * kPairBarriers + kFree;
+    pair_arrive(free);
+    pair_arrive(free + 1);
+    bool fresh = true;
+    for (int b = 0;; b ^= 1) {
+      pair_wait(filled + b);
+      const int set = sh.set[b];
+      if (set < 0) break;
+      const bool last = sh.last[b] != 0;
+      if (fresh) {
+        bounds(set, g0, g1, sys);
+        targets.load(ws, p, g0, g1, sys);
+      }
+      const int done = targets.eval(ws, sh.list[b], sh.count[b], sh.term);
+      if (lane == 0) sh.done[b] = done;
+      pair_arrive(free + b);
+      fresh = last;
+      if (!last) continue;
+      inter += targets.count;
+      targets.store(ws, p);
+    }
   }
-  if (__any_sync(kFull, singular) && lane == 0) record_error(sc, kStageTraversal, 6);
+  if (__any_sync(kFull, targets.singular) && lane == 0) record_error(sc, kStageTraversal, 6);
   inter = warp_sum_ll(inter);
   tests = warp_sum_ll(tests);
   if (lane == 0) {
-    atomicAdd(&sc->interactions, (unsigned long long)inter);
-    atomicAdd(&sc->mac_tests, (unsigned long long)tests);
+    if (inter) atomicAdd(&sc->interactions, (unsigned long long)inter);
+    if (tests) atomicAdd(&sc->mac_tests, (unsigned long long)tests);
   }
 }
 
@@ -1350,10 +1464,15 @@ static cudaError_t grid_of(K kernel, int threads, int sms, int &grid) {
 constexpr int kMixedSplit = 4;
 static bool split_group(int n) { return n < 40000; }
 
+// Whether two warps share a set of the FP64 walk of n particles: up to a few
+// sets per pair of warps that fits (figures at the kernel).
+static bool pair_sets(int n) { return n < 65536; }
+
 cudaError_t configure_traversal(Workspace &ws) {
   const int sms = ws.num_sms > 0 ? ws.num_sms : 148;
-  cudaError_t e = grid_of(traverse_fp64_kernel<32>, kFp64Warps * 32, sms, ws.fp64_grid[0]);
-  if (e == cudaSuccess) e = grid_of(traverse_fp64_kernel<1>, kFp64Warps * 32, sms, ws.fp64_grid[1]);
+  cudaError_t e = grid_of(traverse_fp64_kernel<32, false>, fp64_threads<false>(), sms, ws.fp64_grid[0]);
+  if (e == cudaSuccess) e = grid_of(traverse_fp64_kernel<32, true>, fp64_threads<true>(), sms, ws.fp64_grid[1]);
+  if (e == cudaSuccess) e = grid_of(traverse_fp64_kernel<1, true>, fp64_threads<true>(), sms, ws.fp64_grid[2]);
   if (e == cudaSuccess) e = grid_of(traverse_mixed_kernel<false, 1>, kMixedWarps * 32, sms, ws.mixed_grid[0][0]);
   if (e == cudaSuccess) e = grid_of(traverse_mixed_kernel<true, 1>, kMixedWarps * 32, sms, ws.mixed_grid[1][0]);
   if (e == cudaSuccess) e = grid_of(traverse_mixed_kernel<false, 2>, kMixedWarps * 32, sms, ws.mixed_grid[0][1]);
@@ -1386,10 +1505,14 @@ cudaError_t launch_traversal(Workspace &ws, const TraversalParams &p, cudaStream
   const int track = p.soft > 0.0 ? 0 : 1;
   const int grid = ws.mixed_grid[track][slot] > 0 ? ws.mixed_grid[track][slot] : 148;
   if (p.precision == 0) {
-    if (p.targets > 1)
-      traverse_fp64_kernel<32><<<ws.fp64_grid[0] > 0 ? ws.fp64_grid[0] : 148, kFp64Warps * 32, 0, s>>>(ws, p);
+    const int form = p.targets > 1 ? (pair_sets(ws.n) ? 1 : 0) : 2;
+    const int blocks = ws.fp64_grid[form] > 0 ? ws.fp64_grid[form] : 148;
+    if (form == 2)
+      traverse_fp64_kernel<1, true><<<blocks, fp64_threads<true>(), 0, s>>>(ws, p);
+    else if (form == 1)
+      traverse_fp64_kernel<32, true><<<blocks, fp64_threads<true>(), 0, s>>>(ws, p);
     else
-      traverse_fp64_kernel<1><<<ws.fp64_grid[1] > 0 ? ws.fp64_grid[1] : 148, kFp64Warps * 32, 0, s>>>(ws, p);
+      traverse_fp64_kernel<32, false><<<blocks, fp64_threads<false>(), 0, s>>>(ws, p);
   } else if (slot == 0 && split_group(ws.n))
     (track ? traverse_mixed_kernel<true, 1, false, kMixedSplit> : traverse_mixed_kernel<false, 1, false, kMixedSplit>)
         <<<ws.split_grid[track] > 0 ? ws.split_grid[track] : 148, 32 * kMixedSplit, 0, s>>>(ws, p, AdjointBuffers{});

@@ -26,24 +26,28 @@
 
 namespace nbb {
 
-constexpr int kListCap = 96;               // list entries
-constexpr int kListFull = kListCap - 32;   // evaluated from here on: a round of single entries always fits
 constexpr int kFrontier = 1024;            // stack entries per warp
 // With fewer free entries than this a round takes one node only: plain
 // depth-first order, which adds at most 7 entries per tree level.
 constexpr int kFrontierReserve = 8 * (kMaxLevels + 1);
 static_assert(kFrontierReserve + 64 <= kFrontier, "frontier bounds");
-static_assert(kListCap % 4 == 0, "entries are evaluated in fours");
 
 // Stack entry: node index (30 bits) and what is known about it.
 constexpr unsigned kNodeBits = 0x3fffffffu;
 enum EntryState : unsigned { kUntested = 0u, kAccepted = 1u, kLeaf = 2u, kUndecided = 3u };
 
-struct ListShared {
+// Up to kCap interactions to evaluate, in order.  The list is handed out when
+// no round of single entries (32) fits any more.
+template <int kCap>
+struct ListBuffer {
+  static_assert(kCap % 4 == 0 && kCap >= 64, "entries are evaluated in fours");
+  static constexpr int kListCap = kCap;
   double4 src[kListCap];   // position and scaled mass
-  double low2[kListCap];   // undecided cells: lower end of the crit^2 band
-  double rad2[kListCap];   // undecided cells: squared box radius
+  int2 band[kListCap];     // undecided cells: high words of the squared box radius, of the crit^2 band's lower end
   int2 tag[kListCap];      // preorder index (-1: a zero mass); particle's Morton slot, -1 cell, -skip undecided
+};
+// What one walk keeps beside its list.
+struct Frontier {
   unsigned stack[kFrontier];
   double centre[3], scale;  // the targets' box, in units of 1 / scale
   float half[3];
@@ -58,7 +62,7 @@ __device__ __forceinline__ double box_scale(double side) {
 
 // The bounding box of the warp's targets (every lane passes a target): centre
 // and half extents, these rounded up.
-__device__ __forceinline__ void set_target_box(ListShared &sh, const double4 &t, double side) {
+__device__ __forceinline__ void set_target_box(Frontier &sh, const double4 &t, double side) {
   const double v[3] = {t.x, t.y, t.z};
   const double scale = box_scale(side);
 #pragma unroll
@@ -82,7 +86,7 @@ __device__ __forceinline__ void set_target_box(ListShared &sh, const double4 &t,
 // c.y) against the box: kAccepted or kUndecided, or kUntested when every
 // target opens it.  In FP32 with margins that cover every rounding: an offset
 // is off by less than 2^-22 of itself, a square by less than 2^-20.
-__device__ __forceinline__ unsigned judge_cell(const ListShared &sh, const double4 &a, const double4 &c) {
+__device__ __forceinline__ unsigned judge_cell(const Frontier &sh, const double4 &a, const double4 &c) {
   const double scale = sh.scale;
   const float ox = fabsf((float)((a.x - sh.centre[0]) * scale)), oy = fabsf((float)((a.y - sh.centre[1]) * scale)),
               oz = fabsf((float)((a.z - sh.centre[2]) * scale));
@@ -97,9 +101,16 @@ __device__ __forceinline__ unsigned judge_cell(const ListShared &sh, const doubl
   return near2 > outer ? kAccepted : (far2 < inner ? kUntested : kUndecided);
 }
 
-// The acceptance test of target t at list entry j (an undecided cell):
-// accept_fp64's decision, on the entry's copy of the bands.  What the bands
-// leave open (rare) is decided out of line.
+// The acceptance test of a target at squared distance d2 from an undecided
+// cell: accept_fp64's decision.  The high words decide nearly always (both
+// numbers are not negative, so they order as integers): accepted past the box
+// radius, which is above the crit^2 band, and opened below that band.  What
+// they leave open is decided out of line.
+__device__ __forceinline__ bool band_accepts(int2 band, double d2) {
+  const int h = __double2hiint(d2);
+  return h > band.x && h < 0x7ff00000;
+}
+__device__ __forceinline__ bool band_opens(int2 band, double d2) { return __double2hiint(d2) < band.y; }
 static __device__ __noinline__ bool accept_exact(const double4 *c, const double4 *bp, double tx, double ty, double tz,
                                                  double d2) {
   bool accept = (d2 > c->z) ? true : (d2 < c->y) ? false : (__dsqrt_rn(d2) > c->x);
@@ -111,23 +122,27 @@ static __device__ __noinline__ bool accept_exact(const double4 *c, const double4
   }
   return accept;
 }
-__device__ __forceinline__ bool accept_entry(const ListShared &sh, int j, const Workspace &ws, int pre, const double4 &t,
+template <int kCap>
+__device__ __forceinline__ bool accept_entry(const ListBuffer<kCap> &list, int j, const Workspace &ws, int pre, const double4 &t,
                                              double d2) {
-  if (d2 > sh.rad2[j]) return true;   // past the box radius, which is above the crit^2 band
-  if (d2 < sh.low2[j]) return false;  // below the crit^2 band
+  const int2 band = list.band[j];
+  if (band_accepts(band, d2)) return true;
+  if (band_opens(band, d2)) return false;
   return accept_exact(ws.node_c + pre, ws.node_b + pre, t.x, t.y, t.z, d2);
 }
 
-// Walk the subtree of `root` for the targets in the box of sh; eval(count) is
-// called by the whole warp with entries [0, count) of sh, in preorder, each
-// time the list is full and at the end (inactive entries fill the last block
-// of four), and returns the smallest resume index of the warp's targets
+// Walk the subtree of `root` for the targets in the box of sh.  hand(count,
+// last) is called by the whole warp with entries [0, count) of *list, in
+// preorder, each time the list is full and, with last, at the end (inactive
+// entries fill the last block of four); it may move `list` to another buffer,
+// and returns a resume index that all of the warp's targets have reached
 // (frontier entries before it are dropped: a box that spans distant targets
 // leaves cells undecided that every one of them accepts).  Masses are stored
 // times mscale.  Cells judged are added to `tests`.
-template <class Eval>
-__device__ __forceinline__ void ordered_walk(const Workspace &ws, int m, int root, double mscale, ListShared &sh,
-                                             unsigned &tests, Eval &&eval) {
+template <int kListCap, class Hand>
+__device__ __forceinline__ void ordered_walk(const Workspace &ws, int m, int root, double mscale, Frontier &sh,
+                                             ListBuffer<kListCap> *&list, unsigned &tests, Hand &&hand) {
+  constexpr int kListFull = kListCap - 32;
   const int lane = threadIdx.x & 31;
   const unsigned lt = lanemask_lt();
   int sp = (root >= 0 && root < m) ? 1 : 0;
@@ -140,14 +155,15 @@ __device__ __forceinline__ void ordered_walk(const Workspace &ws, int m, int roo
   // a part of a leaf): the limit only ends a walk over inconsistent records
   long long rounds = 2ll * m + ws.n + 2;
   while (true) {
-    if (ls > kListFull || (sp == 0 && ls > 0)) {
-      if (ls + lane < ((ls + 3) & ~3)) sh.tag[ls + lane] = make_int2(-1, 0);
+    const bool last = sp == 0 || --rounds < 0;
+    if (ls > kListFull || last) {
+      if (ls + lane < ((ls + 3) & ~3)) list->tag[ls + lane] = make_int2(-1, 0);
       __syncwarp();
-      done = eval(ls);
+      done = hand(ls, last);
       __syncwarp();
       ls = 0;
     }
-    if (sp == 0 || --rounds < 0) break;
+    if (last) break;
     // the first k entries of the frontier, lane 0 the first in preorder; a
     // round adds at most 8 entries per node taken
     const int k = min(min(32, sp), max(1, (kFrontier - kFrontierReserve - sp) >> 3));
@@ -239,7 +255,8 @@ __device__ __forceinline__ void ordered_walk(const Workspace &ws, int m, int roo
     const int added = __shfl_sync(0xffffffffu, inc, 31);
     if (sp + added > kFrontier) {  // unreachable (see kFrontierReserve)
       if (lane == 0) record_error(ws.sc, kStageTraversal, 9);
-      return;
+      sp = 0;
+      continue;
     }
     int at = sp + added - 1 - (inc - back);  // the lane's first entry
     if (again) sh.stack[at--] = (unsigned)node | (state << 30);
@@ -255,11 +272,10 @@ __device__ __forceinline__ void ordered_walk(const Workspace &ws, int m, int roo
     const int j = ls + off;
     if (cnt > 0) {
       const double4 v = leaf && first != meta.y ? ws.pm4[first] : a;
-      sh.src[j] = make_double4(v.x, v.y, v.z, __dmul_rn(mscale, v.w));
-      sh.tag[j] = make_int2(v.w != 0.0 ? node : -1, leaf ? first : (state == kUndecided ? -meta.x : -1));
+      list->src[j] = make_double4(v.x, v.y, v.z, __dmul_rn(mscale, v.w));
+      list->tag[j] = make_int2(v.w != 0.0 ? node : -1, leaf ? first : (state == kUndecided ? -meta.x : -1));
       if (state == kUndecided) {
-        sh.low2[j] = c.y;
-        sh.rad2[j] = c.w;
+        list->band[j] = make_int2(__double2hiint(c.w), __double2hiint(c.y));
       }
     }
     if (!single) {
@@ -271,8 +287,8 @@ __device__ __forceinline__ void ordered_walk(const Workspace &ws, int m, int roo
         const int l_node = __shfl_sync(0xffffffffu, node, l), l_j = __shfl_sync(0xffffffffu, j, l);
         for (int i = 1 + lane; i < l_cnt; i += 32) {
           const double4 v = ws.pm4[l_first + i];
-          sh.src[l_j + i] = make_double4(v.x, v.y, v.z, __dmul_rn(mscale, v.w));
-          sh.tag[l_j + i] = make_int2(v.w != 0.0 ? l_node : -1, l_first + i);
+          list->src[l_j + i] = make_double4(v.x, v.y, v.z, __dmul_rn(mscale, v.w));
+          list->tag[l_j + i] = make_int2(v.w != 0.0 ? l_node : -1, l_first + i);
         }
       }
     }

@@ -36,9 +36,9 @@ def _check(nbb, oracle, p, theta, soft, g=1.0):
         assert np.array_equal(a, ref[k]), (k, float(np.max(np.abs(a - ref[k]))))
 
 
-# one target per warp below 8192 particles, 32 above; target groups of up to
-# 32 below 131072, of up to 128 cut into 32 above
-@pytest.mark.parametrize("n", [1, 2, 3, 31, 32, 33, 97, 1025, 8191, 8192, 131071, 131072])
+# one target to a set below 5000 particles, 32 above; two warps to a set below
+# 65536; target groups of up to 32 below 131072, of up to 128 cut into 32 above
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 32, 33, 97, 1025, 4999, 5000, 8191, 8192, 65535, 65536, 131071, 131072])
 def test_sizes(nbb_mod, oracle, n):
     _check(nbb_mod, oracle, _particles("plummer", n), 0.5, 0.01)
 
