@@ -324,7 +324,7 @@ struct TraversalParams {
   int kick = 0;
   int precision = 0;     // 0 FP64 plain, 1 mixed
   int group_size = 32;
-  int targets = 32;  // FP64: targets per warp, 32 or 1 (the build's group_chunk)
+  int targets = 32;  // FP64: targets of a set, 32 or 1 (the build's group_chunk)
   // mixed walk: tree levels below the root staged in shared memory per block
   // (0: none; 1 or 2: the top 9 or 73 cells; level-order builds of a single
   // system only)

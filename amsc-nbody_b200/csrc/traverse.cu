@@ -596,10 +596,11 @@ __device__ __forceinline__ bool vjp_entries(const PairList &list, const int *src
                    dz = __fadd2_rn(make_float2(eb.x, eb.y), ntz);
       const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, eps2)));
       zero = zero || !(r2.x > 0.f) || !(r2.y > 0.f);
-      // a factor of 0 takes an entry out of every sum
+      // a factor of 0 takes an entry (the target itself, one without mass) out
+      // of every sum
       float2 r = make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
-      r.x = sr.x != self && r2.x > 0.f ? r.x : 0.f;
-      r.y = sr.y != self && r2.y > 0.f ? r.y : 0.f;
+      r.x = sr.x != self && r2.x > 0.f && eb.z != 0.f ? r.x : 0.f;
+      r.y = sr.y != self && r2.y > 0.f && eb.w != 0.f ? r.y : 0.f;
       const float2 rr = __fmul2_rn(r, r);
       const float2 gi3 = __fmul2_rn(__fmul2_rn(g2, rr), r);
       const float2 rc = __ffma2_rn(dx, cx, __ffma2_rn(dy, cy, __fmul2_rn(dz, cz)));
@@ -627,8 +628,7 @@ __device__ __forceinline__ bool vjp_entries(const PairList &list, const int *src
     const float tb = (b2 ? tw : ty) + __shfl_xor_sync(kFull, b2 ? ty : tw, 2);
     const float val = (b1 ? tb : ta) + __shfl_xor_sync(kFull, b1 ? ta : tb, 1);
     const int e = e0 + 2 * perm + (b4 ? 1 : 0);
-    const float4 eb = list.b[e >> 1];
-    if (val != 0.f && (b4 ? eb.w : eb.z) != 0.f) {
+    if (val != 0.f) {
       const int sr = src[e];
       double *dst = nullptr;
       if (sr >= 0) dst = reinterpret_cast<double *>(ab.part_g + sr);
@@ -724,11 +724,13 @@ __device__ __forceinline__ float4 list_entry(const double4 &a, const double *gbo
 // the reference's test accepts the node for each of them.  Nodes are
 // examined 64 at a time (two per lane) from a warp-private stack in shared
 // memory, each lane fetching both nodes' 48-byte records (MixedNode) in one
-// round trip and the child lists of the nodes that open; a full stack spills
+// round trip (a node's children are consecutive records); a full stack spills
 // its bottom half to a global extension sized for any walk, so every node
-// gets the acceptance test.  Accepted nodes and the particles of reached leaves go to
-// a shared interaction list as FP32 offsets from the group centre (formed in
-// FP64, then rounded) and are evaluated by all lanes in batches of 32.
+// gets the acceptance test.  Accepted nodes and the particles of reached leaves
+// go to a shared interaction list as FP32 offsets from the group centre (formed
+// in FP64, then rounded) and are evaluated by all lanes in batches of
+// kEvalBatch (32 where sources are tracked).  Bound at 2^20 particles by
+// instruction issue (64 % of the slots, FMA pipe 53 %).
 // With kVjp (one target per lane, sources tracked) the same walk evaluates
 // the vector-Jacobian product above instead of the force.
 //
@@ -1062,9 +1064,9 @@ __global__ void __launch_bounds__(mixed_warps<kSplit>() * 32,
     if (kSplit > 1 && !dealt && wid > 0) tests = tests_before;
     if (ls > 0) {
       if (kVjp && (ls & 7)) {
-        // complete the last block of eight, as below
+        // complete the last block of eight with zero-mass entries
         if (lane < (-ls & 7)) {
-          list.put(ls + lane, 1.0e18f, 1.0e18f, 1.0e18f, 0.f);
+          list.put(ls + lane, 0.f, 0.f, 0.f, 0.f);
           src[ls + lane] = -2;
         }
         __syncwarp();
