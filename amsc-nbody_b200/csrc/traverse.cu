@@ -584,6 +584,10 @@ __device__ __forceinline__ bool vjp_entries(const PairList &list, const int *src
   const float2 g2 = make_float2(g, g), m3 = make_float2(-3.f, -3.f);
   float2 sx = make_float2(0.f, 0.f), sy = sx, sz = sx;
   bool zero = false;
+  // a lane without a target has another lane's position and a cotangent of 0:
+  // an infinite distance keeps it out of every sum, where 0 times a factor of
+  // m / eps^5 that overflows (a source at that position) would be NaN
+  if (!valid) eps2 = make_float2(INFINITY, INFINITY);
 #pragma unroll 1
   for (int e0 = 0; e0 < count; e0 += 8) {
     float2 ux[4], uy[4], uz[4], uw[4];

@@ -97,3 +97,27 @@ def test_mixed_adjoint_blocks(nbb_mod, n, soft):
     for a, b in zip(got, ref):
         a, b = a[..., heavy], b[..., heavy]
         assert np.max(np.abs(a - b)) <= 64 * n * 2.0 ** -24 * np.max(np.abs(b))
+
+
+@pytest.mark.parametrize("n,total", [(2, 1.0), (33, 1.0), (33, 33.0), (65, 1.0), (1000, 1.0), (1000, 1000.0), (40001, 1.0)])
+@pytest.mark.parametrize("soft", [1e-9, 2e-8])
+def test_mixed_adjoint_small_softening(nbb_mod, n, total, soft):
+    """A softening whose m eps^-5 overflows in FP32 and target groups with idle
+    lanes: finite gradients, and those of the direct-summation adjoint as in the
+    test above, each term with at most 64 roundings (a batch's sum and the
+    offset's, which weighs by the group's extent over the pair's distance, up
+    to 128 here)."""
+    from nbb import ics
+
+    p = ics.plummer(n, seed=8, total_mass=total)
+    gp = np.random.default_rng(5).standard_normal((3, n)) / n
+    cfg = nbb_mod.SimulationConfig(1e-3, 0.0, soft, 1.0, precision=nbb_mod.PRECISION_MIXED, group_size=32)
+    sim = nbb_mod.Simulation(p, cfg)
+    sim.initialize()
+    sim.rollout(1, 1)
+    got = sim.backward(gp, gp)
+    sim.close()
+    ref = nbb_mod.direct_rollout_adjoint(p, nbb_mod.SimulationConfig(1e-3, 0.0, soft, 1.0), 1, gp, gp)[1:]
+    for a, b in zip(got, ref):
+        assert np.all(np.isfinite(a))
+        assert np.max(np.abs(a - b)) <= 64 * min(n, 128) * 2.0 ** -24 * np.max(np.abs(b))
