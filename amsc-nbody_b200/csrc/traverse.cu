@@ -78,11 +78,87 @@ struct Fp64Targets {
     t = ws.pm4[valid ? s : g0];
     const double soft = ws.sys_eps ? ws.sys_eps[sys] : p.soft;
     soft2 = __dmul_rn(soft, soft);
-    // no squared distance of the system leaves inv_sqrt_core's range
+    // no squared distance of the system leaves inv_sqrt_core's range; without
+    // softening each is looked at
     in_range = soft2 > 0x1p-900 && soft2 < 0x1p900 && ws.sys_box[4 * sys + 3] < 0x1p400;
     resume = valid ? 0 : INT_MAX;
     ax = ay = az = 0.0;
     count = 0;
+  }
+
+  // Entries [0, n) of the list for 32 targets.  kLook: a squared distance may
+  // leave inv_sqrt_core's range (no softening, or extreme units), so each is
+  // looked at.  A loop of its own: the look as a branch inside one loop slows
+  // the softened form by 4 %.  Step of 2^20 particles: 11.1 ms softened, 12.2
+  // without softening (20.5 with the general form for every term).
+  template <bool kLook, int kCap>
+  __device__ __forceinline__ void eval_sets(const Workspace &ws, const ListBuffer<kCap> &list, int n) {
+    for (int j = 0; j < n; j += 4) {
+      double dx[4], dy[4], dz[4], r2[4], f[4];
+      int pre[4], aux[4];
+      bool act[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const double4 v = list.src[j + q];
+        const int2 tag = list.tag[j + q];
+        pre[q] = tag.x;
+        aux[q] = tag.y;
+        dx[q] = __dsub_rn(v.x, t.x);
+        dy[q] = __dsub_rn(v.y, t.y);
+        dz[q] = __dsub_rn(v.z, t.z);
+        f[q] = v.w;
+        r2[q] = sqdist(dx[q], dy[q], dz[q]);
+        act[q] = pre[q] >= resume && aux[q] != s;
+      }
+      if (min(min(aux[0], aux[1]), min(aux[2], aux[3])) < -1) {
+        // undecided cells: a target that accepts one resumes past it
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          act[q] = act[q] && pre[q] >= resume;
+          if (aux[q] < -1) {
+            act[q] = act[q] && accept_entry(list, j + q, ws, pre[q], t, r2[q]);
+            if (act[q]) resume = -aux[q];
+          }
+        }
+      }
+      // all terms are formed before any is added; the sums take them in
+      // the reference's order
+      bool plain = kLook || in_range;  // inv_sqrt_core gets every term right
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        r2[q] = __dadd_rn(r2[q], soft2);
+        plain = plain && __double2loint(r2[q]) != -1;
+      }
+      if constexpr (kLook) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) plain = plain && (!act[q] || inv_sqrt_in_range(r2[q]));
+      }
+      double inv[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) inv[q] = inv_sqrt_core(r2[q]);
+      if (!plain) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if (kLook && (!act[q] || inv_sqrt_in_range(r2[q]))) continue;
+          inv[q] = inv_sqrt_general(r2[q]);
+          if (act[q] && r2[q] <= 0.0) {
+            singular = true;
+            act[q] = false;
+            ++count;
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) f[q] = __dmul_rn(f[q], __dmul_rn(__dmul_rn(inv[q], inv[q]), inv[q]));
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (act[q]) {
+          ax = __fma_rn(f[q], dx[q], ax);
+          ay = __fma_rn(f[q], dy[q], ay);
+          az = __fma_rn(f[q], dz[q], az);
+          ++count;
+        }
+    }
   }
 
   // Entries [0, n) of the list; returns the smallest resume index.  term:
@@ -91,67 +167,10 @@ struct Fp64Targets {
   __device__ __forceinline__ int eval(const Workspace &ws, const ListBuffer<kCap> &list, int n, double4 *term) {
     const int lane = threadIdx.x & 31;
     if constexpr (kTargets == 32) {
-      for (int j = 0; j < n; j += 4) {
-        double dx[4], dy[4], dz[4], r2[4], f[4];
-        int pre[4], aux[4];
-        bool act[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const double4 v = list.src[j + q];
-          const int2 tag = list.tag[j + q];
-          pre[q] = tag.x;
-          aux[q] = tag.y;
-          dx[q] = __dsub_rn(v.x, t.x);
-          dy[q] = __dsub_rn(v.y, t.y);
-          dz[q] = __dsub_rn(v.z, t.z);
-          f[q] = v.w;
-          r2[q] = sqdist(dx[q], dy[q], dz[q]);
-          act[q] = pre[q] >= resume && aux[q] != s;
-        }
-        if (min(min(aux[0], aux[1]), min(aux[2], aux[3])) < -1) {
-          // undecided cells: a target that accepts one resumes past it
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            act[q] = act[q] && pre[q] >= resume;
-            if (aux[q] < -1) {
-              act[q] = act[q] && accept_entry(list, j + q, ws, pre[q], t, r2[q]);
-              if (act[q]) resume = -aux[q];
-            }
-          }
-        }
-        // all terms are formed before any is added; the sums take them in
-        // the reference's order
-        bool plain = in_range;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          r2[q] = __dadd_rn(r2[q], soft2);
-          plain = plain && __double2loint(r2[q]) != -1;
-        }
-        double inv[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) inv[q] = inv_sqrt_core(r2[q]);
-        if (!plain) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            inv[q] = inv_sqrt_general(r2[q]);
-            if (act[q] && r2[q] <= 0.0) {
-              singular = true;
-              act[q] = false;
-              ++count;
-            }
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) f[q] = __dmul_rn(f[q], __dmul_rn(__dmul_rn(inv[q], inv[q]), inv[q]));
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (act[q]) {
-            ax = __fma_rn(f[q], dx[q], ax);
-            ay = __fma_rn(f[q], dy[q], ay);
-            az = __fma_rn(f[q], dz[q], az);
-            ++count;
-          }
-      }
+      if (in_range)
+        eval_sets<false>(ws, list, n);
+      else
+        eval_sets<true>(ws, list, n);
     } else {
       // lane (el, tl): entry el of each block of kLanes, target tl; lanes
       // el = 0, 1, 2 sum the x, y, z component (in ax)

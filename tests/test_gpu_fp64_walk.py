@@ -75,3 +75,19 @@ def test_rounding_exception(nbb_mod, oracle):
     _check(nbb_mod, oracle, p, 0.5, soft)
     inv = 1.0 / np.sqrt(x)
     assert nbb_mod.compute_accelerations(p, 0.5, soft, 1.0)[0][1] == -((inv * inv) * inv) * h
+
+
+@pytest.mark.parametrize("n", [900, 9001, 65537])
+@pytest.mark.parametrize("shape", ["plummer", "coincident", "zero masses"])
+def test_no_softening(nbb_mod, oracle, shape, n):
+    """Without softening every term's range is looked at on its own."""
+    _check(nbb_mod, oracle, _particles(shape, n), 0.6, 0.0)
+
+
+@pytest.mark.parametrize("n", [900, 9001, 65537])
+def test_singular_pair(nbb_mod, n):
+    p = _particles("plummer", n)
+    for a in (p.x, p.y, p.z):
+        a[n - 1] = a[0]
+    with pytest.raises(nbb_mod.DeviceError, match="Singular"):
+        nbb_mod.compute_accelerations(p, 0.6, 0.0, 1.0)
