@@ -127,7 +127,7 @@ struct Fp64Targets {
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         r2[q] = __dadd_rn(r2[q], soft2);
-        plain = plain && __double2loint(r2[q]) != -1;
+        plain = plain && inv_sqrt_low_word(r2[q]);
       }
       if constexpr (kLook) {
 #pragma unroll

@@ -12,11 +12,12 @@ namespace nbb {
 // shared by both and the residual corrections of Markstein ("Computation of
 // elementary functions on the IBM RISC System/6000 processor", 1990), 10 FP64
 // operations.
-//   y0      the estimate, 20 bits, so y0^2 is exact; r = 1 - x y0^2 is rounded
-//           once and |r| < 2^-18
-//   y       y0 (1 + r/2 + 3/8 r^2): relative error 2^-53 from its rounding,
-//           5/16 |r|^3 < 2^-55.6 from the series
-//   g, d    x y and the exact residual x - g^2
+//   y0      the estimate, 21 significant bits, so y0^2 is exact; r = 1 - x y0^2
+//           is rounded once and |r| < 2^-19 (largest over every high word:
+//           1.95 * 2^-20; the low word does not matter)
+//   y       y0 (1 + r/2 + 3/8 r^2): relative error 2^-54 sqrt(x) from its
+//           rounding, 5/16 |r|^3 < 2^-58 from the series (x in [1, 4))
+//   g, d    x y and the residual x - g^2, each rounded once
 //   s       g + d y/2, in error by less than 2^-103.5 sqrt(x) before its
 //           rounding
 //   e, 1/s  y + y (1 - s y), in error by less than 2^-103.5 / s before its
@@ -24,10 +25,12 @@ namespace nbb {
 // A result rounds wrongly only when the exact value lies that close to the
 // middle of two neighbours.  For the square root that takes an x with
 // m^2 - x = k 2^-106 (|k| < 48, m the middle, sqrt(x) in [1, 2)), for the
-// reciprocal an s with s m - 1 = k 2^-106 (|k| < 8); both sets are small and
-// were enumerated and checked one by one: only s = 2 - 2^-52 comes out wrong
-// (Markstein's exception), and inv_sqrt_in_range leaves it to the general
-// form.
+// reciprocal an s with s m - 1 = k 2^-106 (|k| < 8); both sets are small
+// (tests/test_inv_sqrt_rounding.py enumerates them and runs the sequence in
+// exact arithmetic with every estimate of the bound): only the root s = 2 -
+// 2^-52 comes out wrong (Markstein's exception), which 4 - 2^-51 has whatever
+// the estimate and 4 - 2^-50 for some.  inv_sqrt_in_range leaves these two
+// significands to the general form.
 __device__ __forceinline__ double inv_sqrt_core(double x) {
   double y0;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(x));
@@ -40,9 +43,10 @@ __device__ __forceinline__ double inv_sqrt_core(double x) {
   return __fma_rn(__fma_rn(-s, y, 1.0), y, y);
 }
 // Whether inv_sqrt_core gives the right bits for x: its range, without the
-// one significand that rounds wrongly (all ones, whose root is all ones too).
+// significands that may round wrongly (those with their low words are left out).
+__device__ __forceinline__ bool inv_sqrt_low_word(double x) { return (unsigned)__double2loint(x) < 0xfffffffeu; }
 __device__ __forceinline__ bool inv_sqrt_in_range(double x) {
-  return (unsigned)(__double2hiint(x) - 0x06000000) < 0x78000000u && __double2loint(x) != -1;
+  return (unsigned)(__double2hiint(x) - 0x06000000) < 0x78000000u && inv_sqrt_low_word(x);
 }
 static __device__ __noinline__ double inv_sqrt_general(double x) { return __drcp_rn(__dsqrt_rn(x)); }
 

@@ -91,3 +91,20 @@ def test_singular_pair(nbb_mod, n):
         a[n - 1] = a[0]
     with pytest.raises(nbb_mod.DeviceError, match="Singular"):
         nbb_mod.compute_accelerations(p, 0.6, 0.0, 1.0)
+
+
+# both significands whose root is 2 - 2^-52, in each form of the walk
+@pytest.mark.parametrize("n", [2, 5000, 65537])
+@pytest.mark.parametrize("extent", [2.0 ** -28, 2.0 ** -25])
+def test_rounding_exceptions(nbb_mod, oracle, n, extent):
+    """eps^2 = 4 - 2^-50 and distances that round it to 4 - 2^-50 (the smaller
+    extent: d^2 < 2^-52) or to values from there to 4."""
+    from nbb import ics
+
+    rng = np.random.default_rng(11)
+    z = np.zeros(n)
+    x = rng.uniform(0.0, extent, (3, n))
+    p = ics.ParticleData(rng.uniform(0.5, 1.0, n), x[0].copy(), x[1].copy(), x[2].copy(), z, z, z)
+    soft = 2.0 - 2.0 ** -52
+    assert soft * soft == 4.0 - 2.0 ** -50
+    _check(nbb_mod, oracle, p, 0.5, soft)
