@@ -401,11 +401,13 @@ constexpr int kSpill = 512;      // entries moved to / from the global extension
 static_assert(kStackCap - 7 * kWalkPop >= kSpill && kStackCap <= 2 * kSpill, "stack spill bounds");
 // Entries per evaluated batch of the force walk: the list is evaluated when it
 // holds this many, so each batch's set-up and compensated addition are paid
-// once per kEvalBatch entries.  The walks that track sources (zero softening,
-// the adjoint) keep 32-entry batches and the smaller list, whose shared
-// memory keeps 10 blocks per SM.
+// once per kEvalBatch entries.  A batch's two chains of plain FP32 additions
+// are half as long; 96 entries are 1 % faster (2^20 particles: 2.89 against
+// 2.92 ms a step) and lose half as many terms again in a chain, so 64.  The
+// walks that track sources (zero softening, the adjoint) keep 32-entry batches
+// and the smaller list, whose shared memory keeps 10 blocks per SM.
 #ifndef NBB_EVAL_BATCH
-#define NBB_EVAL_BATCH 96
+#define NBB_EVAL_BATCH 64
 #endif
 constexpr int kEvalBatch = NBB_EVAL_BATCH;
 static_assert(kEvalBatch % 32 == 0 && kEvalBatch >= 32 && kEvalBatch <= 128, "batch of whole warps");

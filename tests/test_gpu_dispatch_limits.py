@@ -121,3 +121,36 @@ def test_mixed_adjoint_small_softening(nbb_mod, n, total, soft):
     for a, b in zip(got, ref):
         assert np.all(np.isfinite(a))
         assert np.max(np.abs(a - b)) <= 64 * min(n, 128) * 2.0 ** -24 * np.max(np.abs(b))
+
+
+@pytest.mark.parametrize("extra,group", [(0, 32), (40000, 32), (0, 64), (0, 128)])
+def test_mixed_batch_sum(nbb_mod, extra, group):
+    """Plain FP32 sums run over 64 entries in two chains before they are added
+    with compensation.  One heavy source and then 95 whose terms are 0.49 ulp
+    of its own: at most the 31 later terms of its chain are lost, and one from
+    adding the two chains (a batch of 96 entries loses 47)."""
+    from nbb import ics
+
+    k = 96
+    n = k + 1 + extra
+    rng = np.random.default_rng(12)
+    x = np.full((3, n), -1.0)  # the sources: one leaf, in this order
+    x[0, k] = -0.25            # the target
+    x[:, k + 1:] = rng.uniform(0.2, 1.0, (3, extra))  # without mass, in cells of their own
+
+    def accel(m):
+        mass = np.zeros(n)
+        mass[0], mass[1:k] = 1.0, m
+        z = np.zeros(n)
+        p = ics.ParticleData(mass, x[0].copy(), x[1].copy(), x[2].copy(), z, z, z)
+        sim = nbb_mod.Simulation(p, nbb_mod.SimulationConfig(1e-3, 0.5, 0.01, 1.0, group_size=group,
+                                                             precision=nbb_mod.PRECISION_MIXED))
+        sim.initialize()
+        a = np.stack(sim.accelerations())[0, k]
+        sim.close()
+        return a
+
+    one = accel(0.0)
+    m = 0.49 * float(np.spacing(np.float32(abs(one)))) / abs(one)
+    kept = (accel(m) - one) / (m * one)
+    assert 95 - 32 - 1 <= kept <= 95 + 1
