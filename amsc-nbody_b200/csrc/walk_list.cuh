@@ -152,10 +152,12 @@ __device__ __forceinline__ void ordered_walk(const Workspace &ws, int m, int roo
   if (lane == 0) sh.stack[0] = (unsigned)root;
   __syncwarp();
   // every round finishes or expands the first node of the frontier (or lists
-  // a part of a leaf): the limit only ends a walk over inconsistent records
-  long long rounds = 2ll * m + ws.n + 2;
+  // a part of a leaf): the limit only ends a walk over inconsistent records,
+  // with an error (one test at the frontier's own: 0.3 % of a walk at 2^20
+  // particles; an error of its own at the end of the loop took 1.2 %)
+  unsigned rounds = 2u * (unsigned)m + (unsigned)ws.n + 2u;
   while (true) {
-    const bool last = sp == 0 || --rounds < 0;
+    const bool last = sp == 0;
     if (ls > kListFull || last) {
       if (ls + lane < ((ls + 3) & ~3)) list->tag[ls + lane] = make_int2(-1, 0);
       __syncwarp();
@@ -169,17 +171,18 @@ __device__ __forceinline__ void ordered_walk(const Workspace &ws, int m, int roo
     const int k = min(min(32, sp), max(1, (kFrontier - kFrontierReserve - sp) >> 3));
     unsigned state = kUntested;
     int node = -1;
+    int nc = 0;  // children that replace or follow the entry; more than the frontier holds: not a tree's node
     if (lane < k) {
       const unsigned ent = sh.stack[sp - 1 - lane];
       node = (int)(ent & kNodeBits);
       state = ent >> 30;
+      if (node >= m) nc = kFrontier + 1;
       if (node < done || node >= m) node = -1;
     }
     sp -= k;
     double4 a = make_double4(0.0, 0.0, 0.0, 0.0), c = a;
     int4 meta = make_int4(0, 0, 0, 0), k0 = make_int4(0, 0, 0, 0), k1 = k0;
     bool keep = false;  // an entry that stays or is listed
-    int nc = 0;         // children that replace or follow the entry
     if (node >= 0) {
       a = ws.node_a[node];
       c = ws.node_c[node];
@@ -253,8 +256,8 @@ __device__ __forceinline__ void ordered_walk(const Workspace &ws, int m, int roo
       if (lane >= o) inc += v;
     }
     const int added = __shfl_sync(0xffffffffu, inc, 31);
-    if (sp + added > kFrontier) {  // unreachable (see kFrontierReserve)
-      if (lane == 0) record_error(ws.sc, kStageTraversal, 9);
+    if (sp + added > kFrontier || rounds-- == 0u) {  // only by inconsistent records (see kFrontierReserve, rounds)
+      if (lane == 0) record_error(ws.sc, kStageTraversal, 4);
       sp = 0;
       continue;
     }
