@@ -2941,7 +2941,7 @@ static void launch_level_order_cells(Workspace &ws, cudaStream_t s) {
 }
 
 cudaError_t launch_level_order_tree(Workspace &ws, double theta, cudaStream_t s) {
-  if (!ws.lo_tiles) return cudaErrorInvalidValue;
+  if (!ws.lo_tiles || (ws.records != kRecordsFp64 && ws.records != kRecordsMixed)) return cudaErrorInvalidValue;
   if (ws.n <= kSmallTree) {
     small_tree_kernel<<<1, kSmallThreads, kSmallTreeBytes, s>>>(ws);
     count_launches(1);

@@ -197,7 +197,7 @@ struct WorkspaceParts {
   bool motion = true;        // their velocities and types
   bool reference = true;     // the reference-numbered build
   bool level_order = false;  // the level-order build
-  int records = kRecordsFp64 | kRecordsMixed;
+  int records = kRecordsFp64 | kRecordsMixed;  // the kinds there is room for
 };
 
 // Allocate every buffer of a workspace for n particles.  All device memory is

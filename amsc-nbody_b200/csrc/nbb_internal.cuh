@@ -135,8 +135,9 @@ constexpr int kTopMax = 73;
 // rest pad a warp.
 constexpr int kLevelOrderChannels = 32;
 
-// Traversal records a build writes: the plain FP64 walk's (node_a, node_b,
-// node_c, node_meta, node_kids) and the mixed walk's (node_m).
+// Traversal records: the plain FP64 walk's (node_a, node_b, node_c, node_meta,
+// node_kids) and the mixed walk's (node_m).  A workspace may hold both kinds, a
+// level-order build writes one.
 constexpr int kRecordsFp64 = 1;
 constexpr int kRecordsMixed = 2;
 
@@ -243,7 +244,7 @@ struct Workspace {
   int lo_items = 0;             // groups per thread of a numbering tile: kScanItems or 1
   int lo_tile_count = 0;        // numbering tiles over n
   int *lo_tiles = nullptr;      // lo_tile_count * kLevelOrderChannels: per-tile counts, then their prefixes
-  int records = kRecordsFp64 | kRecordsMixed;  // host: the records the level-order build writes
+  int records = 0;              // host: the kind of records the level-order build writes, set before it
   int *walk_ext = nullptr;    // walk_warps x walk_ext_cap: the mixed walk's stack below shared memory
 };
 
