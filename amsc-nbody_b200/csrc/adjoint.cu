@@ -21,8 +21,7 @@
 // node c on its root path -- a prefix sum down the tree instead of a scatter
 // over each node's particles.
 //
-//   adj_topology_kernel  preorder parent and Morton particle range per node
-//   adj_parent_kernel    preorder parents from a level-order build
+//   adj_parent_kernel    preorder parents from the level-order build
 //   adjoint_walk_kernel  the plain walk's interactions, vector-Jacobian products;
 //                        node / particle cotangents reduced across the warp
 //                        and added atomically
@@ -80,35 +79,8 @@ __global__ void adj_reset_kernel(DevScalars *sc) {
   if (threadIdx.x == 0) sc->work_counter = 0;
 }
 
-// Preorder parent and Morton-order particle range of every octree node
-// (pre = sum of preorder offsets up the parent chain, as the layout does).
-__global__ void __launch_bounds__(kBlock) adj_topology_kernel(Workspace ws, int *pparent, int2 *prange,
-                                                              int *pre_of) {
-  DevScalars *sc = ws.sc;
-  if (sc->error) return;
-  const int m = sc->n_nodes;
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < m; v += gridDim.x * blockDim.x) {
-    int pre = 0, u = v, guard = 0;
-    while (u != 0) {
-      pre += ws.preoff[u];
-      u = ws.oparent[u];
-      if (u < 0 || ++guard > ws.max_level + 1) break;
-    }
-    if (u != 0 || pre < 0 || pre >= m) {
-      record_error(sc, kStageLayout, 1);
-      continue;
-    }
-    if (pre_of) pre_of[v] = pre;
-    pparent[pre] = (v == 0) ? -1 : pre - ws.preoff[v];
-    const bool leaf = ws.child_count[v] == 0;
-    const int cnt = leaf ? max(ws.ocount[v], 0) : ws.psub[v];
-    const int first = leaf ? ws.ofirst[v] : ws.pfirst[v];
-    prange[pre] = (cnt > 0 && first >= 0 && first + cnt <= ws.n) ? make_int2(first, cnt) : make_int2(0, 0);
-  }
-}
-
-// The same parents from a level-order build: a cell's parent is an index of
-// the same numbering.
+// Preorder parent of every node of a level-order build: a cell's parent is an
+// index of the same numbering.
 __global__ void __launch_bounds__(kBlock) adj_parent_kernel(Workspace ws, int *pparent) {
   DevScalars *sc = ws.sc;
   if (sc->error) return;
@@ -409,7 +381,7 @@ __global__ void __launch_bounds__(kBlock) frozen_level_kernel(Workspace ws, Froz
     }
     const double4 r = (tm > 0.0) ? make_double4(wx / tm, wy / tm, wz / tm, tm) : make_double4(0.0, 0.0, 0.0, 0.0);
     fb.aq_oct[q * cap + v] = r;
-    const int pre = fb.pre_of[v];
+    const int pre = ws.pre_of[v];
     if (pre >= 0 && (size_t)pre < m) fb.node_aq[q * cap + pre] = r;
   }
 }
@@ -599,11 +571,10 @@ cudaError_t launch_adjoint_force(Workspace &ws, const TraversalParams &p, const 
 cudaError_t launch_frozen_force(Workspace &ws, const TraversalParams &p, const FrozenBatch &fb, cudaStream_t s) {
   const int grid = grid_of_ws(ws, 8);
   adj_reset_kernel<<<1, 32, 0, s>>>(ws.sc);
-  adj_topology_kernel<<<grid, kBlock, 0, s>>>(ws, fb.pparent, fb.prange, fb.pre_of);
   frozen_gather_kernel<<<grid, kBlock, 0, s>>>(ws, fb);
   for (int level = ws.max_level; level >= 0; --level) frozen_level_kernel<<<grid, kBlock, 0, s>>>(ws, fb, level);
   frozen_walk_kernel<<<grid, 256, 0, s>>>(ws, p, fb);
-  count_launches(5 + ws.max_level);
+  count_launches(4 + ws.max_level);
   return cudaGetLastError();
 }
 

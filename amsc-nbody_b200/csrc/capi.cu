@@ -1927,9 +1927,6 @@ int nbb_frozen_rollout(const nbb_config *cfg, size_t n, const double *mass, cons
   if (e == cudaSuccess) e = al.get(fb.pm4q, qn);
   if (e == cudaSuccess) e = al.get(fb.aq_oct, qcap);
   if (e == cudaSuccess) e = al.get(fb.node_aq, qcap);
-  if (e == cudaSuccess) e = al.get(fb.pre_of, (size_t)ws.cap_nodes);
-  if (e == cudaSuccess) e = al.get(fb.pparent, (size_t)ws.cap_nodes);
-  if (e == cudaSuccess) e = al.get(fb.prange, (size_t)ws.cap_nodes);
   const double *src[7] = {cmass, cx, cy, cz, cvx, cvy, cvz};
   for (int k = 0; k < 7 && e == cudaSuccess; ++k) {
     if (src[k]) {

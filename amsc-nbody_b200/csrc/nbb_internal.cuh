@@ -453,9 +453,6 @@ struct FrozenBatch {
   double4 *pm4q = nullptr;     // copies * n, Morton order of the unperturbed tree
   double4 *aq_oct = nullptr;   // copies * cap_nodes, by octree id
   double4 *node_aq = nullptr;  // copies * cap_nodes, by preorder id
-  int *pre_of = nullptr;       // cap_nodes
-  int *pparent = nullptr;      // cap_nodes
-  int2 *prange = nullptr;      // cap_nodes
 };
 // Frame capture (capture.cu): device scalars and header fields.
 constexpr unsigned long long kFrameHeaderBytes = 128;  // version-3 header
