@@ -490,8 +490,8 @@ __host__ __device__ constexpr int eval_unroll() {
 
 template <bool kTrackSource, int kTPL, int kUnroll>
 __device__ __forceinline__ bool eval_batch(const PairList &list, const int *src, int count, const int *self,
-                                           const float2 *ntx, const float2 *nty, const float2 *ntz, float2 eps2,
-                                           float3 *sum, float3 *comp) {
+                                           const bool *valid, const float2 *ntx, const float2 *nty, const float2 *ntz,
+                                           float2 eps2, float3 *sum, float3 *comp) {
   float2 px[kTPL], py[kTPL], pz[kTPL];
 #pragma unroll
   for (int q = 0; q < kTPL; ++q) px[q] = py[q] = pz[q] = make_float2(0.f, 0.f);
@@ -515,7 +515,8 @@ __device__ __forceinline__ bool eval_batch(const PairList &list, const int *src,
       float2 f = __fmul2_rn(__fmul2_rn(em, r), rr);
       if (kTrackSource) {
         const bool o0 = src[2 * pr] != self[q], o1 = src[2 * pr + 1] != self[q];
-        singular |= (o0 && !(r2.x > 0.f) && em.x != 0.f) || (o1 && !(r2.y > 0.f) && em.y != 0.f);
+        // (an empty slot has another target's position, and that one's entry is not its own)
+        singular |= valid[q] && ((o0 && !(r2.x > 0.f) && em.x != 0.f) || (o1 && !(r2.y > 0.f) && em.y != 0.f));
         f.x = (o0 && r2.x > 0.f) ? f.x : 0.f;
         f.y = (o1 && r2.y > 0.f) ? f.y : 0.f;
       }
@@ -554,15 +555,16 @@ template <bool kTrackSource, int kTPL>
 __device__ __forceinline__ bool eval_slots(const PairList &list, const int *src, int count, int nq,
                                            LaneTargets<kTPL> &t, float2 eps2) {
   if (kTPL >= 4 && nq >= 4)
-    return eval_batch<kTrackSource, (kTPL >= 4 ? 4 : 1), eval_unroll<kTPL>()>(list, src, count, t.s, t.ntx, t.nty, t.ntz, eps2, t.sum,
-                                                         t.comp);
+    return eval_batch<kTrackSource, (kTPL >= 4 ? 4 : 1), eval_unroll<kTPL>()>(
+        list, src, count, t.s, t.valid, t.ntx, t.nty, t.ntz, eps2, t.sum, t.comp);
   if (kTPL >= 3 && nq == 3)
-    return eval_batch<kTrackSource, (kTPL >= 3 ? 3 : 1), eval_unroll<kTPL>()>(list, src, count, t.s, t.ntx, t.nty, t.ntz, eps2, t.sum,
-                                                         t.comp);
+    return eval_batch<kTrackSource, (kTPL >= 3 ? 3 : 1), eval_unroll<kTPL>()>(
+        list, src, count, t.s, t.valid, t.ntx, t.nty, t.ntz, eps2, t.sum, t.comp);
   if (kTPL >= 2 && nq == 2)
-    return eval_batch<kTrackSource, (kTPL >= 2 ? 2 : 1), eval_unroll<kTPL>()>(list, src, count, t.s, t.ntx, t.nty, t.ntz, eps2, t.sum,
-                                                         t.comp);
-  return eval_batch<kTrackSource, 1, eval_unroll<kTPL>()>(list, src, count, t.s, t.ntx, t.nty, t.ntz, eps2, t.sum, t.comp);
+    return eval_batch<kTrackSource, (kTPL >= 2 ? 2 : 1), eval_unroll<kTPL>()>(
+        list, src, count, t.s, t.valid, t.ntx, t.nty, t.ntz, eps2, t.sum, t.comp);
+  return eval_batch<kTrackSource, 1, eval_unroll<kTPL>()>(list, src, count, t.s, t.valid, t.ntx, t.nty, t.ntz, eps2,
+                                                          t.sum, t.comp);
 }
 
 // ------------------------------------------------- mixed adjoint walk ----

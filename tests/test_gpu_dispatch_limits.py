@@ -154,3 +154,33 @@ def test_mixed_batch_sum(nbb_mod, extra, group):
     m = 0.49 * float(np.spacing(np.float32(abs(one)))) / abs(one)
     kept = (accel(m) - one) / (m * one)
     assert 95 - 32 - 1 <= kept <= 95 + 1
+
+
+@pytest.mark.parametrize("n", [50, 1000, 45001])
+@pytest.mark.parametrize("group", [0, 32, 64, 128])
+def test_mixed_no_softening(nbb_mod, n, group):
+    """Groups that fill only some of a lane's target slots, without softening:
+    theta = 0 against direct summation (as in test_mixed_walk_split; a close
+    pair's offset weighs by the group's extent over the distance, up to 64
+    here), and a pair in one place is still singular."""
+    from nbb import ics
+
+    p = ics.plummer(n, seed=10)
+    cfg = nbb_mod.SimulationConfig(1e-3, 0.0, 0.0, 1.0, group_size=group, precision=nbb_mod.PRECISION_MIXED)
+    sim = nbb_mod.Simulation(p, cfg)
+    sim.initialize()
+    acc = np.stack(sim.accelerations())
+    sim.close()
+    x = np.stack([p.x, p.y, p.z])
+    for i in np.random.default_rng(1).choice(n, min(n, 128), replace=False):
+        d = x - x[:, i:i + 1]
+        r2 = np.sum(d * d, axis=0)
+        r2[i] = 1.0
+        term = p.mass * r2 ** -1.5 * d
+        assert np.all(np.abs(acc[:, i] - term.sum(axis=1)) <= 64 * 80 * 2.0 ** -24 * np.abs(term).sum(axis=1).max())
+    for a in (p.x, p.y, p.z):
+        a[n - 1] = a[0]
+    sim = nbb_mod.Simulation(p, cfg)
+    with pytest.raises(nbb_mod.DeviceError, match="Singular"):
+        sim.initialize()
+    sim.close()
