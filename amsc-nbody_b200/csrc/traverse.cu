@@ -1486,12 +1486,16 @@ static cudaError_t grid_of(K kernel, int threads, int sms, int &grid) {
   return e;
 }
 
-// Whether the mixed walk of n particles in groups of at most 32 gives a group
-// to four warps: while one warp each leaves the GPU unfilled.  Walk of Plummer
-// spheres, one / four warps: 48 / 30 us at 1000 particles, 95 / 60 at 4096,
-// 165 / 103 at 16384, 208 / 165 at 32768, 232 / 337 at 65536.
+// Whether the mixed walk in groups of at most 32 gives a group to four warps:
+// while one warp each leaves the GPU unfilled.  Walk of Plummer spheres, one /
+// four warps: 44 / 28 us at 1000 particles, 86 / 48 at 4000, 153 / 122 at 20000,
+// 208 / 165 at 32768, 232 / 337 at 65536.  An ensemble's small systems split into
+// many groups of few particles, each of which would be walked from the root by
+// four warps: 2 systems of 10000 155 / 95 us, 8 of 2000 83 / 66, 12 of 1300 67 /
+// 65, 12 of 3300 118 / 124, 16 of 2400 101 / 126, 64 of 64 20 / 36, 512 of 64 63 /
+// 196.
 constexpr int kMixedSplit = 4;
-static bool split_group(int n) { return n < 40000; }
+static bool split_group(const Workspace &ws) { return ws.n < 40000 && ws.n_systems <= 12; }
 
 // Whether two warps share a set of the FP64 walk of n particles: up to a few
 // sets per pair of warps that fits (figures at the kernel).
@@ -1542,7 +1546,7 @@ cudaError_t launch_traversal(Workspace &ws, const TraversalParams &p, cudaStream
       traverse_fp64_kernel<32, true><<<blocks, fp64_threads<true>(), 0, s>>>(ws, p);
     else
       traverse_fp64_kernel<32, false><<<blocks, fp64_threads<false>(), 0, s>>>(ws, p);
-  } else if (slot == 0 && split_group(ws.n))
+  } else if (slot == 0 && split_group(ws))
     (track ? traverse_mixed_kernel<true, 1, false, kMixedSplit> : traverse_mixed_kernel<false, 1, false, kMixedSplit>)
         <<<ws.split_grid[track] > 0 ? ws.split_grid[track] : 148, 32 * kMixedSplit, 0, s>>>(ws, p, AdjointBuffers{});
   else if (slot == 0)
@@ -1565,7 +1569,7 @@ cudaError_t launch_adjoint_mixed(Workspace &ws, const TraversalParams &p, const 
   if (ws.walk_warps > 0 && grid * kMixedWarps > ws.walk_warps) grid = ws.walk_warps / kMixedWarps;
   TraversalParams q = p;
   q.cache_depth = 0;
-  if (split_group(ws.n))
+  if (split_group(ws))
     traverse_mixed_kernel<true, 1, true, kMixedSplit>
         <<<ws.split_grid[2] > 0 ? ws.split_grid[2] : 148, 32 * kMixedSplit, 0, s>>>(ws, q, ab);
   else

@@ -184,3 +184,33 @@ def test_mixed_no_softening(nbb_mod, n, group):
     with pytest.raises(nbb_mod.DeviceError, match="Singular"):
         sim.initialize()
     sim.close()
+
+
+@pytest.mark.parametrize("systems", [12, 13])
+def test_mixed_ensemble_split(nbb_mod, systems):
+    """Up to 12 systems four warps take a target group, above it one: forces and
+    gradients of an ensemble (theta = 0) against each system's direct sums, as
+    in the tests of single systems above."""
+    from nbb import ics
+
+    size = 70
+    n = size * systems
+    parts = [ics.plummer(size, seed=30 + k) for k in range(systems)]
+    p = ics.ParticleData(*(np.concatenate(a) for a in zip(*[q.arrays() for q in parts])))
+    ens = ics.Ensemble(p, np.arange(systems + 1, dtype=np.int64) * size, np.full(systems, 0.02))
+    cfg = nbb_mod.SimulationConfig(1e-3, 0.0, 0.02, 1.0, precision=nbb_mod.PRECISION_MIXED, group_size=32)
+    gp = np.random.default_rng(5).standard_normal((3, n)) / size
+    sim = nbb_mod.EnsembleSimulation(ens, cfg)
+    sim.initialize()
+    acc = np.stack(sim.accelerations())
+    sim.rollout(1, 1)
+    got = sim.backward(gp, gp)
+    sim.close()
+    one = nbb_mod.SimulationConfig(1e-3, 0.0, 0.02, 1.0)
+    for k, q in enumerate(parts):
+        at = slice(k * size, (k + 1) * size)
+        ref = np.stack(nbb_mod.compute_accelerations(q, 0.0, 0.02, 1.0))
+        assert np.max(np.abs(acc[:, at] - ref)) <= 64 * size * 2.0 ** -24 * np.max(np.abs(ref))
+        grads = nbb_mod.direct_rollout_adjoint(q, one, 1, gp[:, at], gp[:, at])[1:]
+        for a, b in zip(got, grads):
+            assert np.max(np.abs(a[..., at] - b)) <= 64 * size * 2.0 ** -24 * np.max(np.abs(b))
