@@ -1919,19 +1919,42 @@ __device__ __forceinline__ bool lo_whole_group(const Workspace &ws, int level, i
   return !virt && np <= ws.group_max && compact;
 }
 
+// Whether this lane's leaf of np particles is summed by the whole warp
+// (lo_big_leaf) and not by its thread, decided by the warp together.  A particle
+// takes a thread 100 ns and the warp 12.5, but the warp takes its leaves one
+// after another and the threads work side by side: leaves above a size t take
+// the warp their sum / 8 in a thread's time, the others t at most, and the best
+// of t = largest, largest / 2 .. largest / 32 is taken.  Tree stage, all leaves
+// above 32 by the warp / by this rule: 441 / 180 us for 200 leaves of 1000
+// particles, 130 / 90 for 2000 of 100 (by threads alone 181 and 89).
+constexpr int kBigLeaf = 32;
+__device__ __forceinline__ bool lo_is_big_leaf(int np) {
+  const int largest = __reduce_max_sync(0xffffffffu, np);
+  if (largest <= kBigLeaf) return false;
+  int limit = largest, best = largest;
+#pragma unroll 1
+  for (int t = largest / 2; t >= kBigLeaf && t >= largest / 32; t /= 2) {
+    const int cost = t + __reduce_add_sync(0xffffffffu, np > t ? (np + 7) / 8 : 0);
+    if (cost < best) {
+      best = cost;
+      limit = t;
+    }
+  }
+  return np > limit;
+}
+
 // Sums over the particles of a leaf too large for one thread (mass in w, mass
 // times position in x, y, z), for the lanes whose leaf (first particle pf, np
-// particles) holds more than kBigLeaf.  A sum is a chain in sorted order
+// particles) is big.  A sum is a chain in sorted order
 // (octree_physics.cu:95-154), so a leaf takes its length times an FMA's
 // latency at best: the warp loads 32 particles at a time ahead of four lanes
 // that each carry one component's chain from shared memory.  One thread
 // loading and adding alone took 110 ns per particle: 7.2 ms of the tree stage
 // where leaves hold up to 65536 of 2^22 particles, 1.8 ms now.
-constexpr int kBigLeaf = 32;
-__device__ __forceinline__ double4 lo_big_leaf(const Workspace &ws, int pf, int np, double4 *buf) {
+__device__ __forceinline__ double4 lo_big_leaf(const Workspace &ws, bool big, int pf, int np, double4 *buf) {
   const int lane = threadIdx.x & 31;
   double4 own = make_double4(0.0, 0.0, 0.0, 0.0);
-  unsigned todo = __ballot_sync(0xffffffffu, np > kBigLeaf);
+  unsigned todo = __ballot_sync(0xffffffffu, big);
   while (todo) {
     const int l = __ffs(todo) - 1;
     todo &= todo - 1;
@@ -1959,14 +1982,29 @@ __device__ __forceinline__ double4 lo_big_leaf(const Workspace &ws, int pf, int 
 }
 
 // The sums over a leaf's particles [pf, pe) in sorted order (octree_physics.cu:
-// 95-154), the first one given.
+// 95-154), the first one given; four loads in flight in larger leaves (one took
+// 300 ns a particle, four take 100).
 __device__ __forceinline__ double4 lo_leaf_sums(const Workspace &ws, int pf, int pe, double4 q) {
   double tm = 0.0, wx = 0.0, wy = 0.0, wz = 0.0;
-  for (int i = pf; i < pe;) {
-    tm = __dadd_rn(tm, q.w);
-    wx = __fma_rn(q.w, q.x, wx);
-    wy = __fma_rn(q.w, q.y, wy);
-    wz = __fma_rn(q.w, q.z, wz);
+  const auto add = [&](const double4 &v) {
+    tm = __dadd_rn(tm, v.w);
+    wx = __fma_rn(v.w, v.x, wx);
+    wy = __fma_rn(v.w, v.y, wy);
+    wz = __fma_rn(v.w, v.z, wz);
+  };
+  int i = pf;
+#pragma unroll 1
+  for (; pe - i > 4; i += 4) {
+    double4 v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = ws.pm4[i + 1 + k];
+    add(q);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) add(v[k]);
+    q = v[3];
+  }
+  while (i < pe) {
+    add(q);
     if (++i < pe) q = ws.pm4[i];
   }
   return make_double4(wx, wy, wz, tm);
@@ -2103,12 +2141,13 @@ __global__ void __launch_bounds__(kUpsweepBlock, 32) lo_upsweep_kernel(Workspace
       np = ws.glast[g] + 1 - pf;
       if (pf < 0 || np > ws.n - pf) np = 0;
     }
-    const double4 big = lo_big_leaf(ws, pf, np, s_leaf);
+    const bool big = lo_is_big_leaf(np);
+    const double4 big_sums = lo_big_leaf(ws, big, pf, np, s_leaf);
     if (g >= G) continue;
     const int2 lf = ws.lo_gleaf[g];
     int level = (ws.gspan[g] >> 8) & 255;
-    double4 sums = big, a;
-    if (np > 0 && np <= kBigLeaf) sums = lo_leaf_sums(ws, pf, pf + np, ws.pm4[pf]);
+    double4 sums = big_sums, a;
+    if (np > 0 && !big) sums = lo_leaf_sums(ws, pf, pf + np, ws.pm4[pf]);
     if (!lo_leaf_cell(ws, M, sums, lf, level, pf, pf + np, a)) continue;
     int cell = lf.x;
     // the cell's parent and its neighbours' (which children are first and last)
@@ -2497,7 +2536,8 @@ __global__ void __launch_bounds__(kSmallThreads) small_tree_kernel(Workspace ws)
     unsigned sm, lm;
     int lam;
     masks(sp, sm, lm, lam);
-    const double4 big = lo_big_leaf(ws, pf, pe - pf, s_leaf + 32 * warp);
+    const bool big = lo_is_big_leaf(pe - pf);
+    const double4 big_sums = lo_big_leaf(ws, big, pf, pe - pf, s_leaf + 32 * warp);
     const int ek = __popc(lm);
     int inc = ek;
 #pragma unroll
@@ -2549,7 +2589,7 @@ __global__ void __launch_bounds__(kSmallThreads) small_tree_kernel(Workspace ws)
     }
     const int2 lf = make_int2(bleaf, s_from);
     ws.lo_gleaf[g] = lf;
-    sums = pe - pf > kBigLeaf ? big : lo_leaf_sums(ws, pf, pe, sums);
+    sums = big ? big_sums : lo_leaf_sums(ws, pf, pe, sums);
     double4 a;
     if (lo_leaf_cell(ws, M, sums, lf, lam, pf, pe, a)) keep(bleaf, a);
   }

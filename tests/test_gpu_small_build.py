@@ -59,3 +59,21 @@ def test_small_ensemble(nbb_mod, sizes):
                 assert np.array_equal(got, ref)
             else:  # the same interactions, batched from other list positions: FP32 sums of at most 96 terms
                 assert np.max(np.abs(got - ref)) <= 96 * 2.0 ** -24 * np.max(np.linalg.norm(ref, axis=0))
+
+
+@pytest.mark.parametrize("sizes", [(33,), (40,) * 40, (32, 33) * 20, (400, 1, 3, 50, 399, 4, 5, 6, 200, 2), (1000, 31, 500, 260, 130, 70, 35, 9, 1),
+                                   (100,) * 40, (1500,) + (40,) * 31, (3000, 1500, 700, 90, 45, 33, 32) + (8,) * 30, (1000,) * 33])
+def test_large_leaves(nbb_mod, oracle, sizes):
+    """Leaves of many particles, summed by a thread each or by their warp: one
+    large leaf, many alike and mixed ones, below and above the one-block build."""
+    from nbb import ics
+
+    rng = np.random.default_rng(13)
+    x = np.repeat(rng.uniform(-1.0, 1.0, (3, len(sizes))), sizes, axis=1) + rng.uniform(-1e-9, 1e-9, (3, sum(sizes)))
+    z = np.zeros(x.shape[1])
+    p = ics.ParticleData(rng.uniform(0.5, 1.0, x.shape[1]), *[np.ascontiguousarray(a) for a in x], z, z, z)
+    ax, ay, az, st = nbb_mod.compute_accelerations(p, 0.8, 0.05, 1.0, stats=True)
+    ref = oracle.pipeline(p.mass, p.x, p.y, p.z, theta=0.8, soft=0.05, g=1.0)
+    assert st.interactions == ref["interactions"]
+    for a, k in ((ax, "ax"), (ay, "ay"), (az, "az")):
+        assert np.array_equal(a, ref[k]), (k, float(np.max(np.abs(a - ref[k]))))
