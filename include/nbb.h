@@ -160,7 +160,10 @@ typedef struct {
   int n_groups;         /* unique Morton keys G */
   int n_octree_nodes;   /* M */
   int64_t interactions; /* monopole + leaf-pair interactions evaluated */
-  int64_t mac_tests;    /* acceptance tests evaluated */
+  int64_t mac_tests;    /* cells judged by the walks, each once for the targets that
+                           share a walk: a target group (MIXED), a set of up to 32
+                           targets (FP64; a target's own decision at a cell that its
+                           set's box leaves open is not counted again) */
   int group_size;       /* MIXED: warp target group size in use (32, 64 or 128) */
   int64_t stack_overflow; /* MIXED: nodes accepted because the walk's stack was
                              full (their children would not fit).  The stack's
