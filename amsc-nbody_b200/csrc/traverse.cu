@@ -490,8 +490,8 @@ __host__ __device__ constexpr int eval_unroll() {
 
 template <bool kTrackSource, int kTPL, int kUnroll>
 __device__ __forceinline__ bool eval_batch(const PairList &list, const int *src, int count, const int *self,
-                                           const bool *valid, const float2 *ntx, const float2 *nty, const float2 *ntz,
-                                           float2 eps2, float3 *sum, float3 *comp) {
+                                           const float2 *ntx, const float2 *nty, const float2 *ntz, float2 eps2,
+                                           float3 *sum, float3 *comp) {
   float2 px[kTPL], py[kTPL], pz[kTPL];
 #pragma unroll
   for (int q = 0; q < kTPL; ++q) px[q] = py[q] = pz[q] = make_float2(0.f, 0.f);
@@ -515,8 +515,7 @@ __device__ __forceinline__ bool eval_batch(const PairList &list, const int *src,
       float2 f = __fmul2_rn(__fmul2_rn(em, r), rr);
       if (kTrackSource) {
         const bool o0 = src[2 * pr] != self[q], o1 = src[2 * pr + 1] != self[q];
-        // (an empty slot has another target's position, and that one's entry is not its own)
-        singular |= valid[q] && ((o0 && !(r2.x > 0.f) && em.x != 0.f) || (o1 && !(r2.y > 0.f) && em.y != 0.f));
+        singular |= (o0 && !(r2.x > 0.f) && em.x != 0.f) || (o1 && !(r2.y > 0.f) && em.y != 0.f);
         f.x = (o0 && r2.x > 0.f) ? f.x : 0.f;
         f.y = (o1 && r2.y > 0.f) ? f.y : 0.f;
       }
@@ -556,15 +555,15 @@ __device__ __forceinline__ bool eval_slots(const PairList &list, const int *src,
                                            LaneTargets<kTPL> &t, float2 eps2) {
   if (kTPL >= 4 && nq >= 4)
     return eval_batch<kTrackSource, (kTPL >= 4 ? 4 : 1), eval_unroll<kTPL>()>(
-        list, src, count, t.s, t.valid, t.ntx, t.nty, t.ntz, eps2, t.sum, t.comp);
+        list, src, count, t.s, t.ntx, t.nty, t.ntz, eps2, t.sum, t.comp);
   if (kTPL >= 3 && nq == 3)
     return eval_batch<kTrackSource, (kTPL >= 3 ? 3 : 1), eval_unroll<kTPL>()>(
-        list, src, count, t.s, t.valid, t.ntx, t.nty, t.ntz, eps2, t.sum, t.comp);
+        list, src, count, t.s, t.ntx, t.nty, t.ntz, eps2, t.sum, t.comp);
   if (kTPL >= 2 && nq == 2)
     return eval_batch<kTrackSource, (kTPL >= 2 ? 2 : 1), eval_unroll<kTPL>()>(
-        list, src, count, t.s, t.valid, t.ntx, t.nty, t.ntz, eps2, t.sum, t.comp);
-  return eval_batch<kTrackSource, 1, eval_unroll<kTPL>()>(list, src, count, t.s, t.valid, t.ntx, t.nty, t.ntz, eps2,
-                                                          t.sum, t.comp);
+        list, src, count, t.s, t.ntx, t.nty, t.ntz, eps2, t.sum, t.comp);
+  return eval_batch<kTrackSource, 1, eval_unroll<kTPL>()>(list, src, count, t.s, t.ntx, t.nty, t.ntz, eps2, t.sum,
+                                                          t.comp);
 }
 
 // ------------------------------------------------- mixed adjoint walk ----
@@ -607,10 +606,6 @@ __device__ __forceinline__ bool vjp_entries(const PairList &list, const int *src
   const float2 g2 = make_float2(g, g), m3 = make_float2(-3.f, -3.f);
   float2 sx = make_float2(0.f, 0.f), sy = sx, sz = sx;
   bool zero = false;
-  // a lane without a target has another lane's position and a cotangent of 0:
-  // an infinite distance keeps it out of every sum, where 0 times a factor of
-  // m / eps^5 that overflows (a source at that position) would be NaN
-  if (!valid) eps2 = make_float2(INFINITY, INFINITY);
 #pragma unroll 1
   for (int e0 = 0; e0 < count; e0 += 8) {
     float2 ux[4], uy[4], uz[4], uw[4];
@@ -826,6 +821,10 @@ __global__ void __launch_bounds__(mixed_warps<kSplit>() * 32,
       T.s[q] = g0 + lane + 32 * q;
       T.valid[q] = T.s[q] < g1 && T.s[q] < n;
       tp[q] = ws.pm4[T.valid[q] ? T.s[q] : g0];
+      // an empty slot is the group's first target once more: that one's own entry
+      // must be its own too, or it would be a singular pair without softening, and
+      // with a small one m / eps^5 may overflow in the adjoint and 0 times it is NaN
+      if (kTrackSource && !T.valid[q]) T.s[q] = g0;
       T.sum[q] = make_float3(0.f, 0.f, 0.f);
       T.comp[q] = make_float3(0.f, 0.f, 0.f);
     }
