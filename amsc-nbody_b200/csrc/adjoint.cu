@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kBlock) adj_parent_kernel(Workspace ws, int *p
 // column -- 12 instructions per entry, against 60 of a shuffle butterfly per
 // component.  The walk that took one node at a time was bound by that
 // reduction's latency after each node's; a vector-Jacobian product (rebuild
-// and walk) takes 1.2 ms at 16384 particles where that took 3.2, and 2.6 at
+// and walk) takes 0.9 ms at 16384 particles where that took 3.2, and 2.3 at
 // 65536 (4.3).
 constexpr int kAdjList = 96;
 constexpr int kAdjWarps = 2;
