@@ -751,8 +751,8 @@ __device__ __forceinline__ float4 list_entry(const double4 &a, const double *gbo
 // gets the acceptance test.  Accepted nodes and the particles of reached leaves
 // go to a shared interaction list as FP32 offsets from the group centre (formed
 // in FP64, then rounded) and are evaluated by all lanes in batches of
-// kEvalBatch (32 where sources are tracked).  Bound at 2^20 particles by
-// instruction issue (64 % of the slots, FMA pipe 53 %).
+// kEvalBatch (32 where sources are tracked).  Bound at 2^18 particles by
+// instruction issue (60 % of the slots, FMA pipe 57 %).
 // With kVjp (one target per lane, sources tracked) the same walk evaluates
 // the vector-Jacobian product above instead of the force.
 //
